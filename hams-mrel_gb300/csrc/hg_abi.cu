@@ -24,6 +24,7 @@
 #include "hg_kernels.cuh"
 #include "hg_linalg.cuh"
 #include "hg_fintab.cuh"
+#include "hg_fin_keys.cuh"
 
 using hg::FinState;
 
@@ -71,18 +72,12 @@ struct hg_ctx {
   DevBuf<int> bins;                      // finite depth: pairs binned by the cost of their Green function
   DevBuf<float> tab;                     // finite depth, mixed form: tabulated Green function
   DevBuf<float4> pgauss;                 // mixed form: Gauss points of the panel integrals (relative to ox, oy)
-  // finite depth, mixed form: the near pairs (R/h < 0.05) keyed by (R, zq, zp), built once per mesh and
-  // depth (hg_fill_kernel / hg_fill_fin.cu); z-levels: the mesh's distinct depths (at most 2048)
-  bool zlev_ok = false;
+  // finite depth: the pairs keyed by (R, zq, zp), built once per mesh and depth (hg_fin_keys.cuh); zlev: the
+  // mesh's distinct depths, zsrc / zfld each source's and field point's index among them
+  int nlev = 0;
   DevBuf<double> zlev;
-  DevBuf<short> zsrc, zfld;
-  double near_h = 0.0;
-  int near_tn = -1, near_np = 0, near_nu = 0;
-  DevBuf<unsigned long long> near_tabr, near_tabk;
-  DevBuf<longlong2> near_keys;
-  DevBuf<int> near_cnt, near_slot;
-  DevBuf<int2> near_pairs;
-  DevBuf<double> near_F;
+  DevBuf<int> zsrc, zfld;
+  hg::FinKeys fkeys;
   // deep water, mixed form: the self and adjacent pairs (FP64 Newman integrals) listed once per mesh
   int mnear_tn = -1, mnear_np = 0;
   DevBuf<int> mnear_list, mnear_cnt;
@@ -192,43 +187,30 @@ FinState fin_state(const hg_ctx* c) {
 
 bool mixed(const hg_ctx* c) { return c->o.precision == HG_PREC_MIXED; }
 
-// The mixed form's finite-depth pairs below R/h = 0.05 with their region-
-// method values computed once per distinct (R, zq, zp): the map of near
-// pairs to keys is built on the first frequency of a mesh and depth (one
-// host synchronisation for its size) and kept; every frequency evaluates
-// the keys and assembles the pairs from them.
-int near_pairs_dedup(hg_ctx* c, int tn) {
-  const int n = c->n;
-  if (c->near_tn != tn || c->near_h != c->h) {
-    CK(c->near_cnt.ensure(1 + 16));
-    if (hg::near_count(c->st, c->rec.p, c->fx.p, c->tnf, n, tn, c->h, c->zsrc.p, c->zfld.p, c->near_cnt.p))
-      return fail(c, HG_ERR_CUDA, "near-pair count failed: %s", cudaGetErrorString(cudaGetLastError()));
-    int np = 0;
-    CK(cudaMemcpyAsync(&np, c->near_cnt.p, sizeof(int), cudaMemcpyDeviceToHost, c->st));
-    CK(cudaStreamSynchronize(c->st));
-    const unsigned cap = hg::near_table_size(np);
-    CK(c->near_tabr.ensure(cap));
-    CK(c->near_tabk.ensure(cap));
-    CK(c->near_slot.ensure(cap));
-    CK(c->near_pairs.ensure(np > 0 ? np : 1));
-    CK(c->near_keys.ensure(np > 0 ? np : 1));
-    CK(hg::near_build(c->st, c->rec.p, c->fx.p, c->tnf, n, tn, c->h, c->zsrc.p, c->zfld.p, c->near_tabr.p,
-                      c->near_tabk.p, cap, c->near_cnt.p, c->near_slot.p, c->near_pairs.p, c->near_keys.p));
-    CK(hg::near_map(c->st, np, c->near_pairs.p, c->near_slot.p));
-    int nu = 0;
-    CK(cudaMemcpyAsync(&nu, c->near_cnt.p + 16, sizeof(int), cudaMemcpyDeviceToHost, c->st));
-    CK(cudaStreamSynchronize(c->st));
-    CK(c->near_F.ensure((size_t)6 * (nu > 0 ? nu : 1)));
-    c->near_tabr.release();  // the hash tables are needed only to build the map
-    c->near_tabk.release();
-    c->near_slot.release();
-    c->near_np = np;
-    c->near_nu = nu;
-    c->near_tn = tn;
-    c->near_h = c->h;
+// Finite-depth A and S with the region methods evaluated once per distinct
+// (R, zq, zp): every pair, or with near_only those below R/h = 0.05 over what
+// A and S hold.  The keys are built on the first frequency of a mesh and depth
+// and kept.  *done = false where they do not fit (more than 2^27 pairs, or no
+// room in device memory): the caller takes the per-pair kernels.
+template <int FAST, typename OUT>
+int keyed_fill(hg_ctx* c, int tn, int near_only, OUT* A, OUT* S, bool* done) {
+  hg::FinKeys& K = c->fkeys;
+  *done = false;
+  if (K.tn != tn || K.h != c->h || K.near_only != near_only || K.fast != FAST) {
+    const cudaError_t e = hg::fin_keys_build<FAST>(c->st, K, c->rec.p, c->fx.p, c->tnf, c->n, tn, c->h, near_only,
+                                                   c->zsrc.p, c->zfld.p, c->nlev);
+    if (e == cudaErrorMemoryAllocation) return 0;
+    CK(e);
   }
-  CK(hg::near_fill(c->st, c->rec.p, c->fx.p, c->tnf, tn, c->near_np, c->near_nu, c->near_pairs.p, c->near_keys.p,
-                   c->zlev.p, c->near_F.p, fin_state(c), c->o.grn_kind, c->Af.p, c->Sf.p, tn, tn));
+  const cudaError_t e = hg::fin_keys_fill<FAST, OUT>(c->st, K, c->rec.p, c->fx.p, c->tnf, c->zlev.p, fin_state(c),
+                                                     c->o.grn_kind, A, S, tn, tn);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    K.release();
+    return 0;
+  }
+  CK(e);
+  *done = true;
   return 0;
 }
 
@@ -1165,19 +1147,17 @@ int hg_set_mesh(hg_ctx* c, int n, int ntnd, const double* nodes, const int* ncon
     std::vector<double> lev(z);
     std::sort(lev.begin(), lev.end());
     lev.erase(std::unique(lev.begin(), lev.end()), lev.end());
-    c->zlev_ok = lev.size() <= 2048;
-    if (c->zlev_ok) {
-      std::vector<short> zi(z.size());
-      for (size_t k = 0; k < z.size(); ++k)
-        zi[k] = (short)(std::lower_bound(lev.begin(), lev.end(), z[k]) - lev.begin());
-      CK(c->zlev.ensure(lev.size()));
-      CK(c->zsrc.ensure(n));
-      CK(c->zfld.ensure((size_t)n + nl));
-      CK(cudaMemcpyAsync(c->zlev.p, lev.data(), lev.size() * sizeof(double), cudaMemcpyHostToDevice, c->st));
-      CK(cudaMemcpyAsync(c->zsrc.p, zi.data(), (size_t)n * sizeof(short), cudaMemcpyHostToDevice, c->st));
-      CK(cudaMemcpyAsync(c->zfld.p, zi.data(), ((size_t)n + nl) * sizeof(short), cudaMemcpyHostToDevice, c->st));
-    }
-    c->near_tn = -1;  // the near-pair maps belong to the previous mesh
+    c->nlev = (int)lev.size();
+    std::vector<int> zi(z.size());
+    for (size_t k = 0; k < z.size(); ++k)
+      zi[k] = (int)(std::lower_bound(lev.begin(), lev.end(), z[k]) - lev.begin());
+    CK(c->zlev.ensure(lev.size()));
+    CK(c->zsrc.ensure(n));
+    CK(c->zfld.ensure((size_t)n + nl));
+    CK(cudaMemcpyAsync(c->zlev.p, lev.data(), lev.size() * sizeof(double), cudaMemcpyHostToDevice, c->st));
+    CK(cudaMemcpyAsync(c->zsrc.p, zi.data(), (size_t)n * sizeof(int), cudaMemcpyHostToDevice, c->st));
+    CK(cudaMemcpyAsync(c->zfld.p, zi.data(), ((size_t)n + nl) * sizeof(int), cudaMemcpyHostToDevice, c->st));
+    c->fkeys.release();  // the keys and the near-pair list belong to the previous mesh
     c->mnear_tn = -1;
   }
   CK(cudaStreamSynchronize(c->st));
@@ -1225,18 +1205,26 @@ int hg_fill_factor(hg_ctx* c, int irsp) {
   c->tn = tn;  // rows used by this solve (lid rows only with irsp = 1)
   const FinState fs = fin_state(c);
   const bool deep = c->h < 0.0;
+  const bool special = std::fabs(c->v) < (double)1.e-8f || std::fabs(c->v + 1.0) < (double)1.e-8f;
   CK(cudaEventRecord(c->ev[0], c->st));
   CK(c->ipiv.ensure(n));
   if (!mixed(c)) {
     CK(c->A.ensure((size_t)tn * n));
     CK(c->S.ensure((size_t)tn * n));
-    int* bins = nullptr;  // pair indices are ints: the binned fill needs tn * n < 2^31
-    if (!deep && (long long)tn * n < 2147483647LL) {
-      CK(c->bins.ensure(hg::fin_bins_ints(n, tn)));
-      bins = c->bins.p;
+    bool keyed = false;
+    if (!deep && !special) {
+      const int r = keyed_fill<0>(c, tn, 0, c->A.p, c->S.p, &keyed);
+      if (r) return r;
     }
-    CK(hg::launch_green_fill<double2>(c->st, c->rec.p, c->fx.p, c->tnf, n, tn, fs, deep, c->o.grn_kind, c->A.p, c->S.p, tn,
-                                      c->status.p, bins));
+    if (!keyed) {
+      int* bins = nullptr;  // pair indices are ints: the binned fill needs tn * n < 2^31
+      if (!deep && (long long)tn * n < 2147483647LL) {
+        CK(c->bins.ensure(hg::fin_bins_ints(n, tn)));
+        bins = c->bins.p;
+      }
+      CK(hg::launch_green_fill<double2>(c->st, c->rec.p, c->fx.p, c->tnf, n, tn, fs, deep, c->o.grn_kind, c->A.p, c->S.p,
+                                        tn, c->status.p, bins));
+    }
     if (c->keep && irsp == 0) {
       CK(c->A64.ensure((size_t)tn * n));
       CK(cudaMemcpyAsync(c->A64.p, c->A.p, (size_t)tn * n * sizeof(double2), cudaMemcpyDeviceToDevice, c->st));
@@ -1272,7 +1260,6 @@ int hg_fill_factor(hg_ctx* c, int irsp) {
   } else {
     CK(c->Af.ensure((size_t)tn * n));
     CK(c->Sf.ensure((size_t)tn * n));
-    const bool special = std::fabs(c->v) < (double)1.e-8f || std::fabs(c->v + 1.0) < (double)1.e-8f;
     const bool table = !deep && !special && c->o.grn_kind == 8 &&
                        (c->o.fin_table == 1 || (c->o.fin_table < 0 && (long long)tn * n >= 1000000LL));
     if (table) {
@@ -1285,19 +1272,28 @@ int hg_fill_factor(hg_ctx* c, int irsp) {
       CK(hg::fintab_build(c->st, fs, 1.02 * c->rmax + 1.0, c->tab.p, &tab, near ? 2 : 0));
       CK(hg::launch_green_fill_mixed_fin(c->st, c->rec.p, c->fx.p, c->tnf, n, tn, fs, tab, c->ox, c->oy, c->pgauss.p,
                                          c->tab.p + hg::fintab_floats(), c->Af.p, c->Sf.p, tn, c->status.p));
-      if (near && c->zlev_ok) {
-        const int r = near_pairs_dedup(c, tn);
+      bool keyed = false;
+      if (near) {
+        const int r = keyed_fill<0>(c, tn, 1, c->Af.p, c->Sf.p, &keyed);
         if (r) return r;
-      } else if (near) {
+      }
+      if (near && !keyed) {
         CK(c->bins.ensure(hg::fin_bins_ints(n, tn)));
         CK(hg::launch_fin_near(c->st, c->rec.p, c->fx.p, c->tnf, n, tn, fs, c->o.grn_kind, c->Af.p, c->Sf.p, tn,
                                c->bins.p, tn));
       }
     } else if (!deep) {
-      const bool binned = (long long)tn * n < 2147483647LL;
-      if (binned) CK(c->bins.ensure(hg::fin_bins_ints(n, tn)));
-      CK(hg::launch_green_fill_fin_fma(c->st, c->rec.p, c->fx.p, c->tnf, n, tn, fs, c->o.grn_kind, c->Af.p, c->Sf.p, tn,
-                                       c->status.p, binned ? c->bins.p : nullptr));
+      bool keyed = false;
+      if (!special) {
+        const int r = keyed_fill<1>(c, tn, 0, c->Af.p, c->Sf.p, &keyed);
+        if (r) return r;
+      }
+      if (!keyed) {
+        const bool binned = (long long)tn * n < 2147483647LL;
+        if (binned) CK(c->bins.ensure(hg::fin_bins_ints(n, tn)));
+        CK(hg::launch_green_fill_fin_fma(c->st, c->rec.p, c->fx.p, c->tnf, n, tn, fs, c->o.grn_kind, c->Af.p, c->Sf.p, tn,
+                                         c->status.p, binned ? c->bins.p : nullptr));
+      }
     } else if (!special && c->o.grn_kind == 8) {
       const int r = ensure_mnear(c, tn);
       if (r) return r;

@@ -5,7 +5,7 @@
 // FinGrnExtSubs.f90:370-503), below the single precision the mixed form
 // stores, and saves the separate multiply and add instructions on GB300's
 // FP64 pipes, which bound this kernel.
-#include "hg_fill_kernel.cuh"
+#include "hg_fin_keys_impl.cuh"
 
 namespace hg {
 
@@ -17,5 +17,10 @@ cudaError_t launch_green_fill_fin_fma(cudaStream_t st, const double* rec, const 
   k_green_fill<false, float2, 1><<<grid, FILL_ROWS, 0, st>>>(rec, fx, ldf, n, tn, fs, grn_kind, A, S, lda, status, tn);
   return cudaGetLastError();
 }
+
+template cudaError_t fin_keys_build<1>(cudaStream_t, FinKeys&, const double*, const double*, int, int, int, double, int,
+                                       const int*, const int*, int);
+template cudaError_t fin_keys_fill<1, float2>(cudaStream_t, FinKeys&, const double*, const double*, int, const double*,
+                                              const FinState&, int, float2*, float2*, long, int);
 
 }  // namespace hg

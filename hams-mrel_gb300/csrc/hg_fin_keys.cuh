@@ -1,0 +1,89 @@
+// Finite-depth fill with FINGREEN3D's region methods evaluated once per
+// distinct (R, zq, zp).
+//
+// The Green function minus its Rankine pair depends on a pair only through
+// the horizontal distance R and the two depths.  Meshes repeat these triples
+// bit for bit (mirror images, stacked panels, equal bodies at offsets that
+// round alike), and even an irregular mesh repeats every R (the pair and its
+// transpose) and every depth (a panel's whole row).  So the pairs are keyed,
+// once per mesh and depth, by the bits of R as the pair kernel computes it
+// and the indices of their depths, and a frequency then evaluates
+//   per depth and term     the cosines and sines of the two eigenvalue series,
+//   per R and term         K0, K1 of the two series, and J, Y once per R,
+//   per key                the partial sums and Wynn's extrapolation,
+//   per pair               the Rankine pair, the Newman integral and A, S.
+// Every value comes from the same operations in the same order as the per-pair
+// form (hg_green.cuh), so the results agree bit for bit.  Keys are exact:
+// rounding R to share more of them changes the epsilon-extrapolated values of
+// whole matrices coherently (measured: F moves to 1.2e-4).
+//
+// What bounds it: the FP64 pipe (about one operation per clock and SM), in the
+// extrapolation's reciprocals: n^2 / 2 of them per sum of n terms, three sums
+// per key.  They run from shared memory, one sum per thread, the level pairs
+// of the epsilon table fused into one pass.
+#pragma once
+#include <cuda_runtime.h>
+#include <vector>
+#include "hg_common.cuh"
+
+namespace hg {
+
+struct FinState;
+
+// Bands of keys, in the order of their R: 0 LINTON, 1..7 PIDCOCK, 8..13
+// EIGENE (both by series length), 14 EIGEN.
+constexpr int kKeyBins = 15;
+constexpr int kKeyPid0 = 1, kKeyEps0 = 8, kKeyEig = 14;
+// Largest mesh the keys take: 2^27 pairs (28 bits of R slot), 2^18 depths.
+constexpr long long kKeyMaxPairs = 1LL << 27;
+constexpr int kKeyMaxLevels = 1 << 18;
+
+// Consecutive R (and their keys) of one band whose Bessel table fits the
+// table budget.
+struct KeyGroup {
+  int bin, r0, r1, k0, k1;
+};
+
+struct BesselJY {
+  double2 j, y;  // orders 0 and 1
+};
+
+// The keys of one mesh and depth, and the scratch their evaluation uses.
+struct FinKeyData {
+  int tn = -1, near_only = 0, fast = 0, nlev = 0;
+  double h = 0.0;
+  int np = 0, nr = 0, nk = 0;
+  int* pidx = nullptr;     // near_only: pair index i + j tn of each listed pair
+  int* pkey = nullptr;     // key of each (listed) pair
+  int4* keys = nullptr;    // (R index, source depth, field depth, series length)
+  double* rval = nullptr;  // distinct R, grouped by band
+  int* rnt = nullptr;      // series length of each R
+  double* F = nullptr;     // region values, 6 per key
+  double* zt = nullptr;    // per-depth tables
+  double* kt = nullptr;    // Bessel tables of the groups in flight
+  BesselJY* jy = nullptr;  // at wk R
+  size_t zt_cap = 0, kt_cap = 0;
+};
+struct FinKeys : FinKeyData {
+  std::vector<KeyGroup> groups;
+  FinKeys() = default;
+  FinKeys(const FinKeys&) = delete;
+  FinKeys& operator=(const FinKeys&) = delete;
+  ~FinKeys() { release(); }
+  void release();  // frees the device memory: no keys afterwards
+};
+
+// Build the keys of the pairs (field row i < tn, source j < n): all of them, or
+// with near_only those below R/h = 0.05.  cudaErrorMemoryAllocation where they
+// do not fit (the caller takes the per-pair kernels).
+template <int FAST>
+cudaError_t fin_keys_build(cudaStream_t st, FinKeys& K, const double* rec, const double* fx, int ldf, int n, int tn,
+                           double h, int near_only, const int* zsrc, const int* zfld, int nlev);
+
+// Evaluate the keys at fs and write A and S of their pairs (the others are
+// left alone).
+template <int FAST, typename OUT>
+cudaError_t fin_keys_fill(cudaStream_t st, FinKeys& K, const double* rec, const double* fx, int ldf, const double* zlev,
+                          const FinState& fs, int grn_kind, OUT* A, OUT* S, long lda, int ndiag);
+
+}  // namespace hg

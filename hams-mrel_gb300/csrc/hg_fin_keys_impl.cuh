@@ -1,0 +1,647 @@
+// Kernels of hg_fin_keys.cuh, compiled once without fused multiply-adds (plain
+// form, and the mixed form's pairs below R/h = 0.05) and once with them (small
+// problems of the mixed form), as the per-pair kernels are.
+#pragma once
+#include "hg_fill_kernel.cuh"
+#include "hg_fin_keys.cuh"
+
+namespace hg {
+namespace {
+
+constexpr unsigned long long kKeyEmpty = ~0ull;
+constexpr int kZBits = 18;
+constexpr size_t kTableBudget = (size_t)256 << 20;  // bytes of Bessel tables in flight
+constexpr int kMaxSegs = 16;
+
+__device__ __forceinline__ unsigned key_hash(unsigned long long k, unsigned mask) {
+  k ^= k >> 33; k *= 0xff51afd7ed558ccdull; k ^= k >> 33; k *= 0xc4ceb9fe1a85ec53ull; k ^= k >> 33;
+  return (unsigned)k & mask;
+}
+
+// Slot of key in an open-addressing table of mask + 1 slots (inserted if
+// absent); the table holds at most half its slots, so one is found.
+__device__ __forceinline__ unsigned key_insert(unsigned long long* tab, unsigned mask, unsigned long long key) {
+  unsigned s = key_hash(key, mask);
+  for (unsigned probe = 0; probe <= mask; ++probe) {
+    unsigned long long seen = *(volatile unsigned long long*)&tab[s];
+    if (seen != key) {
+      if (seen == kKeyEmpty) seen = atomicCAS(&tab[s], kKeyEmpty, key);
+      if (seen != kKeyEmpty && seen != key) {
+        s = (s + 1) & mask;
+        continue;
+      }
+    }
+    break;
+  }
+  return s;
+}
+
+// Series length of the region method at R (d_series_eps; 10 terms for EIGEN).
+__device__ __forceinline__ int key_terms(double rhp) {
+  if (rhp < 0.0005) return 0;
+  if (rhp < 0.05) return min((int)(SPD(-1010.10) * rhp + SPD(100.50)), 101);
+  if (rhp < 0.5) return (int)(SPD(-88.89) * rhp + SPD(54.45));
+  return 10;
+}
+__device__ __forceinline__ int key_bin(double rhp) {
+  if (rhp < 0.0005) return 0;
+  if (rhp < 0.05) return kKeyPid0 + min(6, max(0, (100 - key_terms(rhp)) / 8));
+  if (rhp < 0.5) return kKeyEps0 + min(5, max(0, (54 - key_terms(rhp)) / 8));
+  return kKeyEig;
+}
+// Rows (terms i = 2, 3, ...) a band's table holds: its longest series.
+inline int bin_rows(int b) {
+  if (b < kKeyPid0) return 0;
+  if (b < kKeyEps0) return b == kKeyPid0 ? 100 : 100 - 8 * (b - kKeyPid0);
+  if (b < kKeyEig) return 54 - 8 * (b - kKeyEps0);
+  return 9;
+}
+inline int bin_width(int b) { return (b >= kKeyPid0 && b < kKeyEps0) ? 2 : 1; }  // K0, K1 pairs per term
+
+// INSERT = false: count the near pairs; true: insert every pair's R and key
+// (near_only: list the near pairs).  R as fin_green computes it.
+template <int FAST, bool INSERT>
+__global__ void __launch_bounds__(128)
+k_key_pairs(const double* __restrict__ rec, const double* __restrict__ fx, int ldf, int n, int tn, double h, int near_only,
+            const int* __restrict__ zsrc, const int* __restrict__ zfld, unsigned long long* __restrict__ tabr,
+            unsigned long long* __restrict__ tabk, unsigned mask, int* __restrict__ counter, int* __restrict__ pidx,
+            int* __restrict__ pslot) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int j = blockIdx.y;
+  bool take = false;
+  double rr = 0.0;
+  if (i < tn) {
+    const double* pr = rec + (size_t)j * PR_SIZE;
+    const double xpq = pr[PR_XQ] - fx[i], ypq = pr[PR_XQ + 1] - fx[i + ldf];
+    rr = sqrt(xpq * xpq + ypq * ypq);
+    take = !near_only || fabs(rr / h) < 0.05;
+  }
+  int at = i + j * tn;
+  if (near_only) {
+    const unsigned act = __ballot_sync(0xffffffffu, take);
+    if (!act) return;
+    const int lane = threadIdx.x & 31, leader = __ffs(act) - 1;
+    int base = 0;
+    if (lane == leader) base = atomicAdd(counter, __popc(act));
+    base = __shfl_sync(0xffffffffu, base, leader);
+    if (!INSERT || !take) return;
+    at = base + __popc(act & ((1u << lane) - 1u));
+    pidx[at] = i + j * tn;
+  }
+  if (!INSERT || !take) return;
+  const unsigned sr = key_insert(tabr, mask, (unsigned long long)__double_as_longlong(rr));
+  const unsigned long long key = ((unsigned long long)sr << (2 * kZBits)) | ((unsigned long long)zsrc[j] << kZBits) |
+                                 (unsigned long long)zfld[i];
+  pslot[at] = (int)key_insert(tabk, mask, key);
+}
+
+// Counter of each lane's bin, one atomic per bin and warp; returns the place
+// of the lane (SCATTER: the cursors advance).
+__device__ __forceinline__ int bin_place(int* counters, int b) {
+  const unsigned peers = __match_any_sync(__activemask(), b);
+  const int lane = threadIdx.x & 31, leader = __ffs(peers) - 1;
+  int base = 0;
+  if (lane == leader) base = atomicAdd(&counters[b], __popc(peers));
+  return __shfl_sync(peers, base, leader) + __popc(peers & ((1u << lane) - 1u));
+}
+
+// Occupied R slots, counted by band and then placed at the bands' cursors.
+template <int FAST, bool SCATTER>
+__global__ void k_key_r(const unsigned long long* __restrict__ tabr, unsigned cap, double h, int* __restrict__ cursor,
+                        int* __restrict__ slot2r, double* __restrict__ rval, int* __restrict__ rnt) {
+  const unsigned s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= cap || tabr[s] == kKeyEmpty) return;
+  const double rr = __longlong_as_double((long long)tabr[s]), rhp = fabs(rr / h);
+  const int at = bin_place(cursor, key_bin(rhp));
+  if (SCATTER) {
+    slot2r[s] = at;
+    rval[at] = rr;
+    rnt[at] = key_terms(rhp);
+  }
+}
+
+// Occupied key slots, counted by group (the piece of R their R lies in) and
+// then placed at the groups' cursors.
+template <int FAST, bool SCATTER>
+__global__ void k_key_unique(const unsigned long long* __restrict__ tabk, unsigned cap, const int* __restrict__ slot2r,
+                             const int* __restrict__ rnt, const int* __restrict__ gend, int ngroups,
+                             int* __restrict__ cursor, int* __restrict__ slot2k, int4* __restrict__ keys) {
+  const unsigned s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= cap || tabk[s] == kKeyEmpty) return;
+  const unsigned long long key = tabk[s];
+  const int r = slot2r[key >> (2 * kZBits)];
+  int lo = 0, hi = ngroups - 1;  // first group whose end is beyond r
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (gend[mid] > r) hi = mid;
+    else lo = mid + 1;
+  }
+  const int at = bin_place(cursor, lo);
+  if (SCATTER) {
+    slot2k[s] = at;
+    const unsigned zm = (1u << kZBits) - 1u;
+    keys[at] = make_int4(r, (int)((key >> kZBits) & zm), (int)(key & zm), rnt[r]);
+  }
+}
+
+template <int FAST>
+__global__ void k_key_map(int np, int* __restrict__ pslot, const int* __restrict__ slot2k) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k < np) pslot[k] = slot2k[pslot[k]];
+}
+
+// Per-depth tables, rows i - 2 of nlev entries: cos and sin of um (z + h) as a
+// source and cos as a field depth, the same for umt = (i - 1) pi / h, then
+// cosh and sinh of wk (z + h).
+struct ZTab {
+  double2* src;   // sin, cos of um (z + h)
+  double2* srct;  // of umt (z + h)
+  double* fld;    // cos of um (z + h)
+  double* fldt;
+  double2* hyp;   // cosh, sinh of wk (z + h)
+  int nlev;
+};
+constexpr int kZRows = 100;
+size_t ztab_doubles(int nlev) { return (size_t)kZRows * nlev * 6 + (size_t)2 * nlev; }
+ZTab ztab_of(double* p, int nlev) {
+  const size_t row = (size_t)kZRows * nlev;
+  ZTab t;
+  t.src = reinterpret_cast<double2*>(p);
+  t.srct = reinterpret_cast<double2*>(p + 2 * row);
+  t.hyp = reinterpret_cast<double2*>(p + 4 * row);
+  t.fld = p + 4 * row + 2 * (size_t)nlev;
+  t.fldt = t.fld + row;
+  t.nlev = nlev;
+  return t;
+}
+
+template <int FAST>
+__global__ void __launch_bounds__(128)
+k_key_depths(FinState s, const double* __restrict__ zlev, ZTab t, int pid) {
+  const int z = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y + 2;
+  if (z >= t.nlev) return;
+  const double h = s.h, zf = zlev[z], wk = s.wk;
+  if (i == 2) t.hyp[z] = make_double2(cosh(wk * (zf + h)), sinh(wk * (zf + h)));
+  if (i > s.nk) return;
+  const size_t e = (size_t)(i - 2) * t.nlev + z;
+  const double um = s.wvn[i - 1];
+  double su, cu;
+  sincos(um * (zf + h), &su, &cu);
+  t.src[e] = make_double2(su, cu);
+  t.fld[e] = cos(um * (zf + h));
+  if (!pid) return;
+  const double umt = (i - 1) * HG_PI / h;
+  sincos(umt * (zf + h), &su, &cu);
+  t.srct[e] = make_double2(su, cu);
+  t.fldt[e] = cos(umt * (zf + h));
+}
+
+// The pieces of R whose Bessel tables are in flight: entry (i - 2) len + r -
+// r0 from base on (PIDCOCK: the second series' table follows the first's).
+struct KeySeg {
+  int r0, len, rows, pid;
+  long base;
+};
+struct KeySegs {
+  KeySeg s[kMaxSegs];
+  int n;
+};
+__device__ __forceinline__ const KeySeg& seg_of(const KeySegs& g, int r) {
+  int k = 0;
+  while (k + 1 < g.n && r >= g.s[k].r0 + g.s[k].len) ++k;
+  return g.s[k];
+}
+
+template <int FAST>
+__global__ void __launch_bounds__(128)
+k_key_bessel(FinState s, KeySegs g, int r0, int r1, const double* __restrict__ rval, const int* __restrict__ rnt,
+             double2* __restrict__ kt, BesselJY* __restrict__ jy) {
+  const int r = r0 + blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y + 2;
+  if (r >= r1) return;
+  const double rr = rval[r];
+  if (i == 2) {
+    double j0, j1, y0, y1;
+    d_jy01b(s.wk * rr, j0, j1, y0, y1);
+    jy[r] = BesselJY{make_double2(j0, j1), make_double2(y0, y1)};
+  }
+  if (i > rnt[r] || i > s.nk) return;
+  const KeySeg& q = seg_of(g, r);
+  const long e = q.base + (long)(i - 2) * q.len + (r - q.r0);
+  const double um = s.wvn[i - 1];
+  double k0, k1;
+  d_ik01a(um * rr, k0, k1);
+  kt[e] = make_double2(k0, k1);
+  if (q.pid) {
+    const double umt = (i - 1) * HG_PI / s.h;
+    d_ik01a(umt * rr, k0, k1);
+    kt[e + (long)q.rows * q.len] = make_double2(k0, k1);
+  }
+}
+
+// Limes (d_limes, hg_green.cuh) on s[0..n] and scratch a[] with stride STR,
+// the a and s steps of a level in one pass: a(i) needs s(i), s(i+1) and the
+// old a(i+1), s(i - 1) the new a(i - 1), a(i) and the old s(i).
+template <int STR>
+__device__ __forceinline__ double limes_pass(int n, double* __restrict__ s, double* __restrict__ a) {
+  double a_max = 0.0, rl = s[n * STR];
+  for (int k = 1; n - 2 * k >= 0; ++k) {
+    const int last = n - 2 * k + 1;
+    double s1 = s[STR];
+    double ap;
+    {
+      const double s0 = s[0], ao = (k == 1) ? 0.0 : a[STR];
+      ap = (s1 != s0) ? ao + 1.0 / (s1 - s0) : ao;
+      a[0] = ap;
+    }
+#pragma unroll 4
+    for (int i = 1; i <= last; ++i) {
+      const double s2 = s[(i + 1) * STR];
+      const double ao = (k == 1) ? 0.0 : a[(i + 1) * STR];
+      const double an = (s2 != s1) ? ao + 1.0 / (s2 - s1) : ao;
+      const double sn = (an != ap) ? s1 + 1.0 / (an - ap) : s1;
+      a[i * STR] = an;
+      s[(i - 1) * STR] = sn;
+      if (fabs(ap) > a_max) {
+        a_max = fabs(ap);
+        rl = sn;
+        if (s1 == sn) return rl;
+      }
+      s1 = s2;
+      ap = an;
+    }
+  }
+  return rl;
+}
+
+// The two expressions of PIDCOCK's terms whose fused form matters.  The
+// extrapolation turns their last bit into differences far above single
+// precision, so the contracted build spells out the fused operations that the
+// contracted per-pair kernel (d_series_eps) takes; the plain build rounds
+// every product.
+// A coefficient (um^2 + v^2) / ((um^2 + v^2) h - v):
+template <int FAST>
+__device__ __forceinline__ double pid_ac(double um, double v, double h) {
+  if (!FAST) return (um * um + v * v) / ((um * um + v * v) * h - v);
+  const double t = fma(v, v, __dmul_rn(um, um));
+  return t / fma(t, h, -v);
+}
+// A difference a x - b y, the first product fused:
+template <int FAST>
+__device__ __forceinline__ double pid_diff(double a, double x, double b, double y) {
+  return FAST ? fma(a, x, -__dmul_rn(b, y)) : a * x - b * y;
+}
+
+// One sum of one key per thread (warps of 32 keys of one sum: 0 G, 1 dG/dR,
+// 2 dG/dz): partial sums into shared memory, extrapolated there into
+// F[6 key + 2 sum].
+constexpr int kSerThreads = 128;
+template <int FAST, bool PID>
+__global__ void __launch_bounds__(kSerThreads)
+k_key_series(FinState s, KeySegs g, int k0, int k1, const int4* __restrict__ keys, ZTab t, const double2* __restrict__ kt,
+             int rows, double* __restrict__ F) {
+  extern __shared__ double sm[];
+  const int lane = threadIdx.x & 31;
+  const int task = blockIdx.x * (kSerThreads / 32) + (threadIdx.x >> 5);
+  const int q = task % 3, u = k0 + (task / 3) * 32 + lane;
+  if (u >= k1) return;
+  double* sq = sm + threadIdx.x;
+  double* sa = sm + (size_t)(rows + 1) * kSerThreads + threadIdx.x;
+  const int4 key = keys[u];
+  const int nt = min(key.w, s.nk);
+  const KeySeg& sg = seg_of(g, key.x);
+  const double2* kr = kt + sg.base + (key.x - sg.r0);
+  const long kstep = sg.len, kpid = (long)sg.rows * sg.len;
+  const double h = s.h, v = s.v;
+  double sum = 0.0;
+  sq[0] = 0.0;
+  for (int i = 2; i <= nt; ++i) {
+    const double um = s.wvn[i - 1];
+    const size_t zr = (size_t)(i - 2) * t.nlev;
+    const double2 kk = kr[(i - 2) * kstep];
+    const double2 sc = t.src[zr + key.y];
+    const double cp = t.fld[zr + key.z];
+    const double k0 = kk.x, k1 = kk.y, su = sc.x, cu = sc.y;
+    if (!PID) {
+      const double tkh = 2.0 * um * h, pm = 4.0 / (1.0 + sin(tkh) / tkh) / h;
+      if (q == 0) sum = sum + pm * k0 * cu * cp;
+      else if (q == 1) sum = sum - pm * um * k1 * cu * cp;
+      else sum = sum - pm * um * k0 * su * cp;
+    } else {
+      const double umt = (i - 1) * HG_PI / h;
+      const double2 kkt = kr[(i - 2) * kstep + kpid];
+      const double2 sct = t.srct[zr + key.y];
+      const double cpt = t.fldt[zr + key.z];
+      const double k0t = kkt.x, k1t = kkt.y, st = sct.x, ct = sct.y;
+      const double ac = pid_ac<FAST>(um, v, h);
+      if (q < 2) {
+        const double am = ac * cu * cp, amt = ct * cpt / h;
+        if (q == 0) sum = sum + pid_diff<FAST>(am, k0, amt, k0t);
+        else sum = sum + pid_diff<FAST>(umt * amt, k1t, um * am, k1);
+      } else {
+        const double dam = -(um * ac * su * cp), damt = -(umt * st * cpt / h);
+        sum = sum - pid_diff<FAST>(damt, k0t, dam, k0);
+      }
+    }
+    sq[(i - 1) * kSerThreads] = sum;
+  }
+  F[6 * (size_t)u + 2 * q] = limes_pass<kSerThreads>(nt - 1, sq, sa);
+}
+
+// The rest of EIGENE and PIDCOCK (d_series_eps) around the extrapolated sums,
+// and EIGEN (d_eigen) whole: one key per thread.
+template <int FAST>
+__global__ void __launch_bounds__(128)
+k_key_finish(FinState s, KeySegs g, int k0, int k1, int pid_end, int eig0, const int4* __restrict__ keys,
+             const double* __restrict__ rval, const double* __restrict__ zlev, const BesselJY* __restrict__ jy, ZTab t,
+             const double2* __restrict__ kt, double* __restrict__ F) {
+  const int u = k0 + blockIdx.x * blockDim.x + threadIdx.x;
+  if (u >= k1) return;
+  const int4 key = keys[u];
+  const double r = rval[key.x], zf = zlev[key.y], zp = zlev[key.z], h = s.h;
+  const BesselJY b = jy[key.x];
+  const double2 hf = t.hyp[key.y];
+  const double hp = t.hyp[key.z].x;
+  double gq[6];
+  double* out = F + 6 * (size_t)u;
+  if (u < pid_end) {
+    d_prop_factors(s, r, hf.x, hf.y, hp, b.j.x, b.j.y, b.y.x, b.y.y, gq, true);
+    const double l0 = out[0], l1 = out[2], l2 = out[4];
+    double is, ir, iz;
+    d_imgs_all(r, zf, zp, h, is, ir, iz);
+    gq[0] = gq[0] + 4.0 * l0 + is;
+    gq[2] = gq[2] + 4.0 * l1 + ir;
+    gq[4] = gq[4] + 4.0 * l2 + iz;
+  } else if (u < eig0) {
+    d_prop_factors(s, r, hf.x, hf.y, hp, b.j.x, b.j.y, b.y.x, b.y.y, gq, false);
+    gq[0] += out[0]; gq[2] += out[2]; gq[4] += out[4];
+  } else {
+    d_prop_factors(s, r, hf.x, hf.y, hp, b.j.x, b.j.y, b.y.x, b.y.y, gq, false);
+    const KeySeg& sg = seg_of(g, key.x);
+    const double2* kr = kt + sg.base + (key.x - sg.r0);
+    for (int i = 2; i <= 10; ++i) {
+      const double km = s.wvn[i - 1], tkh = 2.0 * km * h;
+      const double pm = 4.0 / (1.0 + sin(tkh) / tkh) / h;
+      const size_t zr = (size_t)(i - 2) * t.nlev;
+      const double2 kk = kr[(long)(i - 2) * sg.len];
+      const double k0 = kk.x, k1 = kk.y;
+      const double2 sc = t.src[zr + key.y];
+      const double skzf = sc.x, ckzf = sc.y, ckzp = t.fld[zr + key.z];
+      const double rm1 = pm * k0 * ckzf * ckzp, rm2 = -(pm * km * k1 * ckzf * ckzp),
+                   rm3 = -(pm * km * k0 * skzf * ckzp);
+      gq[0] += rm1; gq[2] += rm2; gq[4] += rm3;
+      if (fabs(rm1) < SPD(1.e-6) && fabs(rm2) < SPD(1.e-6) && fabs(rm3) < SPD(1.e-6)) break;
+    }
+  }
+  d_sub_rankine(r, zf, zp, gq[0], gq[2], gq[4]);
+  for (int q = 0; q < 6; ++q) out[q] = gq[q];
+}
+
+// LINTON keys: few (R/h < 0.0005), each an adaptive quadrature of its own
+// length, so `lanes` of them per warp.
+template <int FAST>
+__global__ void k_key_linton(FinState s, int nk, int lanes, const int4* __restrict__ keys, const double* __restrict__ rval,
+                             const double* __restrict__ zlev, double* __restrict__ F) {
+  const int u = blockIdx.x * lanes + threadIdx.x;
+  if ((int)threadIdx.x >= lanes || u >= nk) return;
+  const int4 key = keys[u];
+  double f[6];
+  fin_regions(s, rval[key.x], zlev[key.y], zlev[key.z], f, 0);
+  for (int q = 0; q < 6; ++q) F[6 * (size_t)u + q] = f[q];
+}
+
+template <int FAST, typename OUT>
+__global__ void __launch_bounds__(128)
+k_key_fill(const double* __restrict__ rec, const double* __restrict__ fx, int ldf, int tn, long np,
+           const int* __restrict__ pidx, const int* __restrict__ pkey, const double* __restrict__ F, FinState fs,
+           int grn_kind, OUT* __restrict__ A, OUT* __restrict__ S, long lda, int ndiag) {
+  for (long k = blockIdx.x * (long)blockDim.x + threadIdx.x; k < np; k += (long)gridDim.x * blockDim.x) {
+    const int p = pidx ? pidx[k] : (int)k;
+    const int i = p % tn, j = p / tn;
+    fill_pair<false, OUT>(rec + (size_t)j * PR_SIZE, fx[i], fx[i + ldf], fx[i + 2 * (size_t)ldf], i, j, fs, grn_kind, A, S,
+                          lda, ndiag, F + 6 * (size_t)pkey[k]);
+  }
+}
+
+template <typename T>
+cudaError_t key_alloc(T** p, size_t count) {
+  return cudaMalloc((void**)p, (count ? count : 1) * sizeof(T));
+}
+
+struct KeyScratch {  // build-time device memory, freed on every way out
+  void* p[8] = {};
+  int n = 0;
+  ~KeyScratch() {
+    for (int k = 0; k < n; ++k) cudaFree(p[k]);
+  }
+  template <typename T>
+  cudaError_t get(T** q, size_t count) {
+    const cudaError_t e = key_alloc(q, count);
+    if (e == cudaSuccess) p[n++] = *q;
+    return e;
+  }
+};
+
+#define KE(call)                          \
+  do {                                    \
+    const cudaError_t e_ = (call);        \
+    if (e_ != cudaSuccess) return e_;     \
+  } while (0)
+
+template <int FAST>
+cudaError_t keys_build_body(cudaStream_t st, FinKeys& K, const double* rec, const double* fx, int ldf, int n, int tn,
+                            double h, int near_only, const int* zsrc, const int* zfld) {
+  KeyScratch sc;
+  const dim3 g((tn + 127) / 128, n);
+  int* cnt = nullptr;  // pair counter, then the cursors of the bands
+  KE(sc.get(&cnt, 1 + 16));
+  KE(cudaMemsetAsync(cnt, 0, 17 * sizeof(int), st));
+  K.np = tn * n;
+  if (near_only) {
+    k_key_pairs<FAST, false><<<g, 128, 0, st>>>(rec, fx, ldf, n, tn, h, 1, zsrc, zfld, nullptr, nullptr, 0, cnt, nullptr,
+                                                nullptr);
+    KE(cudaMemcpyAsync(&K.np, cnt, sizeof(int), cudaMemcpyDeviceToHost, st));
+    KE(cudaStreamSynchronize(st));
+    KE(cudaMemsetAsync(cnt, 0, sizeof(int), st));
+  }
+  if (K.np == 0) return cudaSuccess;
+  size_t free_b = 0, total_b = 0;
+  KE(cudaMemGetInfo(&free_b, &total_b));
+  unsigned cap = 4096;
+  while (cap < 2u * (unsigned)K.np) cap <<= 1;
+  if ((size_t)24 * cap + (size_t)96 * K.np > free_b / 4) return cudaErrorMemoryAllocation;
+  unsigned long long *tabr = nullptr, *tabk = nullptr;
+  int *slot2r = nullptr, *slot2k = nullptr;
+  KE(sc.get(&tabr, cap));
+  KE(sc.get(&tabk, cap));
+  KE(sc.get(&slot2r, cap));
+  KE(sc.get(&slot2k, cap));
+  if (near_only) KE(key_alloc(&K.pidx, K.np));
+  KE(key_alloc(&K.pkey, K.np));
+  KE(cudaMemsetAsync(tabr, 0xff, (size_t)cap * sizeof(*tabr), st));
+  KE(cudaMemsetAsync(tabk, 0xff, (size_t)cap * sizeof(*tabk), st));
+  k_key_pairs<FAST, true><<<g, 128, 0, st>>>(rec, fx, ldf, n, tn, h, near_only, zsrc, zfld, tabr, tabk, cap - 1, cnt,
+                                             K.pidx, K.pkey);
+  // distinct R by band
+  const unsigned cb = (cap + 255) / 256;
+  int hc[16] = {};
+  k_key_r<FAST, false><<<cb, 256, 0, st>>>(tabr, cap, h, cnt + 1, nullptr, nullptr, nullptr);
+  KE(cudaMemcpyAsync(hc, cnt + 1, kKeyBins * sizeof(int), cudaMemcpyDeviceToHost, st));
+  KE(cudaStreamSynchronize(st));
+  int start[kKeyBins + 1] = {0};
+  for (int b = 0; b < kKeyBins; ++b) start[b + 1] = start[b] + hc[b];
+  K.nr = start[kKeyBins];
+  KE(key_alloc(&K.rval, K.nr));
+  KE(key_alloc(&K.rnt, K.nr));
+  KE(key_alloc(&K.jy, K.nr));
+  KE(cudaMemcpyAsync(cnt + 1, start, kKeyBins * sizeof(int), cudaMemcpyHostToDevice, st));
+  k_key_r<FAST, true><<<cb, 256, 0, st>>>(tabr, cap, h, cnt + 1, slot2r, K.rval, K.rnt);
+  // groups of R whose table fits the budget, and the keys in their order
+  std::vector<int> gend;
+  for (int b = 0; b < kKeyBins; ++b) {
+    const size_t per = (size_t)bin_rows(b) * bin_width(b) * sizeof(double2);
+    const int step = per ? (int)(kTableBudget / per) : 1 << 30;
+    for (int r = start[b]; r < start[b + 1];) {
+      const int e = (step < start[b + 1] - r) ? r + step : start[b + 1];
+      K.groups.push_back(KeyGroup{b, r, e, 0, 0});
+      gend.push_back(e);
+      r = e;
+    }
+  }
+  const int ng = (int)gend.size();
+  int *dend = nullptr, *cur = nullptr;
+  KE(sc.get(&dend, ng));
+  KE(sc.get(&cur, ng));
+  KE(cudaMemcpyAsync(dend, gend.data(), ng * sizeof(int), cudaMemcpyHostToDevice, st));
+  KE(cudaMemsetAsync(cur, 0, ng * sizeof(int), st));
+  k_key_unique<FAST, false><<<cb, 256, 0, st>>>(tabk, cap, slot2r, K.rnt, dend, ng, cur, nullptr, nullptr);
+  std::vector<int> kc(ng), ks(ng);
+  KE(cudaMemcpyAsync(kc.data(), cur, ng * sizeof(int), cudaMemcpyDeviceToHost, st));
+  KE(cudaStreamSynchronize(st));
+  for (int q = 0; q < ng; ++q) {
+    ks[q] = K.nk;
+    K.groups[q].k0 = K.nk;
+    K.nk += kc[q];
+    K.groups[q].k1 = K.nk;
+  }
+  KE(key_alloc(&K.keys, K.nk));
+  KE(key_alloc(&K.F, (size_t)6 * K.nk));
+  KE(cudaMemcpyAsync(cur, ks.data(), ng * sizeof(int), cudaMemcpyHostToDevice, st));
+  k_key_unique<FAST, true><<<cb, 256, 0, st>>>(tabk, cap, slot2r, K.rnt, dend, ng, cur, slot2k, K.keys);
+  k_key_map<FAST><<<(K.np + 255) / 256, 256, 0, st>>>(K.np, K.pkey, slot2k);
+  KE(cudaGetLastError());
+  return cudaStreamSynchronize(st);
+}
+
+}  // namespace
+
+template <int FAST>
+cudaError_t fin_keys_build(cudaStream_t st, FinKeys& K, const double* rec, const double* fx, int ldf, int n, int tn,
+                           double h, int near_only, const int* zsrc, const int* zfld, int nlev) {
+  K.release();
+  if ((long long)tn * n > kKeyMaxPairs || nlev > kKeyMaxLevels) return cudaErrorMemoryAllocation;
+  const cudaError_t e = keys_build_body<FAST>(st, K, rec, fx, ldf, n, tn, h, near_only, zsrc, zfld);
+  if (e != cudaSuccess) {
+    K.release();
+    if (e == cudaErrorMemoryAllocation) cudaGetLastError();  // the per-pair kernels run instead
+    return e;
+  }
+  K.tn = tn;
+  K.h = h;
+  K.near_only = near_only;
+  K.fast = FAST;
+  K.nlev = nlev;
+  return cudaSuccess;
+}
+
+template <int FAST, typename OUT>
+cudaError_t fin_keys_fill(cudaStream_t st, FinKeys& K, const double* rec, const double* fx, int ldf, const double* zlev,
+                          const FinState& fs, int grn_kind, OUT* A, OUT* S, long lda, int ndiag) {
+  if (K.np == 0) return cudaSuccess;
+  if (K.zt_cap < ztab_doubles(K.nlev)) {
+    cudaFree(K.zt);
+    K.zt = nullptr;
+    K.zt_cap = 0;
+    KE(key_alloc(&K.zt, ztab_doubles(K.nlev)));
+    K.zt_cap = ztab_doubles(K.nlev);
+  }
+  const ZTab zt = ztab_of(K.zt, K.nlev);
+  bool any_pid = false;
+  int most = 0;
+  for (const KeyGroup& q : K.groups) {
+    any_pid = any_pid || (q.bin >= kKeyPid0 && q.bin < kKeyEps0);
+    most = bin_rows(q.bin) > most ? bin_rows(q.bin) : most;
+  }
+  if (most > 0)
+    k_key_depths<FAST><<<dim3((K.nlev + 127) / 128, most), 128, 0, st>>>(fs, zlev, zt, any_pid ? 1 : 0);
+  size_t gi = 0;
+  if (K.groups[0].bin == 0) {
+    size_t ge = 0;
+    while (ge < K.groups.size() && K.groups[ge].bin == 0) ++ge;
+    const int nl = K.groups[ge - 1].k1;
+    int lanes = (nl + 152 * 16 - 1) / (152 * 16);
+    lanes = lanes < 1 ? 1 : lanes > 32 ? 32 : lanes;
+    k_key_linton<FAST><<<(nl + lanes - 1) / lanes, 32, 0, st>>>(fs, nl, lanes, K.keys, K.rval, zlev, K.F);
+    gi = ge;
+  }
+  while (gi < K.groups.size()) {  // as many groups at a time as the table holds
+    KeySegs g = {};
+    size_t used = 0;
+    const size_t g0 = gi;
+    int rows = 0;
+    while (gi < K.groups.size() && g.n < kMaxSegs) {
+      const KeyGroup& q = K.groups[gi];
+      const size_t cnt = (size_t)bin_rows(q.bin) * bin_width(q.bin) * (q.r1 - q.r0);
+      if (g.n && (used + cnt) * sizeof(double2) > kTableBudget) break;
+      g.s[g.n++] = KeySeg{q.r0, q.r1 - q.r0, bin_rows(q.bin), bin_width(q.bin) == 2 ? 1 : 0, (long)used};
+      used += cnt;
+      rows = bin_rows(q.bin) > rows ? bin_rows(q.bin) : rows;
+      ++gi;
+    }
+    if (K.kt_cap < used) {
+      KE(cudaStreamSynchronize(st));
+      cudaFree(K.kt);
+      K.kt = nullptr;
+      K.kt_cap = 0;
+      KE(key_alloc(&K.kt, 2 * used));
+      K.kt_cap = used;
+    }
+    double2* kt = reinterpret_cast<double2*>(K.kt);
+    const int r0 = K.groups[g0].r0, r1 = K.groups[gi - 1].r1;
+    k_key_bessel<FAST><<<dim3((r1 - r0 + 127) / 128, rows), 128, 0, st>>>(fs, g, r0, r1, K.rval, K.rnt, kt, K.jy);
+    const int ka = K.groups[g0].k0, kb = K.groups[gi - 1].k1;
+    int pid_end = ka, eig0 = ka;
+    int prows = 0, erows = 0;
+    for (size_t q = g0; q < gi; ++q) {
+      const KeyGroup& w = K.groups[q];
+      if (w.bin < kKeyEps0) {
+        pid_end = w.k1;
+        prows = bin_rows(w.bin) > prows ? bin_rows(w.bin) : prows;
+      } else if (w.bin < kKeyEig) {
+        erows = bin_rows(w.bin) > erows ? bin_rows(w.bin) : erows;
+      }
+      if (w.bin < kKeyEig) eig0 = w.k1;
+    }
+    auto blocks = [](int keys) { return (unsigned)((((keys + 31) / 32) * 3 + kSerThreads / 32 - 1) / (kSerThreads / 32)); };
+    if (pid_end > ka) {
+      const size_t smem = (size_t)2 * (prows + 1) * kSerThreads * sizeof(double);
+      KE(cudaFuncSetAttribute(k_key_series<FAST, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      k_key_series<FAST, true><<<blocks(pid_end - ka), kSerThreads, smem, st>>>(fs, g, ka, pid_end, K.keys, zt, kt, prows,
+                                                                               K.F);
+    }
+    if (eig0 > pid_end) {
+      const size_t smem = (size_t)2 * (erows + 1) * kSerThreads * sizeof(double);
+      KE(cudaFuncSetAttribute(k_key_series<FAST, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      k_key_series<FAST, false><<<blocks(eig0 - pid_end), kSerThreads, smem, st>>>(fs, g, pid_end, eig0, K.keys, zt, kt,
+                                                                                  erows, K.F);
+    }
+    k_key_finish<FAST><<<(kb - ka + 127) / 128, 128, 0, st>>>(fs, g, ka, kb, pid_end, eig0, K.keys, K.rval, zlev, K.jy, zt,
+                                                             kt, K.F);
+  }
+  long fb = ((long)K.np + 127) / 128;
+  if (fb > 152L * 64) fb = 152L * 64;
+  k_key_fill<FAST, OUT><<<(unsigned)fb, 128, 0, st>>>(rec, fx, ldf, K.tn, K.np, K.pidx, K.pkey, K.F, fs, grn_kind, A, S, lda,
+                                                     ndiag);
+  return cudaGetLastError();
+}
+
+}  // namespace hg

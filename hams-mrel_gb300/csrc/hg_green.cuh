@@ -15,6 +15,7 @@
 // instead of restarted from E_1 on every series term.  Loops that hit their
 // cap set HG_DEV_SERIES_CAP in the status word.
 #pragma once
+#include <string.h>
 #include "hg_common.cuh"
 
 #ifdef __CUDACC__
@@ -288,6 +289,103 @@ HGD inline double d_eix(double x) {  // EIX :146-172
   return exp(x) / x * ei;
 }
 
+// Divisors of the K0/K1 power series, known in advance: k*k and k*(k+1) with
+// their correctly rounded reciprocals, and the partial sums of 1/k in the order
+// the series adds them.
+#ifdef __CUDA_ARCH__
+#define HGD_CONST __constant__ const
+#else
+#define HGD_CONST static const
+#endif
+HGD_CONST double c_kk[51] = {0.0,
+1.0, 4.0, 9.0, 16.0, 25.0, 36.0, 49.0, 64.0, 81.0, 100.0,
+    121.0, 144.0, 169.0, 196.0, 225.0, 256.0, 289.0, 324.0, 361.0, 400.0,
+    441.0, 484.0, 529.0, 576.0, 625.0, 676.0, 729.0, 784.0, 841.0, 900.0,
+    961.0, 1024.0, 1089.0, 1156.0, 1225.0, 1296.0, 1369.0, 1444.0, 1521.0, 1600.0,
+    1681.0, 1764.0, 1849.0, 1936.0, 2025.0, 2116.0, 2209.0, 2304.0, 2401.0, 2500.0};
+HGD_CONST double c_kk1[51] = {0.0,
+2.0, 6.0, 12.0, 20.0, 30.0, 42.0, 56.0, 72.0, 90.0, 110.0,
+    132.0, 156.0, 182.0, 210.0, 240.0, 272.0, 306.0, 342.0, 380.0, 420.0,
+    462.0, 506.0, 552.0, 600.0, 650.0, 702.0, 756.0, 812.0, 870.0, 930.0,
+    992.0, 1056.0, 1122.0, 1190.0, 1260.0, 1332.0, 1406.0, 1482.0, 1560.0, 1640.0,
+    1722.0, 1806.0, 1892.0, 1980.0, 2070.0, 2162.0, 2256.0, 2352.0, 2450.0, 2550.0};
+HGD_CONST double c_rcp_kk[51] = {0.0,
+1.0, 0.25, 0.1111111111111111, 0.0625,
+    0.04, 0.027777777777777776, 0.02040816326530612, 0.015625,
+    0.012345679012345678, 0.01, 0.008264462809917356, 0.006944444444444444,
+    0.005917159763313609, 0.00510204081632653, 0.0044444444444444444, 0.00390625,
+    0.0034602076124567475, 0.0030864197530864196, 0.002770083102493075, 0.0025,
+    0.0022675736961451248, 0.002066115702479339, 0.001890359168241966, 0.001736111111111111,
+    0.0016, 0.0014792899408284023, 0.0013717421124828531, 0.0012755102040816326,
+    0.0011890606420927466, 0.0011111111111111111, 0.001040582726326743, 0.0009765625,
+    0.0009182736455463728, 0.0008650519031141869, 0.0008163265306122449, 0.0007716049382716049,
+    0.0007304601899196494, 0.0006925207756232687, 0.0006574621959237344, 0.000625,
+    0.000594883997620464, 0.0005668934240362812, 0.0005408328826392645, 0.0005165289256198347,
+    0.0004938271604938272, 0.0004725897920604915, 0.0004526935264825713, 0.00043402777777777775,
+    0.00041649312786339027, 0.0004};
+HGD_CONST double c_rcp_kk1[51] = {0.0,
+0.5, 0.16666666666666666, 0.08333333333333333, 0.05,
+    0.03333333333333333, 0.023809523809523808, 0.017857142857142856, 0.013888888888888888,
+    0.011111111111111112, 0.00909090909090909, 0.007575757575757576, 0.00641025641025641,
+    0.005494505494505495, 0.004761904761904762, 0.004166666666666667, 0.003676470588235294,
+    0.0032679738562091504, 0.0029239766081871343, 0.002631578947368421, 0.002380952380952381,
+    0.0021645021645021645, 0.001976284584980237, 0.0018115942028985507, 0.0016666666666666668,
+    0.0015384615384615385, 0.0014245014245014246, 0.0013227513227513227, 0.0012315270935960591,
+    0.0011494252873563218, 0.001075268817204301, 0.0010080645161290322, 0.000946969696969697,
+    0.00089126559714795, 0.0008403361344537816, 0.0007936507936507937, 0.0007507507507507507,
+    0.0007112375533428165, 0.0006747638326585695, 0.000641025641025641, 0.0006097560975609756,
+    0.0005807200929152149, 0.0005537098560354374, 0.0005285412262156448, 0.000505050505050505,
+    0.0004830917874396135, 0.00046253469010175765, 0.0004432624113475177, 0.00042517006802721087,
+    0.00040816326530612246, 0.000392156862745098};
+HGD_CONST double c_harm[51] = {0.0,
+1.0, 1.5, 1.8333333333333333, 2.083333333333333,
+    2.283333333333333, 2.4499999999999997, 2.5928571428571425, 2.7178571428571425,
+    2.8289682539682537, 2.9289682539682538, 3.0198773448773446, 3.103210678210678,
+    3.180133755133755, 3.251562326562327, 3.3182289932289937, 3.3807289932289937,
+    3.439552522640758, 3.4951080781963135, 3.547739657143682, 3.597739657143682,
+    3.6453587047627294, 3.690813250217275, 3.73429151108684, 3.7759581777535067,
+    3.8159581777535068, 3.854419716215045, 3.8914567532520823, 3.927171038966368,
+    3.9616537975870574, 3.9949871309203906, 4.02724519543652, 4.05849519543652,
+    4.08879822573955, 4.118209990445433, 4.146781419016861, 4.174559196794639,
+    4.201586223821666, 4.22790201329535, 4.2535430389363755, 4.278543038936376,
+    4.302933282838815, 4.326742806648339, 4.349998620601827, 4.3727258933290996,
+    4.394948115551322, 4.416687245986104, 4.4379638417307845, 4.4587971750641175,
+    4.4792053383294235, 4.499205338329423};
+
+// a / d, correctly rounded, for a small integer d (here below 2^12) whose
+// correctly rounded reciprocal rd is at hand (Markstein 1990; Brisebarre,
+// Muller and Raina 2004): q = a rd is within 1.5 units in the last place, the
+// residual a - d q is then exact (d is short), and q + residual rd is off the
+// true quotient by far less than its distance from any midpoint (a multiple
+// of 1 / (2 d) units).  Three FP64 operations where the general division
+// takes about ten.
+HGD inline double div_small(double a, double d, double rd) {
+  const double q = a * rd;
+  return fma(fma(-d, q, a), rd, q);
+}
+
+// fabs(num / den) < 1e-15 as the rounded division decides it.  The high words
+// of |num| and of 1e-15 |den| decide it unless they agree to about one part
+// in 2^19; only then is the division made.
+HGD inline int hi_word(double x) {
+#ifdef __CUDA_ARCH__
+  return __double2hiint(x);
+#else
+  long long b;
+  memcpy(&b, &x, sizeof b);
+  return (int)(b >> 32);
+#endif
+}
+HGD inline bool ratio_below(double num, double den) {
+  const double a = fabs(num), t = 1.0e-15 * fabs(den);
+  const int ha = hi_word(a), ht = hi_word(t);
+  if (ht < 0x7ff00000) {
+    if (ha + 1 < ht) return true;
+    if (ha > ht + 1) return false;
+  }
+  return fabs(num / den) < 1.0e-15;
+}
+
 // IK01A :538-640, returning K0 and K1.
 HGD inline void d_ik01a(double x, double& bk0, double& bk1) {
   if (x == 0.0) { bk0 = 1.0e+300; bk1 = 1.0e+300; return; }
@@ -297,16 +395,16 @@ HGD inline void d_ik01a(double x, double& bk0, double& bk1) {
     bi0 = 1.0;
     double r = 1.0;
     for (int k = 1; k <= 50; ++k) {
-      r = 0.25 * r * x2 / (double)(k * k);
+      r = div_small(0.25 * r * x2, c_kk[k], c_rcp_kk[k]);
       bi0 += r;
-      if (fabs(r / bi0) < 1.0e-15) break;
+      if (ratio_below(r, bi0)) break;
     }
     bi1 = 1.0;
     r = 1.0;
     for (int k = 1; k <= 50; ++k) {
-      r = 0.25 * r * x2 / (double)(k * (k + 1));
+      r = div_small(0.25 * r * x2, c_kk1[k], c_rcp_kk1[k]);
       bi1 += r;
-      if (fabs(r / bi1) < 1.0e-15) break;
+      if (ratio_below(r, bi1)) break;
     }
     bi1 = 0.5 * x * bi1;
   } else {
@@ -335,12 +433,11 @@ HGD inline void d_ik01a(double x, double& bk0, double& bk1) {
   }
   if (x <= 9.0) {
     const double ct = -(log(x / 2.0) + 0.5772156649015329);
-    double k0v = 0.0, w0 = 0.0, r = 1.0, ww = 0.0;
+    double k0v = 0.0, r = 1.0, ww = 0.0;
     for (int k = 1; k <= 50; ++k) {
-      w0 += 1.0 / k;
-      r = 0.25 * r / (double)(k * k) * x2;
-      k0v += r * (w0 + ct);
-      if (fabs((k0v - ww) / k0v) < 1.0e-15) break;
+      r = div_small(0.25 * r, c_kk[k], c_rcp_kk[k]) * x2;
+      k0v += r * (c_harm[k] + ct);
+      if (ratio_below(k0v - ww, k0v)) break;
       ww = k0v;
     }
     bk0 = k0v + ct;
@@ -468,17 +565,16 @@ struct FinState {
 };
 
 // Imaginary (propagating) part shared by the three series methods:
-// P0 (i J0 - Y0) etc. of EIGEN/EIGENE/PIDCOCK.
-HGD inline void d_prop_part(const FinState& s, double r, double zf, double zp, double g[6],
-                                            bool pid) {
+// P0 (i J0 - Y0) etc. of EIGEN/EIGENE/PIDCOCK, from the factors
+// czf = cosh wk (zf + h), szf = sinh wk (zf + h), czp = cosh wk (zp + h) and
+// the Bessel functions at wk r.
+HGD inline void d_prop_factors(const FinState& s, double r, double czf, double szf, double czp, double j0, double j1,
+                               double y0, double y1, double g[6], bool pid) {
   const double wk = s.wk, h = s.h;
-  const double p0 = HG_PI / s.nm0 * cosh(wk * (zf + h)) * cosh(wk * (zp + h));
+  const double p0 = HG_PI / s.nm0 * czf * czp;
   // DP0 carries WK inside (PIDCOCK :601) or outside (EIGEN :317, EIGENE :442);
   // kept in the reference's order so the rounding matches.
-  const double dp0 = pid ? wk * HG_PI / s.nm0 * sinh(wk * (zf + h)) * cosh(wk * (zp + h))
-                         : wk * (HG_PI / s.nm0 * sinh(wk * (zf + h)) * cosh(wk * (zp + h)));
-  double j0, j1, y0, y1;
-  d_jy01b(wk * r, j0, j1, y0, y1);
+  const double dp0 = pid ? wk * HG_PI / s.nm0 * szf * czp : wk * (HG_PI / s.nm0 * szf * czp);
   g[0] = -p0 * y0;  g[1] = p0 * j0;
   g[2] = wk * p0 * y1; g[3] = -(wk * p0) * j1;
   g[4] = -dp0 * y0; g[5] = dp0 * j0;
@@ -486,6 +582,13 @@ HGD inline void d_prop_part(const FinState& s, double r, double zf, double zp, d
     g[0] += 2.0 / h * (0.5772156649015328 + log(r / 4.0 / h));
     g[2] += 2.0 / (r * h);
   }
+}
+HGD inline void d_prop_part(const FinState& s, double r, double zf, double zp, double g[6],
+                                            bool pid) {
+  const double wk = s.wk, h = s.h;
+  double j0, j1, y0, y1;
+  d_jy01b(wk * r, j0, j1, y0, y1);
+  d_prop_factors(s, r, cosh(wk * (zf + h)), sinh(wk * (zf + h)), cosh(wk * (zp + h)), j0, j1, y0, y1, g, pid);
 }
 
 // EIGEN (R/h >= 0.5), FinGreen3D.f90:281-362.  g = [re0, im0, re1, im1, re2, im2]

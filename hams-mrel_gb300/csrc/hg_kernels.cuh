@@ -37,27 +37,6 @@ cudaError_t launch_green_fill_fin_fma(cudaStream_t st, const double* rec, const 
 // bins: scratch of fin_bins_ints(n, tn) ints.
 cudaError_t launch_fin_near(cudaStream_t st, const double* rec, const double* fx, int ldf, int n, int tn,
                             const FinState& fs, int grn_kind, float2* A, float2* S, long lda, int* bins, int ndiag);
-// The same pairs with their region-method values computed once per distinct
-// (R, zq, zp), keyed exactly (hg_fill_fin.cu).  zsrc[n] / zfld[tn]: index of
-// each source's / field point's depth in the mesh's distinct depths zlev (at
-// most 2048).  near_count: number of near pairs into *counter (device).
-// near_build: two hash tables of near_table_size(np) slots (cap) - R's bits,
-// then the keys -, the pairs listed as (i + j tn, key slot), the distinct
-// keys grouped by cost into ukeys (R's bits, depth indices) with
-// slot2u[slot] = key index; counters[1 + 15] = number of keys afterwards.
-// near_map: pair slots to key indices.  near_fill (per frequency): the
-// region methods per key into F (6 doubles each), then A(i, j), S(i, j) of
-// every near pair.
-int near_count(cudaStream_t st, const double* rec, const double* fx, int ldf, int n, int tn, double h,
-               const short* zsrc, const short* zfld, int* counter);
-unsigned near_table_size(int npairs);
-cudaError_t near_build(cudaStream_t st, const double* rec, const double* fx, int ldf, int n, int tn, double h,
-                       const short* zsrc, const short* zfld, unsigned long long* tabr, unsigned long long* tabk,
-                       unsigned cap, int* counters, int* slot2u, int2* pairs, longlong2* ukeys);
-cudaError_t near_map(cudaStream_t st, int np, int2* pairs, const int* slot2u);
-cudaError_t near_fill(cudaStream_t st, const double* rec, const double* fx, int ldf, int tn, int np, int nu,
-                      const int2* pairs, const longlong2* ukeys, const double* zlev, double* F, const FinState& fs,
-                      int grn_kind, float2* A, float2* S, long lda, int ndiag);
 // Tabulated finite-depth Green function of the mixed form (hg_fintab.cu):
 // fintab_floats() floats of device scratch; rmax = largest horizontal
 // distance between a field point and a source; gmin = first R segment built
