@@ -455,17 +455,92 @@ k_key_finish(FinState s, KeySegs g, int k0, int k1, int pid_end, int eig0, const
   for (int q = 0; q < 6; ++q) out[q] = gq[q];
 }
 
-// LINTON keys: few (R/h < 0.0005), each an adaptive quadrature of its own
-// length, so `lanes` of them per warp.
+// d_aquad<0> (adaptive Gauss-Kronrod 7-15 of d_gfun) by the 16 lanes of a half
+// warp: lanes 0..6 take the Gauss nodes, 7..14 the nodes the Kronrod rule
+// adds, and every lane forms both sums and walks the same interval stack.
+// hm: the half's lanes.
 template <int FAST>
-__global__ void k_key_linton(FinState s, int nk, int lanes, const int4* __restrict__ keys, const double* __restrict__ rval,
-                             const double* __restrict__ zlev, double* __restrict__ F) {
-  const int u = blockIdx.x * lanes + threadIdx.x;
-  if ((int)threadIdx.x >= lanes || u >= nk) return;
+__device__ double aquad_half(const LintonPar& lp, double a, double b, double eps, int tag, unsigned hm, int& flags) {
+  const int kMaxStack = 64;
+  double sa[kMaxStack], sb[kMaxStack];
+  const int j = threadIdx.x & 15;
+  const double node = j < 7 ? c_xgq[j] : c_xkq[j < 15 ? 2 * (j - 7) : 14];
+  int top = 1, guard = 0;
+  sa[0] = a; sb[0] = b;
+  double total = 0.0;
+  while (top > 0) {
+    --top;
+    const double aa = sa[top], bb = sb[top];
+    const double t = 0.5 * (bb + aa + (bb - aa) * node);
+    const double mine = d_gfun(lp, t, tag);
+    double gi = 0.0, gk = 0.0;
+    for (int i = 0; i < 7; ++i) gi += c_wgq[i] * (bb - aa) / 2.0 * __shfl_sync(hm, mine, i, 16);
+    for (int i = 1; i <= 15; ++i) {
+      const double f = __shfl_sync(hm, mine, i % 2 == 0 ? i / 2 - 1 : 7 + (i - 1) / 2, 16);
+      gk += c_wkq[i - 1] * (bb - aa) / 2.0 * f;
+    }
+    const double err = pow(200.0 * fabs(gk - gi), 1.5);
+    if (err > eps && fabs(aa - bb) > eps && top + 2 <= kMaxStack && guard < 4096) {
+      const double mid = (aa + bb) / 2.0;
+      sa[top] = mid; sb[top] = bb; ++top;
+      sa[top] = aa; sb[top] = mid; ++top;
+    } else {
+      if (err > eps && fabs(aa - bb) > eps) flags |= HG_DEV_QUAD_STACK;
+      total += gk;
+    }
+    ++guard;
+  }
+  return total;
+}
+
+// LINTON keys, one per warp: few (R/h < 0.0005) and each a long serial chain
+// for one thread (three adaptive quadratures of some hundred integrand values,
+// each of them error functions summed as series: 8.8 ms for the 168 keys of
+// the three cylinders, 19 ms for the irregular hull's 1547).  The lanes take
+// the 20 terms of the series side by side and then the 15 nodes of a
+// quadrature interval, the two half warps different integrals (1.8 ms for the hull); sums are formed
+// in d_linton's order.
+template <int FAST>
+__global__ void __launch_bounds__(128)
+k_key_linton(FinState s, int nk, const int4* __restrict__ keys, const double* __restrict__ rval,
+             const double* __restrict__ zlev, double* __restrict__ F) {
+  const int u = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (u >= nk) return;
   const int4 key = keys[u];
-  double f[6];
-  fin_regions(s, rval[key.x], zlev[key.y], zlev[key.z], f, 0);
-  for (int q = 0; q < 6; ++q) F[6 * (size_t)u + q] = f[q];
+  const double r = rval[key.x], zf = zlev[key.y], zp = zlev[key.z], h = s.h, wk = s.wk;
+  const double eps = SPD(1.e-6), a = d_linton_a(s);
+  const double czf = cosh(wk * (zf + h)), czp = cosh(wk * (zp + h)), szf = sinh(wk * (zf + h));
+  double rm[3] = {0.0, 0.0, 0.0};
+  int mine = 0, flags = 0;
+  if (lane < 20) d_linton_term(s, lane + 1, a, r, zf, zp, czf, czp, szf, rm, mine);
+  __syncwarp();
+  double re[3] = {0.0, 0.0, 0.0};
+  for (int i = 1; i <= 20; ++i) {
+    double t[3];
+    for (int k = 0; k < 3; ++k) t[k] = __shfl_sync(0xffffffffu, rm[k], i - 1);
+    flags |= __shfl_sync(0xffffffffu, mine, i - 1);
+    for (int k = 0; k < 3; ++k) re[k] += t[k];
+    if (d_linton_last(i, t)) break;
+  }
+  const LintonPar lp{s.v, r, zf, zp, h};
+  const double pa = a * h;
+  const bool low = lane < 16;
+  const unsigned hm = low ? 0xffffu : 0xffff0000u;
+  int qf = 0;
+  const double first = aquad_half<FAST>(lp, 0.0, pa / 2.0, eps, low ? 1 : 2, hm, qf);
+  const double third = low ? aquad_half<FAST>(lp, 0.0, pa / 2.0, eps, 3, hm, qf) : 0.0;
+  __syncwarp();
+  double q[3], g[6];
+  q[0] = __shfl_sync(0xffffffffu, first, 0);
+  q[1] = __shfl_sync(0xffffffffu, first, 16);
+  q[2] = __shfl_sync(0xffffffffu, third, 0);
+  flags |= __shfl_sync(0xffffffffu, qf, 0) | __shfl_sync(0xffffffffu, qf, 16);
+  d_linton_rest(s, a, r, zf, zp, czf, czp, szf, re, q, g);
+  if (r == 0.0) { g[2] = 0.0; g[3] = 0.0; }
+  if (lane == 0) {
+    for (int k = 0; k < 6; ++k) F[6 * (size_t)u + k] = g[k];
+    if (flags) hg_set_status(s.status, flags);
+  }
 }
 
 template <int FAST, typename OUT>
@@ -637,9 +712,7 @@ cudaError_t fin_keys_fill(cudaStream_t st, FinKeys& K, const double* rec, const 
     size_t ge = 0;
     while (ge < K.groups.size() && K.groups[ge].bin == 0) ++ge;
     const int nl = K.groups[ge - 1].k1;
-    int lanes = (nl + 152 * 16 - 1) / (152 * 16);
-    lanes = lanes < 1 ? 1 : lanes > 32 ? 32 : lanes;
-    k_key_linton<FAST><<<(nl + lanes - 1) / lanes, 32, 0, st>>>(fs, nl, lanes, K.keys, K.rval, zlev, K.F);
+    k_key_linton<FAST><<<(nl + 3) / 4, 128, 0, st>>>(fs, nl, K.keys, K.rval, zlev, K.F);
     gi = ge;
   }
   while (gi < K.groups.size()) {  // as many groups at a time as the table holds

@@ -712,7 +712,7 @@ HGD_TABLE double c_wkq[15] = {0.022935322010529, 0.063092092629979, 0.1047900103
 // wider than eps.  kind 0 integrates d_gfun(tag), kind 1 d_ffun(no, tag).
 template <int KIND>
 HGD inline double d_aquad(const LintonPar& lp, double r, double wvn, int no, double a, double b,
-                                 double eps, int tag, int* status) {
+                                 double eps, int tag, int& flags) {
   const int kMaxStack = 64;
   double sa[kMaxStack], sb[kMaxStack];
   int top = 0;
@@ -743,7 +743,7 @@ HGD inline double d_aquad(const LintonPar& lp, double r, double wvn, int no, dou
       sa[top] = mid; sb[top] = bb; ++top;   // right half, popped second
       sa[top] = aa; sb[top] = mid; ++top;   // left half, popped first
     } else {
-      if (err > eps && fabs(aa - bb) > eps) hg_set_status(status, HG_DEV_QUAD_STACK);
+      if (err > eps && fabs(aa - bb) > eps) flags |= HG_DEV_QUAD_STACK;
       total += gk;
     }
     ++guard;
@@ -752,7 +752,7 @@ HGD inline double d_aquad(const LintonPar& lp, double r, double wvn, int no, dou
 }
 
 // SA0 / DSA0 (:1389-1524): series for the m=0 coefficient and its R-derivative.
-HGD inline void d_sa0(double r, double pa, double wk, double& sa, double& dsa, int* status) {
+HGD inline void d_sa0(double r, double pa, double wk, double& sa, double& dsa, int& flags) {
   const double ga = 0.5772156649015328, eps = SPD(1.e-6);
   const double x = (r / pa) * (r / pa), ex = exp(-x), lg = log(wk * r / 2.0);
   // SA0 uses E_{n+1}(x), DSA0 uses E_n(x), n = 1, 2, ...
@@ -777,7 +777,7 @@ HGD inline void d_sa0(double r, double pa, double wk, double& sa, double& dsa, i
       if (!(fabs(rm) > eps)) ddone = true;
     }
     if (sdone && ddone) break;
-    if (n == 400) hg_set_status(status, HG_DEV_SERIES_CAP);
+    if (n == 400) flags |= HG_DEV_SERIES_CAP;
     sgn = -sgn;
     facn *= (n + 1);
     e_n = e_np1;
@@ -788,7 +788,7 @@ HGD inline void d_sa0(double r, double pa, double wk, double& sa, double& dsa, i
 }
 
 // SAM / DSAM (:1575-1693) for m >= 1.
-HGD inline void d_sam(double r, double pa, double wvn, double& sa, double& dsa, int* status) {
+HGD inline void d_sam(double r, double pa, double wvn, double& sa, double& dsa, int& flags) {
   const double eps = SPD(1.e-6);
   const double x = (wvn * pa / 2.0) * (wvn * pa / 2.0), ex = exp(-x);
   double e = d_e1xa(x);  // E_{n+1} for n = 0
@@ -808,7 +808,7 @@ HGD inline void d_sam(double r, double pa, double wvn, double& sa, double& dsa, 
       if (!(fabs(rm) > eps)) ddone = true;
     }
     if (sdone && ddone) break;
-    if (n == 400) hg_set_status(status, HG_DEV_SERIES_CAP);
+    if (n == 400) flags |= HG_DEV_SERIES_CAP;
     sgn = -sgn;
     facn *= (n + 1);
     e = (ex - x * e) / (double)(n + 1);
@@ -817,78 +817,87 @@ HGD inline void d_sam(double r, double pa, double wvn, double& sa, double& dsa, 
   dsa = ds / 4.0 / HG_PI;
 }
 
-HGD inline void d_linton(const FinState& st, double r, double zf, double zp, double g[6]) {
-  const double eps = SPD(1.e-6), v = st.v, wk = st.wk, h = st.h;
+// Splitting parameter of the method: pa = a h (a depends on v alone).
+HGD inline double d_linton_a(const FinState& st) {
+  const double v = st.v;
   double a;
   if (v < 0.02) a = 3324.2 * (v * v * v) - 258.89 * (v * v) + 8.3958 * v + 1.3208;
   else if (v < 0.1) a = -30.303 * (v * v * v) - 2.8138 * (v * v) + 2.7740 * v + 0.05052;
   else if (v < 1.0) a = 1.5699 * (v * v * v) - 2.5075 * (v * v) + 1.8316 * v + 0.1077;
   else a = -0.000069641 * (v * v * v) - 0.0017082 * (v * v) + 0.45566 * v + 0.80551;
-  a = fabs(a) / (wk * h);
+  return fabs(a) / (st.wk * st.h);
+}
+
+// Term i = 1 .. 20 of the series with coefficients COEF/DCOEF (:1170-1340).
+HGD inline void d_linton_term(const FinState& st, int i, double a, double r, double zf, double zp, double czf, double czp,
+                              double szf, double rm[3], int& flags) {
+  const double eps = SPD(1.e-6), wk = st.wk, h = st.h;
   const double pa = a * h, dnt = pa * pa / 4.0;
+  double cof, dcof;
+  const double km = (i == 1) ? wk : st.wvn[i - 1];
+  if (i == 1) {
+    if (fabs(r) < SPD(1.e-6)) {
+      cof = -d_eix(wk * wk * dnt) / 4.0 / HG_PI;
+      dcof = 0.0;
+    } else if (r / a <= 0.5) {
+      d_sa0(r, pa, wk, cof, dcof, flags);
+    } else {
+      double j0, j1, y0, y1;
+      d_jy01b(wk * r, j0, j1, y0, y1);
+      LintonPar dummy{};
+      cof = -y0 / 4.0 - d_aquad<1>(dummy, r, wk, 1, 0.0, dnt, eps, 1, flags);
+      dcof = wk * y1 / 4.0 - d_aquad<1>(dummy, r, wk, 1, 0.0, dnt, eps, 2, flags);
+    }
+  } else {
+    if (fabs(r) < SPD(1.e-6)) {
+      cof = d_e1xa(km * km * dnt) / 4.0 / HG_PI;
+      dcof = 0.0;
+    } else if (r / a <= 1.0) {
+      d_sam(r, pa, km, cof, dcof, flags);
+    } else {
+      LintonPar dummy{};
+      double p1 = dnt + 100.0;
+      for (int it = 0; fabs(d_ffun(r, km, i, p1, 1)) > eps; ++it) {
+        if (it > 100000) { flags |= HG_DEV_SERIES_CAP; break; }
+        p1 += 100.0;
+      }
+      cof = d_aquad<1>(dummy, r, km, i, dnt, p1, eps, 1, flags);
+      p1 = dnt + 100.0;
+      for (int it = 0; fabs(d_ffun(r, km, i, p1, 2)) > eps; ++it) {
+        if (it > 100000) { flags |= HG_DEV_SERIES_CAP; break; }
+        p1 += 100.0;
+      }
+      dcof = d_aquad<1>(dummy, r, km, i, dnt, p1, eps, 2, flags);
+    }
+  }
+  if (i == 1) {
+    rm[0] = -(cof / st.nm0 * czf * czp);
+    rm[1] = -(dcof / st.nm0 * czf * czp);
+    rm[2] = -(cof * wk / st.nm0 * szf * czp);
+  } else {
+    const double nm = h / 2.0 * (1.0 + sin(2.0 * km * h) / (2.0 * km * h));
+    double s1, c1;
+    sincos(km * (zf + h), &s1, &c1);
+    const double c2 = cos(km * (zp + h));
+    rm[0] = -(cof / nm * c1 * c2);
+    rm[1] = -(dcof / nm * c1 * c2);
+    rm[2] = cof * km / nm * s1 * c2;
+  }
+}
+// The series ends at the first term after the second whose parts are all small.
+HGD inline bool d_linton_last(int i, const double rm[3]) {
+  const double eps = SPD(1.e-6);
+  return i > 2 && fabs(rm[0]) < eps && fabs(rm[1]) < eps && fabs(rm[2]) < eps;
+}
+
+// The rest of the method from the series' sums re[3] and the integrals
+// q[3] over [0, pa / 2] of d_gfun's three integrands.
+HGD inline void d_linton_rest(const FinState& st, double a, double r, double zf, double zp, double czf, double czp,
+                              double szf, const double re[3], const double q[3], double g[6]) {
+  const double v = st.v, wk = st.wk, h = st.h, pa = a * h, p4 = 4.0 * HG_PI;
   const double sr = sqrt(r * r + (zf - zp) * (zf - zp));
   const double sr1 = sqrt(r * r + (2.0 * h + zf + zp) * (2.0 * h + zf + zp));
   const double sr2 = sqrt(r * r + (zf + zp) * (zf + zp));
-  const double p4 = 4.0 * HG_PI;
-
-  // III. evanescent series with coefficients COEF/DCOEF (:1170-1340)
-  double re0 = 0.0, re1 = 0.0, re2 = 0.0;
-  const double czf = cosh(wk * (zf + h)), czp = cosh(wk * (zp + h)), szf = sinh(wk * (zf + h));
-  for (int i = 1; i <= 20; ++i) {
-    double cof, dcof;
-    const double km = (i == 1) ? wk : st.wvn[i - 1];
-    if (i == 1) {
-      if (fabs(r) < SPD(1.e-6)) {
-        cof = -d_eix(wk * wk * dnt) / 4.0 / HG_PI;
-        dcof = 0.0;
-      } else if (r / a <= 0.5) {
-        d_sa0(r, pa, wk, cof, dcof, st.status);
-      } else {
-        double j0, j1, y0, y1;
-        d_jy01b(wk * r, j0, j1, y0, y1);
-        LintonPar dummy{};
-        cof = -y0 / 4.0 - d_aquad<1>(dummy, r, wk, 1, 0.0, dnt, eps, 1, st.status);
-        dcof = wk * y1 / 4.0 - d_aquad<1>(dummy, r, wk, 1, 0.0, dnt, eps, 2, st.status);
-      }
-    } else {
-      if (fabs(r) < SPD(1.e-6)) {
-        cof = d_e1xa(km * km * dnt) / 4.0 / HG_PI;
-        dcof = 0.0;
-      } else if (r / a <= 1.0) {
-        d_sam(r, pa, km, cof, dcof, st.status);
-      } else {
-        LintonPar dummy{};
-        double p1 = dnt + 100.0;
-        for (int it = 0; fabs(d_ffun(r, km, i, p1, 1)) > eps; ++it) {
-          if (it > 100000) { hg_set_status(st.status, HG_DEV_SERIES_CAP); break; }
-          p1 += 100.0;
-        }
-        cof = d_aquad<1>(dummy, r, km, i, dnt, p1, eps, 1, st.status);
-        p1 = dnt + 100.0;
-        for (int it = 0; fabs(d_ffun(r, km, i, p1, 2)) > eps; ++it) {
-          if (it > 100000) { hg_set_status(st.status, HG_DEV_SERIES_CAP); break; }
-          p1 += 100.0;
-        }
-        dcof = d_aquad<1>(dummy, r, km, i, dnt, p1, eps, 2, st.status);
-      }
-    }
-    double rm1, rm2, rm3;
-    if (i == 1) {
-      rm1 = -(cof / st.nm0 * czf * czp);
-      rm2 = -(dcof / st.nm0 * czf * czp);
-      rm3 = -(cof * wk / st.nm0 * szf * czp);
-    } else {
-      const double nm = h / 2.0 * (1.0 + sin(2.0 * km * h) / (2.0 * km * h));
-      double s1, c1;
-      sincos(km * (zf + h), &s1, &c1);
-      const double c2 = cos(km * (zp + h));
-      rm1 = -(cof / nm * c1 * c2);
-      rm2 = -(dcof / nm * c1 * c2);
-      rm3 = cof * km / nm * s1 * c2;
-    }
-    re0 += rm1; re1 += rm2; re2 += rm3;
-    if (i > 2 && fabs(rm1) < eps && fabs(rm2) < eps && fabs(rm3) < eps) break;
-  }
 
   // IV. error-function image sums
   double e0 = 0.0, e1 = 0.0, e2 = 0.0;
@@ -917,14 +926,9 @@ HGD inline void d_linton(const FinState& st, double r, double zf, double zp, dou
     e2 = e2 - ef1 / (p4 * (sr1 * sr1)) * dsr1z + df1 / (p4 * sr1 * pa) * dsr1z + dsr2z / (p4 * (sr2 * sr2));
   }
 
-  // V. integral over [0, PA/2]
-  LintonPar lp{v, r, zf, zp, h};
-  const double q1 = d_aquad<0>(lp, 0.0, 0.0, 0, 0.0, pa / 2.0, eps, 1, st.status);
-  const double q2 = d_aquad<0>(lp, 0.0, 0.0, 0, 0.0, pa / 2.0, eps, 2, st.status);
-  const double q3 = d_aquad<0>(lp, 0.0, 0.0, 0, 0.0, pa / 2.0, eps, 3, st.status);
-  re0 = re0 - e0 - v / 2.0 / HG_PI * q1;
-  re1 = re1 - e1 + v / 2.0 / HG_PI * q2;
-  re2 = re2 - e2 - v / 2.0 / HG_PI * q3;
+  const double re0 = re[0] - e0 - v / 2.0 / HG_PI * q[0];
+  const double re1 = re[1] - e1 + v / 2.0 / HG_PI * q[1];
+  const double re2 = re[2] - e2 - v / 2.0 / HG_PI * q[2];
 
   double bj0, bj1, by0, by1;
   d_jy01b(wk * r, bj0, bj1, by0, by1);
@@ -934,6 +938,25 @@ HGD inline void d_linton(const FinState& st, double r, double zf, double zp, dou
   g[0] = -p4 * re0; g[1] = -p4 * im0;
   g[2] = -p4 * re1; g[3] = -p4 * im1;
   g[4] = -p4 * re2; g[5] = -p4 * im2;
+}
+
+HGD inline void d_linton(const FinState& st, double r, double zf, double zp, double g[6]) {
+  const double eps = SPD(1.e-6), wk = st.wk, h = st.h, a = d_linton_a(st);
+  const double czf = cosh(wk * (zf + h)), czp = cosh(wk * (zp + h)), szf = sinh(wk * (zf + h));
+  int flags = 0;
+  double re[3] = {0.0, 0.0, 0.0}, q[3];
+  for (int i = 1; i <= 20; ++i) {
+    double rm[3];
+    d_linton_term(st, i, a, r, zf, zp, czf, czp, szf, rm, flags);
+    for (int k = 0; k < 3; ++k) re[k] += rm[k];
+    if (d_linton_last(i, rm)) break;
+  }
+  // V. integrals over [0, PA/2]
+  LintonPar lp{st.v, r, zf, zp, h};
+  const double pa = a * h;
+  for (int k = 0; k < 3; ++k) q[k] = d_aquad<0>(lp, 0.0, 0.0, 0, 0.0, pa / 2.0, eps, k + 1, flags);
+  d_linton_rest(st, a, r, zf, zp, czf, czp, szf, re, q, g);
+  if (flags) hg_set_status(st.status, flags);
 }
 
 // FINGREEN3D_R dispatch (FinGreen3D.f90:160-226): the Green function minus
