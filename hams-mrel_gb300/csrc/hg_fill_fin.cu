@@ -6,6 +6,7 @@
 // separately rounded products the series reproduce the reference's
 // arithmetic.  The mixed form, whose matrices are single precision, uses the
 // instantiation of hg_fill_fin_fma.cu instead (same code, contracted).
+#define HG_NO_CONTRACTION 1
 #include "hg_fin_keys_impl.cuh"
 
 namespace hg {

@@ -50,6 +50,18 @@ __device__ __forceinline__ int key_bin(double rhp) {
   if (rhp < 0.5) return kKeyEps0 + min(5, max(0, (54 - key_terms(rhp)) / 8));
   return kKeyEig;
 }
+// Place of R inside its band, kKeySub steps: R sorted this finely, the lanes of
+// a warp sum Bessel series of about one length and on one side of the branches
+// at x = 9 and 18.
+constexpr int kKeySub = 256;
+__device__ __forceinline__ int key_sub(double rhp, int bin) {
+  double t;  // 0 .. 1 over the band (bands of eight terms: see key_terms)
+  if (bin == 0) t = rhp / 0.0005;
+  else if (bin < kKeyEps0) t = (1010.10 * rhp - 0.5) / 8.0 - (bin - kKeyPid0);
+  else if (bin < kKeyEig) t = (88.89 * rhp - 0.45) / 8.0 - (bin - kKeyEps0);
+  else t = 1.0 - 0.5 / rhp;
+  return bin * kKeySub + min(kKeySub - 1, max(0, (int)(t * kKeySub)));
+}
 // Rows (terms i = 2, 3, ...) a band's table holds: its longest series.
 inline int bin_rows(int b) {
   if (b < kKeyPid0) return 0;
@@ -106,14 +118,14 @@ __device__ __forceinline__ int bin_place(int* counters, int b) {
   return __shfl_sync(peers, base, leader) + __popc(peers & ((1u << lane) - 1u));
 }
 
-// Occupied R slots, counted by band and then placed at the bands' cursors.
+// Occupied R slots, counted by place in the order of R and then placed at its cursors.
 template <int FAST, bool SCATTER>
 __global__ void k_key_r(const unsigned long long* __restrict__ tabr, unsigned cap, double h, int* __restrict__ cursor,
                         int* __restrict__ slot2r, double* __restrict__ rval, int* __restrict__ rnt) {
   const unsigned s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= cap || tabr[s] == kKeyEmpty) return;
   const double rr = __longlong_as_double((long long)tabr[s]), rhp = fabs(rr / h);
-  const int at = bin_place(cursor, key_bin(rhp));
+  const int at = bin_place(cursor, key_sub(rhp, key_bin(rhp)));
   if (SCATTER) {
     slot2r[s] = at;
     rval[at] = rr;
@@ -406,6 +418,10 @@ k_key_series(FinState s, KeySegs g, int k0, int k1, const int4* __restrict__ key
   F[6 * (size_t)u + 2 * q] = limes_pass<kSerThreads>(nt - 1, sq, sa);
 }
 
+inline unsigned series_blocks(int keys) {
+  return (unsigned)((((keys + 31) / 32) * 3 + kSerThreads / 32 - 1) / (kSerThreads / 32));
+}
+
 // The rest of EIGENE and PIDCOCK (d_series_eps) around the extrapolated sums,
 // and EIGEN (d_eigen) whole: one key per thread.
 template <int FAST>
@@ -586,9 +602,10 @@ cudaError_t keys_build_body(cudaStream_t st, FinKeys& K, const double* rec, cons
                             double h, int near_only, const int* zsrc, const int* zfld) {
   KeyScratch sc;
   const dim3 g((tn + 127) / 128, n);
-  int* cnt = nullptr;  // pair counter, then the cursors of the bands
-  KE(sc.get(&cnt, 1 + 16));
-  KE(cudaMemsetAsync(cnt, 0, 17 * sizeof(int), st));
+  constexpr int kPlaces = kKeyBins * kKeySub;
+  int* cnt = nullptr;  // pair counter, then the cursors of the order of R
+  KE(sc.get(&cnt, 1 + kPlaces));
+  KE(cudaMemsetAsync(cnt, 0, (1 + kPlaces) * sizeof(int), st));
   K.np = tn * n;
   if (near_only) {
     k_key_pairs<FAST, false><<<g, 128, 0, st>>>(rec, fx, ldf, n, tn, h, 1, zsrc, zfld, nullptr, nullptr, 0, cnt, nullptr,
@@ -617,17 +634,21 @@ cudaError_t keys_build_body(cudaStream_t st, FinKeys& K, const double* rec, cons
                                              K.pidx, K.pkey);
   // distinct R by band
   const unsigned cb = (cap + 255) / 256;
-  int hc[16] = {};
+  std::vector<int> hc(kPlaces);
   k_key_r<FAST, false><<<cb, 256, 0, st>>>(tabr, cap, h, cnt + 1, nullptr, nullptr, nullptr);
-  KE(cudaMemcpyAsync(hc, cnt + 1, kKeyBins * sizeof(int), cudaMemcpyDeviceToHost, st));
+  KE(cudaMemcpyAsync(hc.data(), cnt + 1, kPlaces * sizeof(int), cudaMemcpyDeviceToHost, st));
   KE(cudaStreamSynchronize(st));
   int start[kKeyBins + 1] = {0};
-  for (int b = 0; b < kKeyBins; ++b) start[b + 1] = start[b] + hc[b];
-  K.nr = start[kKeyBins];
+  for (int q = 0; q < kPlaces; ++q) {
+    const int c = hc[q];
+    hc[q] = K.nr;
+    K.nr += c;
+    start[q / kKeySub + 1] = K.nr;
+  }
   KE(key_alloc(&K.rval, K.nr));
   KE(key_alloc(&K.rnt, K.nr));
   KE(key_alloc(&K.jy, K.nr));
-  KE(cudaMemcpyAsync(cnt + 1, start, kKeyBins * sizeof(int), cudaMemcpyHostToDevice, st));
+  KE(cudaMemcpyAsync(cnt + 1, hc.data(), kPlaces * sizeof(int), cudaMemcpyHostToDevice, st));
   k_key_r<FAST, true><<<cb, 256, 0, st>>>(tabr, cap, h, cnt + 1, slot2r, K.rval, K.rnt);
   // groups of R whose table fits the budget, and the keys in their order
   std::vector<int> gend;
@@ -753,17 +774,16 @@ cudaError_t fin_keys_fill(cudaStream_t st, FinKeys& K, const double* rec, const 
       }
       if (w.bin < kKeyEig) eig0 = w.k1;
     }
-    auto blocks = [](int keys) { return (unsigned)((((keys + 31) / 32) * 3 + kSerThreads / 32 - 1) / (kSerThreads / 32)); };
     if (pid_end > ka) {
       const size_t smem = (size_t)2 * (prows + 1) * kSerThreads * sizeof(double);
       KE(cudaFuncSetAttribute(k_key_series<FAST, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      k_key_series<FAST, true><<<blocks(pid_end - ka), kSerThreads, smem, st>>>(fs, g, ka, pid_end, K.keys, zt, kt, prows,
+      k_key_series<FAST, true><<<series_blocks(pid_end - ka), kSerThreads, smem, st>>>(fs, g, ka, pid_end, K.keys, zt, kt, prows,
                                                                                K.F);
     }
     if (eig0 > pid_end) {
       const size_t smem = (size_t)2 * (erows + 1) * kSerThreads * sizeof(double);
       KE(cudaFuncSetAttribute(k_key_series<FAST, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      k_key_series<FAST, false><<<blocks(eig0 - pid_end), kSerThreads, smem, st>>>(fs, g, pid_end, eig0, K.keys, zt, kt,
+      k_key_series<FAST, false><<<series_blocks(eig0 - pid_end), kSerThreads, smem, st>>>(fs, g, pid_end, eig0, K.keys, zt, kt,
                                                                                   erows, K.F);
     }
     k_key_finish<FAST><<<(kb - ka + 127) / 128, 128, 0, st>>>(fs, g, ka, kb, pid_end, eig0, K.keys, K.rval, zlev, K.jy, zt,

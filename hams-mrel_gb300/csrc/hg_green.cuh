@@ -227,16 +227,21 @@ HGD inline void inf_green(double xq, double yq, double zq, double xp, double yp,
 // ===================================================================
 // Finite depth: special functions (FinGrnExtSubs.f90)
 // ===================================================================
-// x**k for an integer k by binary powering, the evaluation order a Fortran
-// compiler uses for an integer exponent.
-HGD inline double powi(double x, int m) {
-  unsigned n = (unsigned)m;
-  double y = (n % 2u) ? x : 1.0;
-  while (n >>= 1) {
-    x = x * x;
-    if (n % 2u) y = y * x;
-  }
-  return y;
+// p[k] = x**k, k = 1 .. 12, each by binary powering (the evaluation order a
+// Fortran compiler uses for an integer exponent), the squares shared.
+HGD inline void powers12(double x, double p[13]) {
+  p[1] = x;
+  p[2] = x * x;
+  p[4] = p[2] * p[2];
+  p[8] = p[4] * p[4];
+  p[3] = p[1] * p[2];
+  p[5] = p[1] * p[4];
+  p[6] = p[2] * p[4];
+  p[7] = p[3] * p[4];
+  p[9] = p[1] * p[8];
+  p[10] = p[2] * p[8];
+  p[11] = p[3] * p[8];
+  p[12] = p[4] * p[8];
 }
 HGD inline double d_error(double x) {  // ERROR :62-93
   const double x2 = x * x;
@@ -365,25 +370,30 @@ HGD inline double div_small(double a, double d, double rd) {
 }
 
 // fabs(num / den) < 1e-15 as the rounded division decides it.  The high words
-// of |num| and of 1e-15 |den| decide it unless they agree to about one part
-// in 2^19; only then is the division made.
+// of two positive doubles differ by 2^20 times the logarithm (base 2) of their
+// ratio, to 0.09 either way; 1e-15 is 2^-49.83, so outside a window around it
+// they decide, and only inside is the division made.
 HGD inline int hi_word(double x) {
 #ifdef __CUDA_ARCH__
-  return __double2hiint(x);
+  return __double2hiint(x) & 0x7fffffff;
 #else
   long long b;
   memcpy(&b, &x, sizeof b);
-  return (int)(b >> 32);
+  return (int)(b >> 32) & 0x7fffffff;
 #endif
 }
+// 1: below, 0: not below, -1: undecided; slack (in 2^-20) widens the window for
+// a num known only to that relative accuracy.
+HGD inline int ratio_guess(double num, double den, int slack) {
+  const int hn = hi_word(num), hd = hi_word(den), g = hd - hn;
+  if (hn >= 0x7ff00000 || hd >= 0x7ff00000 || hd < (60 << 20)) return -1;
+  if (g > 52533657 + slack) return 1;   // 50.1 2^20
+  if (g < 52009369 - slack) return 0;   // 49.6 2^20
+  return -1;
+}
 HGD inline bool ratio_below(double num, double den) {
-  const double a = fabs(num), t = 1.0e-15 * fabs(den);
-  const int ha = hi_word(a), ht = hi_word(t);
-  if (ht < 0x7ff00000) {
-    if (ha + 1 < ht) return true;
-    if (ha > ht + 1) return false;
-  }
-  return fabs(num / den) < 1.0e-15;
+  const int t = ratio_guess(num, den, 0);
+  return t < 0 ? fabs(num / den) < 1.0e-15 : t != 0;
 }
 
 // IK01A :538-640, returning K0 and K1.
@@ -392,17 +402,18 @@ HGD inline void d_ik01a(double x, double& bk0, double& bk1) {
   const double x2 = x * x;
   double bi0, bi1;
   if (x <= 18.0) {
+    const double xq = 0.25 * x2;  // the factor 0.25 is exact wherever it is applied
     bi0 = 1.0;
     double r = 1.0;
     for (int k = 1; k <= 50; ++k) {
-      r = div_small(0.25 * r * x2, c_kk[k], c_rcp_kk[k]);
+      r = div_small(r * xq, c_kk[k], c_rcp_kk[k]);
       bi0 += r;
       if (ratio_below(r, bi0)) break;
     }
     bi1 = 1.0;
     r = 1.0;
     for (int k = 1; k <= 50; ++k) {
-      r = div_small(0.25 * r * x2, c_kk1[k], c_rcp_kk1[k]);
+      r = div_small(r * xq, c_kk1[k], c_rcp_kk1[k]);
       bi1 += r;
       if (ratio_below(r, bi1)) break;
     }
@@ -419,14 +430,16 @@ HGD inline void d_ik01a(double x, double& bk0, double& bk1) {
     if (x >= 35.0) k0 = 9;
     if (x >= 50.0) k0 = 7;
     const double ca = exp(x) / sqrt(2.0 * HG_PI * x), xr = 1.0 / x;
+    double p[13];
+    powers12(xr, p);
     double s0 = 1.0, s1 = 1.0;
     for (int k = 1; k <= 12; ++k) {
       if (k > k0) break;
-      s0 += A[k - 1] * powi(xr, k);
+      s0 += A[k - 1] * p[k];
     }
     for (int k = 1; k <= 12; ++k) {
       if (k > k0) break;
-      s1 += B[k - 1] * powi(xr, k);
+      s1 += B[k - 1] * p[k];
     }
     bi0 = ca * s0;
     bi1 = ca * s1;
@@ -434,10 +447,20 @@ HGD inline void d_ik01a(double x, double& bk0, double& bk1) {
   if (x <= 9.0) {
     const double ct = -(log(x / 2.0) + 0.5772156649015329);
     double k0v = 0.0, r = 1.0, ww = 0.0;
+    const double xq = 0.25 * x2;
     for (int k = 1; k <= 50; ++k) {
-      r = div_small(0.25 * r, c_kk[k], c_rcp_kk[k]) * x2;
+      r = div_small(r, c_kk[k], c_rcp_kk[k]) * xq;
+#ifdef HG_NO_CONTRACTION
+      // the sum grew by the term to within half a unit, a ninth of the threshold: the term decides
+      const double term = r * (c_harm[k] + ct);
+      k0v += term;
+      int t = ratio_guess(term, k0v, 524288);
+      if (t < 0) t = ratio_below(k0v - ww, k0v);
+      if (t) break;
+#else  // the product of one use, so that it is fused into the sum
       k0v += r * (c_harm[k] + ct);
       if (ratio_below(k0v - ww, k0v)) break;
+#endif
       ww = k0v;
     }
     bk0 = k0v + ct;
@@ -445,8 +468,10 @@ HGD inline void d_ik01a(double x, double& bk0, double& bk1) {
     const double A1[8] = {0.125, 0.2109375, 1.0986328125, 1.1775970458984e01, 2.1461706161499e02,
                           5.9511522710323e03, 2.3347645606175e05, 1.2312234987631e07};
     const double xr2 = 1.0 / x2;
+    double p[13];
+    powers12(xr2, p);
     double s = 1.0;
-    for (int k = 0; k < 8; ++k) s += A1[k] * powi(xr2, k + 1);
+    for (int k = 0; k < 8; ++k) s += A1[k] * p[k + 1];
     bk0 = 0.5 / x * s / bi0;
   }
   bk1 = (1.0 / x - bi1 * bk0) / bi0;
