@@ -509,24 +509,75 @@ cudaError_t panel(cudaStream_t st, bool use_cluster, int n, typename cx<R>::T* A
   return cudaGetLastError();
 }
 
+// C -= A B for an inner dimension of at most 16 (the update between 16-wide
+// complex128 panels) on the FP64 pipes: a 16 x 16 tile of C per CTA of 64
+// threads, operands staged once.  With two FP64 operations a clock and SM the
+// product is bound by that pipe, and small tiles are what spreads it evenly
+// over the SMs.
+constexpr int kZupdT = 16, kZupdK = 16;
+__global__ void __launch_bounds__(64)
+k_zupdate(int m, int n, int k, const double2* __restrict__ A, long lda, const double2* __restrict__ B, long ldb,
+          double2* __restrict__ C, long ldc) {
+  __shared__ double2 as[kZupdK][kZupdT], bs[kZupdK][kZupdT + 1];
+  const int m0 = blockIdx.x * kZupdT, n0 = blockIdx.y * kZupdT;
+  const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3;  // rows tx, tx + 8; columns ty, ty + 8
+  double2 c[2][2];
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int r = m0 + tx + 8 * i, q = n0 + ty + 8 * j;
+      c[i][j] = (r < m && q < n) ? C[r + (long)q * ldc] : make_double2(0.0, 0.0);
+    }
+#pragma unroll
+  for (int e = threadIdx.x; e < kZupdK * kZupdT; e += 64) {
+    const int r = e % kZupdT, l = e / kZupdT;
+    as[l][r] = (l < k && m0 + r < m) ? A[m0 + r + (long)l * lda] : make_double2(0.0, 0.0);
+    bs[r][l] = (r < k && n0 + l < n) ? B[r + (long)(n0 + l) * ldb] : make_double2(0.0, 0.0);
+  }
+  __syncthreads();
+#pragma unroll 4
+  for (int l = 0; l < kZupdK; ++l) {
+    const double2 a[2] = {as[l][tx], as[l][tx + 8]}, b[2] = {bs[l][ty], bs[l][ty + 8]};
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        c[i][j].x = fma(a[i].y, b[j].y, fma(-a[i].x, b[j].x, c[i][j].x));
+        c[i][j].y = fma(-a[i].y, b[j].x, fma(-a[i].x, b[j].y, c[i][j].y));
+      }
+  }
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int r = m0 + tx + 8 * i, q = n0 + ty + 8 * j;
+      if (r < m && q < n) C[r + (long)q * ldc] = c[i][j];
+    }
+}
+// Up to this many entries of C the update runs there, beyond it as sliced
+// tensor-core products.
+constexpr long kZupdMax = 400000;
+
 // Columns [c0, c1) of A through one level of right-looking blocking with
 // 32-wide panels (pivots applied only inside [c0, c1)).  With aux, the
 // update of the columns beyond the next panel runs on aux->side (see getrf).
-// Complex128 with zws (zgemm_tc_work_bytes of the update): each update is one
-// sliced product on the tensor cores, on st.
+// Complex128 with zws (zgemm_tc_work_bytes of the update) or narrow: 16-wide
+// panels, each update one product on st, on the FP64 pipes or, large and with
+// zws, sliced on the tensor cores.
 template <typename R>
 cudaError_t factor_columns(cudaStream_t st, bool use_cluster, int n, typename cx<R>::T* A, long lda, int c0, int c1,
                            int* ipiv, int* info, int* perm = nullptr, const LuAux* aux = nullptr, void* zws = nullptr,
-                           size_t zws_bytes = 0) {
+                           size_t zws_bytes = 0, bool narrow = false) {
   typedef typename cx<R>::T T;
   T mone, one;
   mone.x = -1; mone.y = 0; one.x = 1; one.y = 0;
   bool side_pending = false;
   cudaError_t e = cudaSuccess;
-  // complex128 on the tensor cores: 16-wide panels (their FP64 rank-1
-  // updates, the panel's bound, are half those of 32-wide ones; the updates
-  // between panels are tensor-core products either way)
-  const int nbp = (sizeof(R) == 8 && zws) ? kNB / 2 : kNB;
+  // 16-wide complex128 panels: their FP64 rank-1 updates, the panel's bound,
+  // are half those of 32-wide ones
+  const bool zn = sizeof(R) == 8 && (zws || narrow);
+  const int nbp = zn ? kNB / 2 : kNB;
   for (int k = c0; k < c1; k += nbp) {
     const int jb = (c1 - k < nbp) ? c1 - k : nbp;
     e = panel<R>(st, use_cluster, n, A, lda, k, jb, ipiv, info);
@@ -545,7 +596,11 @@ cudaError_t factor_columns(cudaStream_t st, bool use_cluster, int n, typename cx
     const T* L21 = A + (k + jb) + (long)k * lda;
     const T* U12 = A + k + (long)(k + jb) * lda;
     T* A22 = A + (k + jb) + (long)(k + jb) * lda;
-    if (sizeof(R) == 8 && zws) {
+    if (zn && (!zws || (long)m * rest <= kZupdMax)) {
+      k_zupdate<<<dim3((m + kZupdT - 1) / kZupdT, (rest + kZupdT - 1) / kZupdT), 64, 0, st>>>(
+          m, rest, jb, reinterpret_cast<const double2*>(L21), lda, reinterpret_cast<const double2*>(U12), lda,
+          reinterpret_cast<double2*>(A22), lda);
+    } else if (zn) {
       e = zgemm_tc(st, m, rest, jb, reinterpret_cast<const double2*>(L21), lda, reinterpret_cast<const double2*>(U12), lda,
                    reinterpret_cast<double2*>(A22), lda, zws, zws_bytes, info);
       if (e != cudaSuccess) return e;
@@ -715,7 +770,12 @@ cudaError_t getrf(cudaStream_t st, int n, typename cx<R>::T* A, long lda, int* i
   const bool use_cluster = panel_cluster_supported<R>(n);
   const bool tc = sizeof(R) == 4 && tc_passes != 0 && n >= kTcMinN && work &&
                   work_bytes >= lu_work_bytes(n, tc_passes) && cgemm_tc_supported();
-  if (!tc) return factor_columns<R>(st, use_cluster, n, A, lda, 0, n, ipiv, info, nullptr, aux);
+  if (!tc) {
+    // Complex128 below the tensor cores' order: 16-wide panels and their own update kernel
+    const bool narrow = sizeof(R) == 8 && n < kTcMinN && panel_cluster_supported<R>(n, kNB / 2);
+    return factor_columns<R>(st, narrow || use_cluster, n, A, lda, 0, n, ipiv, info, nullptr, narrow ? nullptr : aux,
+                             nullptr, 0, narrow);
+  }
   // Two levels: 256-wide outer panels factorised by the 32-wide loop above,
   // then U12 = L11^-1 A12 and the tensor-core update A22 -= L21 U12.  U12
   // is formed as A12 - (I - L11^-1) A12 on the tensor cores too, with

@@ -25,6 +25,7 @@
 #include <cooperative_groups.h>
 
 #include "hg_linalg.cuh"
+#include "hg_rcp.cuh"
 #include "hg_tma.cuh"
 
 namespace cg = cooperative_groups;
@@ -410,7 +411,7 @@ k_getf2_cluster_push(float2* __restrict__ P, long lda, int m, int jb, int rpc, i
 // 16 bulk copies, a bounded mbarrier wait; no cluster barrier and no remote
 // loads per column) with the arithmetic of k_getf2_cluster<double>.  The
 // message also carries the reciprocal of the candidate's entry in column jj,
-// formed once by its sender (three FP64 divisions).  Reuse of the two message
+// formed once by its sender.  Reuse of the two message
 // slots is safe for the reasons given above.
 constexpr int kPanelNBZ = 16;
 struct __align__(16) PanelMsgZ {
@@ -437,10 +438,27 @@ __device__ __forceinline__ void warp_best_z(double& v, int& idx) {
   v = (km == 0ull) ? -1.0 : __longlong_as_double((long long)(km - 1ull));
 }
 
+// 1 / a by Smith's scaling, the reciprocals on the integer pipes (hg_rcp.cuh):
+// one thread forms it while the cluster waits, and three dependent FP64
+// divisions are most of a microsecond there.
+__device__ __forceinline__ double2 c_recip_z(double2 a) {
+  const bool re = fabs(a.x) >= fabs(a.y);
+  const double big = re ? a.x : a.y, small = re ? a.y : a.x;
+  const double q = small * rcp_any(big), d = rcp_any(fma(small, q, big));
+  return re ? make_double2(d, -q * d) : make_double2(q * d, -d);
+}
+
+// G column groups share the panel's rows: thread t works on row t mod (512 /
+// G) and columns t / (512 / G), + G, + 2 G, ...  The update is bound by the
+// FP64 pipe of the scheduler a warp sits on (one warp instruction takes 64
+// cycles there), so a short panel, whose rows would fill only a few warps,
+// spreads its columns over the others.  The thread that updates column jj + 1
+// takes its entry's |re| + |im| for the next pivot search from the register.
+template <int G>
 __global__ void __launch_bounds__(kClusterThreads, 1)
 k_getf2_cluster_push_z(double2* __restrict__ P, long lda, int m, int jb, int rpc, int* __restrict__ ipiv, int k0,
                        int* __restrict__ info) {
-  constexpr int kWarps = kClusterThreads / 32;
+  constexpr int kWarps = kClusterThreads / 32, RT = kClusterThreads / G, NC = kPanelNBZ / G;
   cg::cluster_group cluster = cg::this_cluster();
   const int rank = (int)cluster.block_rank();
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -452,6 +470,7 @@ k_getf2_cluster_push_z(double2* __restrict__ P, long lda, int m, int jb, int rpc
   __shared__ int red_i[kWarps];
   __shared__ int s_bad;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tr = tid % RT, g = tid / RT;
   const int r0 = rank * rpc;
   const int rl = max(0, min(rpc, m - r0));
   constexpr uint32_t kMsgBytes = sizeof(PanelMsgZ);
@@ -467,22 +486,23 @@ k_getf2_cluster_push_z(double2* __restrict__ P, long lda, int m, int jb, int rpc
     mbar_expect_tx(&mbar[0], kClusterCTAs * kMsgBytes);
     if (jb > 1) mbar_expect_tx(&mbar[1], kClusterCTAs * kMsgBytes);
   }
-  cluster.sync();  // barriers initialised and armed everywhere before any copy
+  cluster.sync();  // barriers initialised and armed everywhere before any copy, tiles loaded
+
+  // this thread's candidate for the current column (rows >= jj): |re| + |im|, first row on ties
+  double v = -1.0;
+  int idx = INT_MAX;
+  auto consider = [&](double2 a, int gr) {
+    const double av = fabs(a.x) + fabs(a.y);
+    if (av > v || (av == v && gr < idx)) { v = av; idx = gr; }
+  };
+  if (g == 0)
+    for (int r = tr; r < rl; r += RT) consider(tile[r], r0 + r);
 
   bool bad = false;
   for (int jj = 0; jj < jb; ++jj) {
     const int q = jj & 1;
     const int oj = jj / rpc, lj = jj - oj * rpc;
-    // (a) this CTA's candidate for column jj (rows >= jj): |re| + |im|, first row on ties
-    double v = -1.0;
-    int idx = INT_MAX;
-    for (int r = tid; r < rl; r += blockDim.x) {
-      if (r0 + r >= jj) {
-        const double2 a = tile[jj * rpc + r];
-        const double av = fabs(a.x) + fabs(a.y);
-        if (av > v || (av == v && r0 + r < idx)) { v = av; idx = r0 + r; }
-      }
-    }
+    // (a) this CTA's candidate
     warp_best_z(v, idx);
     if (lane == 0) { red_v[warp] = v; red_i[warp] = idx; }
     __syncthreads();  // also orders every thread's column jj - 1 updates before the copies below
@@ -495,7 +515,7 @@ k_getf2_cluster_push_z(double2* __restrict__ P, long lda, int m, int jb, int rpc
       if (lane == 0) {
         msg.val = v;
         msg.idx = idx;
-        if (v > 0.0) msg.rcp = c_recip(tile[jj * rpc + (idx - r0)]);
+        if (v > 0.0) msg.rcp = c_recip_z(tile[jj * rpc + (idx - r0)]);
       }
       if (lane < jb) {
         if (idx != INT_MAX) msg.cand[lane] = tile[lane * rpc + (idx - r0)];
@@ -530,33 +550,43 @@ k_getf2_cluster_push_z(double2* __restrict__ P, long lda, int m, int jb, int rpc
       if (!(pmax > 0.0) && *info == 0) *info = k0 + jj + 1;
     }
     // (e) row jj becomes the pivot row; the owner of row p takes old row jj
+    v = -1.0;
+    idx = INT_MAX;
+    const double2 rp = pmax > 0.0 ? recv[q][op].rcp : make_double2(0.0, 0.0);
+    double2 x0 = make_double2(0.0, 0.0);
+    if (G > 1) {  // column jj is read by every group and rewritten by one
+      if (tr < rl) x0 = tile[jj * rpc + tr];
+      __syncthreads();
+    }
     if (swap && rank == oj && tid < jb) tile[tid * rpc + lj] = prow[tid];
-    if (pmax > 0.0) {
-      const double2 rp = recv[q][op].rcp;
-      for (int r = tid; r < rl; r += blockDim.x) {
-        const int gr = r0 + r;
-        if (gr <= jj) continue;
-        if (swap && gr == p)
-          for (int c = 0; c < jb; ++c) tile[c * rpc + r] = jrow[c];
-        const double2 l = c_mul(tile[jj * rpc + r], rp);
-        tile[jj * rpc + r] = l;
+    for (int r = tr; r < rl; r += RT) {
+      const int gr = r0 + r;
+      if (gr <= jj) continue;
+      if (!(pmax > 0.0)) {  // a zero column: nothing to eliminate
+        if (jj + 1 < jb && (jj + 1) % G == g) consider(tile[(jj + 1) * rpc + r], gr);
+        continue;
+      }
+      const bool isp = swap && gr == p;
+      const double2 l = c_mul(isp ? jrow[jj] : (G > 1 ? x0 : tile[jj * rpc + r]), rp);
+      double2 a[NC];
 #pragma unroll
-        for (int c0 = 0; c0 < kPanelNBZ; c0 += 8) {
-          if (c0 + 8 <= jj + 1 || c0 >= jb) continue;
-          double2 u[8], a[8];
+      for (int t = 0; t < NC; ++t) {
+        const int c = g + t * G;
+        if (c > jj && c < jb) a[t] = isp ? jrow[c] : tile[c * rpc + r];
+      }
 #pragma unroll
-          for (int t = 0; t < 8; ++t) {
-            const int c = c0 + t;
-            if (c > jj && c < jb) {
-              u[t] = prow[c];
-              a[t] = tile[c * rpc + r];
-            }
-          }
-#pragma unroll
-          for (int t = 0; t < 8; ++t) {
-            const int c = c0 + t;
-            if (c > jj && c < jb) tile[c * rpc + r] = c_sub(a[t], c_mul(l, u[t]));
-          }
+      for (int t = 0; t < NC; ++t) {
+        const int c = g + t * G;
+        if (c > jj && c < jb) {
+          const double2 u = prow[c];
+          a[t].x = fma(l.y, u.y, fma(-l.x, u.x, a[t].x));
+          a[t].y = fma(-l.y, u.x, fma(-l.x, u.y, a[t].y));
+          tile[c * rpc + r] = a[t];
+          if (c == jj + 1) consider(a[t], gr);
+        } else if (c == jj) {
+          tile[c * rpc + r] = l;
+        } else if (c < jj && isp) {
+          tile[c * rpc + r] = jrow[c];
         }
       }
     }
@@ -848,10 +878,15 @@ cudaError_t panel_cluster<double>(cudaStream_t st, double2* P, long lda, int m, 
   const size_t smem = (size_t)rpc * jb * sizeof(double2);
   if (jb > kPanelNBZ || smem > (size_t)(kPanelSmemMax - kPushStaticSmem))
     return panel_cluster_smem<double>(st, P, lda, m, jb, ipiv, k0, info);
-  cudaError_t e = cudaFuncSetAttribute(k_getf2_cluster_push_z, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  // column groups: as many as leave every row of a CTA a thread
+  auto kern = k_getf2_cluster_push_z<1>;
+  if (rpc <= 32) kern = k_getf2_cluster_push_z<16>;
+  else if (rpc <= 64) kern = k_getf2_cluster_push_z<8>;
+  else if (rpc <= 128) kern = k_getf2_cluster_push_z<4>;
+  else if (rpc <= 256) kern = k_getf2_cluster_push_z<2>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_getf2_cluster_push_z, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             kPanelSmemMax - kPushStaticSmem);
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kPanelSmemMax - kPushStaticSmem);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(kClusterCTAs, 1, 1);
@@ -865,7 +900,7 @@ cudaError_t panel_cluster<double>(cudaStream_t st, double2* P, long lda, int m, 
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k_getf2_cluster_push_z, P, lda, m, jb, rpc, ipiv, k0, info);
+  return cudaLaunchKernelEx(&cfg, kern, P, lda, m, jb, rpc, ipiv, k0, info);
 }
 
 

@@ -94,4 +94,26 @@ HG_HD double rcp_rn(double x) {
   return rcp_from_seed(b, rcp_seed(0x3f800000u | ((uint32_t)(b >> 29) & 0x7fffffu)));
 }
 
+// 1 / x for any x.
+HG_HD double rcp_any(double x) { return rcp_in_range(rcp_bits(x)) ? rcp_rn(x) : 1.0 / x; }
+
+#ifdef __CUDACC__
+// 1 / sqrt(x), x >= 0, within about a unit of the last place: a single-precision
+// seed (22 bits) and one third-order step in FP64, five FP64 operations against
+// about twenty for 1.0 / sqrt(x).  Outside the seed's range the latter.
+__device__ __forceinline__ double rsqrt_near(double x) {
+#ifdef __CUDA_ARCH__
+  const uint32_t hi = (uint32_t)(rcp_bits(x) >> 32);
+  if (hi - 0x38500000u >= 0x0f500000u) return 1.0 / sqrt(x);  // below 2^-122, above 2^122, NaN
+  const float f = (float)x;
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(f));
+  const double y = (double)r, e = fma(-x * y, y, 1.0);
+  return fma(fma(e, 0.375, 0.5) * e, y, y);
+#else
+  return 1.0;
+#endif
+}
+#endif
+
 }  // namespace hg
