@@ -319,7 +319,7 @@ k_green_fill_mixed(const double* __restrict__ rec, const double* __restrict__ fx
     if (flag) {
       if (mixed_near(d2f, fl2)) {
         double s64, e0, e1, e2;
-        newman_pair(tile + jj * PR_SIZE, xp, yp, zp, s64, e0, e1, e2);
+        newman_pair_ref(tile + jj * PR_SIZE, xp, yp, zp, s64, e0, e1, e2);
         sij = (float)s64; d0 = (float)e0; d1 = (float)e1; d2 = (float)e2;
       } else if (d2f <= 0.0064f * fl2) {
         newman_pair_f(pfs[jj], xpf - px[4], ypf - px[5], zpf - px[6], sij, d0, d1, d2);
@@ -420,7 +420,7 @@ k_green_fill_mixed_near(const double* __restrict__ rec, const double* __restrict
     const float dxf = (float)(pr[PR_XQ] - ox) - xpf, dyf = (float)(pr[PR_XQ + 1] - oy) - ypf, zqf = (float)pr[PR_XQ + 2];
     const float dzf = zpf - zqf;
     double s64, e0, e1, e2;
-    newman_pair(pr, xp, yp, zp, s64, e0, e1, e2);
+    newman_pair_ref(pr, xp, yp, zp, s64, e0, e1, e2);
     const float sij = (float)s64, d0 = (float)e0, d1 = (float)e1, d2 = (float)e2;
     float2 g[4];
     inf_green_f(dxf, dyf, zpf + zqf, dzf, vf, 1, g);

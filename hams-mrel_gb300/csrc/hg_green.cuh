@@ -1,11 +1,11 @@
 // Device-side free-surface Green functions and Newman panel integrals.
 //
 // Deep water: the Wu-Noblesse global approximation used by HAMS-MREL
-// (src/InfGreen_Appr.f90:104-872).  The GPU form evaluates exp(vv),
-// exp(-dd) and log(dd-vv) once per pair and shares one sincos between each
-// J/Y Bessel pair: the reference's BesselY0/Y1 (:674-760) use the same
-// modulus and phase polynomials as BesselJ0/J1 (:583-671), so
-// Y = f*sin(theta)/sqrt(x) and J = f*cos(theta)/sqrt(x) come from one call.
+// (src/InfGreen_Appr.f90:104-872).  exp(vv), exp(-dd) and log(dd-vv) are
+// evaluated once per pair, and each J/Y Bessel pair shares one sincos: the
+// reference's BesselY0/Y1 (:674-760) use the same modulus and phase
+// polynomials as BesselJ0/J1 (:583-671), so Y = f*sin(theta)/sqrt(x) and
+// J = f*cos(theta)/sqrt(x) come from one call.
 //
 // Finite depth: the region-decomposed Green function of src/FinGreen3D.f90
 // (Linton / Pidcock / eigenfunction series with Wynn's epsilon algorithm),
@@ -17,6 +17,7 @@
 #pragma once
 #include <string.h>
 #include "hg_common.cuh"
+#include "hg_rcp.cuh"
 
 #ifdef __CUDACC__
 #define HGD __host__ __device__
@@ -36,8 +37,21 @@ namespace hg {
 // Newman (1986) closed-form integral of 1/r and grad(1/r) over a flat
 // panel, SingularIntgr.f90:44-244 (triangles) and :252-445 (quads).
 // pr = 36-double source-panel record (hg_common.cuh).
+//
+// GB300's FP64 pipe (two operations a clock and SM) bounds every caller, so
+// the work is arranged to spend few of them: vertex terms are formed once and
+// shared by the two edges that meet there, distances come from one
+// reciprocal square root, 1 / l and 1 / (s - l) run on the integer pipes
+// (hg_rcp.cuh), and the edges' angles are added as the argument of one complex
+// product: one atan2 instead of four, its multiple of 2 pi taken from the four
+// single-precision angles.
+//
+// newman_pair is the form of the complex128 matrices; newman_pair_ref, in the
+// reference's order of operations, that of entries rounded to single precision,
+// where a last bit of the double now and then moves the stored value by one
+// unit (outputs by up to 2e-8 near an irregular frequency).
 // ===================================================================
-HGD inline void newman_pair(const double* __restrict__ pr, double xf0, double xf1,
+__device__ __forceinline__ void newman_pair_ref(const double* __restrict__ pr, double xf0, double xf1,
                                             double xf2, double& sij, double& d0, double& d1,
                                             double& d2) {
   const double p0 = xf0 - pr[PR_PO], p1 = xf1 - pr[PR_PO + 1], p2 = xf2 - pr[PR_PO + 2];
@@ -85,124 +99,189 @@ HGD inline void newman_pair(const double* __restrict__ pr, double xf0, double xf
   d2 = sg * (pr[PR_UI + 2] * sxt + pr[PR_UJ + 2] * syt + pr[PR_UK + 2] * szt);
 }
 
+// The angles' sum edge by edge (x, y, z in the panel's frame).
+static __device__ __noinline__ double newman_angles(const double* __restrict__ pr, double x, double y, double z) {
+  const int nv = (int)pr[PR_NCN];
+  double szt = 0.0;
+  for (int e = 0; e < nv; ++e) {
+    const int nx = (e + 1 == nv) ? 0 : e + 1;
+    if (nv == 4 && fabs(pr[PR_L + e]) < 1.0e-8) continue;
+    const double dx = pr[PR_KSI + e] - x, dy = pr[PR_ETA + e] - y, ex = pr[PR_KSI + nx] - x, ey = pr[PR_ETA + nx] - y;
+    const double dksi = pr[PR_KSI + nx] - pr[PR_KSI + e], deta = pr[PR_ETA + nx] - pr[PR_ETA + e], z2 = z * z;
+    const double b1 = deta * (dx * dx + z2) - dksi * dx * dy, a1 = sqrt(dx * dx + dy * dy + z2) * z * dksi;
+    const double b2 = deta * (ex * ex + z2) - dksi * ex * ey, a2 = sqrt(ex * ex + ey * ey + z2) * z * dksi;
+    szt += atan2(b1 * a2 - b2 * a1, a1 * a2 + b1 * b2);
+  }
+  return szt;
+}
+
+__device__ __forceinline__ void newman_pair(const double* __restrict__ pr, double xf0, double xf1, double xf2,
+                                            double& sij, double& d0, double& d1, double& d2) {
+  const double p0 = xf0 - pr[PR_PO], p1 = xf1 - pr[PR_PO + 1], p2 = xf2 - pr[PR_PO + 2];
+  const double x = fma(pr[PR_UI + 2], p2, fma(pr[PR_UI + 1], p1, pr[PR_UI] * p0));
+  const double y = fma(pr[PR_UJ + 2], p2, fma(pr[PR_UJ + 1], p1, pr[PR_UJ] * p0));
+  const double z = fma(pr[PR_UK + 2], p2, fma(pr[PR_UK + 1], p1, pr[PR_UK] * p0));
+  const int nv = (int)pr[PR_NCN];
+  const bool tri = (nv == 3);
+  const bool flat = fabs(z) < 1.0e-6;  // in the panel's plane: no angle terms
+  const double z2 = z * z;
+  // vertex terms: offset, p = dx^2 + z^2, q = dx dy, distance r
+  double dx = pr[PR_KSI] - x, dy = pr[PR_ETA] - y;
+  double va = fma(dx, dx, z2), vq = dx * dy, vr = fma(dy, dy, va);
+  vr = vr > 0.0 ? vr * rsqrt_near(vr) : 0.0;
+  const double fdx = dx, fdy = dy, fa = va, fq = vq, fr = vr;
+  double st = 0.0, sxt = 0.0, syt = 0.0, szt = 0.0;
+  double zr = 1.0, zi = 0.0;        // product of the edges' complex numbers
+  float turns = 0.f;                // sum of their angles, single precision
+  bool plain = false;               // a factor out of the product's safe range: add the angles one by one
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    if (e >= nv) break;
+    const int nx = (e + 1 == nv) ? 0 : e + 1;
+    double ex, ey, wa, wq, wr;
+    if (nx == 0) {
+      ex = fdx; ey = fdy; wa = fa; wq = fq; wr = fr;
+    } else {
+      ex = pr[PR_KSI + nx] - x;
+      ey = pr[PR_ETA + nx] - y;
+      wa = fma(ex, ex, z2);
+      wq = ex * ey;
+      wr = fma(ey, ey, wa);
+      wr = wr > 0.0 ? wr * rsqrt_near(wr) : 0.0;
+    }
+    const double l = pr[PR_L + e];
+    if (tri || !(fabs(l) < 1.0e-8)) {
+      const double dksi = pr[PR_KSI + nx] - pr[PR_KSI + e], deta = pr[PR_ETA + nx] - pr[PR_ETA + e];
+      if (!flat) {
+        const double zd = z * dksi, a1 = vr * zd, a2 = wr * zd;
+        const double b1 = fma(deta, va, -(dksi * vq)), b2 = fma(deta, wa, -(dksi * wq));
+        const double im = fma(b1, a2, -(b2 * a1)), re = fma(a1, a2, b1 * b2);
+        const float fi = (float)im, fre = (float)re, fm = fmaxf(fabsf(fi), fabsf(fre));
+        plain = plain || !(fm > 1e-30f && fm < 1e30f);
+        turns += atan2f(fi, fre);
+        const double t = fma(zr, re, -(zi * im));
+        zi = fma(zr, im, zi * re);
+        zr = t;
+      }
+      const double s = vr + wr, gap = s - l;
+      if (!(fabs(gap) < 1.0e-6)) {
+        const double lg = log((s + l) * rcp_any(gap)) * rcp_any(l);
+        sxt = fma(-deta, lg, sxt);
+        syt = fma(dksi, lg, syt);
+        st = fma(fma(dksi, dy, -(deta * dx)), lg, st);  // deta (x - ksi) - dksi (y - eta)
+      }
+    }
+    dx = ex; dy = ey; va = wa; vq = wq; vr = wr;
+  }
+  if (!flat) {
+    if (!plain) {
+      szt = atan2(zi, zr);
+      szt = fma(rintf((turns - (float)szt) * 0.15915494f), 2.0 * HG_PI, szt);
+    } else {
+      szt = newman_angles(pr, x, y, z);
+    }
+  }
+  const double sg = tri ? 1.0 : -1.0;
+  sij = sg * fma(-z, szt, st);
+  d0 = sg * fma(pr[PR_UK], szt, fma(pr[PR_UJ], syt, pr[PR_UI] * sxt));
+  d1 = sg * fma(pr[PR_UK + 1], szt, fma(pr[PR_UJ + 1], syt, pr[PR_UI + 1] * sxt));
+  d2 = sg * fma(pr[PR_UK + 2], szt, fma(pr[PR_UJ + 2], syt, pr[PR_UI + 2] * sxt));
+}
+
 // ===================================================================
-// Deep water
+// Deep water.  As above FP64 operations are what counts: Horner steps are
+// fused, the nine divisions left of some thirty-five are reciprocals on the
+// integer pipes, and the distances' square roots come with their reciprocals
+// (measured at 6048 panels: see k_green_fill).
 // ===================================================================
-HGD inline double poly_a(double t) {
-  double g = (21859.0 + -4838.6 * t) * t;
-  g = (-41592.9 + g) * t; g = (42002.57 + g) * t; g = (-24314.21 + g) * t;
-  g = (8418.94 + g) * t; g = (-1763.96 + g) * t; g = (215.896 + g) * t;
-  g = (-13.328 + g) * t; return 1.21 + g;
-}
-HGD inline double poly_b(double t) {
-  double g = (-29030.24 + 7671.22 * t) * t;
-  g = (44894.06 + g) * t; g = (-36618.81 + g) * t; g = (17137.74 + g) * t;
-  g = (-4780.77 + g) * t; g = (796.534 + g) * t; g = (-67.92 + g) * t;
-  g = (5.373 + g) * t; return 0.938 + g;
-}
-HGD inline double poly_c(double t) {
-  double g = (9136.4 + -3272.62 * t) * t;
-  g = (-9844.35 + g) * t; g = (5155.67 + g) * t; g = (-1397.89 + g) * t;
-  g = (209.653 + g) * t; g = (-9.747 + g) * t; return 1.268 + g;
-}
-HGD inline double poly_d(double t) {
-  double g = (128170.2 + -33744.6 * t) * t;
-  g = (-205690.43 + g) * t; g = (181856.75 + g) * t; g = (-96293.05 + g) * t;
-  g = (31127.39 + g) * t; g = (-6072.07 + g) * t; g = (667.16 + g) * t;
-  g = (-40.97 + g) * t; return 0.632 + g;
-}
-HGD inline double poly_da(double t) {
-  double g = (-46688.0 + 12622.25 * t) * t;
-  g = (68220.87 + g) * t; g = (-48811.41 + g) * t; g = (16370.75 + g) * t;
-  g = (-1187.71 + g) * t; g = (-754.85 + g) * t; g = (249.69 + g) * t;
-  g = (-24.53 + g) * t; return 2.948 + g;
-}
-HGD inline double poly_db(double t) {
-  double g = (-76209.82 + 19923.28 * t) * t;
-  g = (118879.26 + g) * t; g = (-97014.11 + g) * t; g = (44270.15 + g) * t;
-  g = (-11336.19 + g) * t; g = (1565.35 + g) * t; g = (-76.765 + g) * t;
-  g = (2.894 + g) * t; return 1.11 + g;
-}
-HGD inline double poly_dc(double t) {
-  double g = (3168.35 + -1590.27 * t) * t;
-  g = (-2318.58 + g) * t; g = (847.8 + g) * t; g = (-148.24 + g) * t;
-  return 14.19 + g;
+template <int N>
+__device__ __forceinline__ double horner(const double (&c)[N], double t) {
+  double g = c[N - 1];
+#pragma unroll
+  for (int k = N - 2; k >= 0; --k) g = fma(g, t, c[k]);
+  return g;
 }
 
 // Havelock wave term GF and its horizontal derivative GFh at the
-// non-dimensional horizontal distance hh = v*R and depth vv = v*(z+zeta).
-HGD inline void havelock(double hh, double vv, double2& gf, double2& gfh) {
+// non-dimensional horizontal distance hh = v*R and depth vv = v*(z+zeta):
+// dd = |(hh, vv)|, alpha = -vv / dd, beta = hh / dd, ihh = 1 / hh (used
+// beyond 3).
+__device__ __forceinline__ void havelock(double hh, double vv, double dd, double alpha, double beta, double ihh,
+                                         double2& gf, double2& gfh) {
   const double gama = 0.5772156649;
-  const double dd = sqrt(hh * hh + vv * vv);
-  const double alpha = -vv / dd, beta = hh / dd, rho = dd / (1.0 + dd);
+  const double omr = rcp_any(1.0 + dd), rho = dd * omr;  // rho = dd / (1 + dd), omr = 1 - rho
   const double ev = exp(vv), emd = exp(-dd);
-  const double dd3 = 1.0 + dd * dd * dd;
-  const double omr = 1.0 - rho, omr3 = omr * omr * omr;
-  double pp = (log(0.5 * (dd - vv)) + gama - 2.0 * dd * dd) * ev + dd * dd - vv;
-  double rr = (1.0 - beta) * poly_a(rho) - beta * poly_b(rho) -
-              alpha * poly_c(rho) / (1.0 + 6.0 * alpha * rho * omr) + beta * (1.0 - beta) * poly_d(rho);
-  const double l0 = 2.0 * pp / dd3 + 2.0 * (rho * omr3 * rr);
+  const double id3 = rcp_any(fma(dd * dd, dd, 1.0));
+  const double ro3 = rho * (omr * omr * omr), ob = 1.0 - beta, lam = dd - vv;
+  const double pa = horner({1.21, -13.328, 215.896, -1763.96, 8418.94, -24314.21, 42002.57, -41592.9, 21859.0, -4838.6},
+                           rho);
+  const double pb = horner({0.938, 5.373, -67.92, 796.534, -4780.77, 17137.74, -36618.81, 44894.06, -29030.24, 7671.22},
+                           rho);
+  const double pc = horner({1.268, -9.747, 209.653, -1397.89, 5155.67, -9844.35, 9136.4, -3272.62}, rho);
+  const double pd = horner({0.632, -40.97, 667.16, -6072.07, 31127.39, -96293.05, 181856.75, -205690.43, 128170.2,
+                            -33744.6}, rho);
+  const double da = horner({2.948, -24.53, 249.69, -754.85, -1187.71, 16370.75, -48811.41, 68220.87, -46688.0, 12622.25},
+                           rho);
+  const double db = horner({1.11, 2.894, -76.765, 1565.35, -11336.19, 44270.15, -97014.11, 118879.26, -76209.82,
+                            19923.28}, rho);
+  const double dc = horner({14.19, -148.24, 847.8, -2318.58, 3168.35, -1590.27}, rho);
+  const double bob = beta * ob, dd2 = dd * dd;
+  const double pp = fma(fma(-2.0, dd2, log(0.5 * lam) + gama), ev, dd2 - vv);
+  double rr = fma(bob, pd, fma(-(alpha * pc), rcp_any(fma(6.0 * alpha, rho * omr, 1.0)), fma(-beta, pb, ob * pa)));
+  const double l0 = 2.0 * fma(pp, id3, ro3 * rr);
   double j0, j1, h0, h1;
   if (hh <= 3.0) {
-    const double yy = (hh / 3.0) * (hh / 3.0);
-    j0 = 0.999999999 + (-2.249999879 + (1.265623060 + (-0.316394552 + (0.044460948 +
-         (-0.003954479 + 0.000212950 * yy) * yy) * yy) * yy) * yy) * yy;
-    j1 = (0.5 + (-0.562499992 + (0.210937377 + (-0.039550040 + (0.004447331 + (-0.000330547 +
-          0.000015525 * yy) * yy) * yy) * yy) * yy) * yy) * hh;
-    h0 = (1.909859164 + (-1.909855001 + (0.687514637 + (-0.126164557 + (0.013828813 -
-          0.000876918 * yy) * yy) * yy) * yy) * yy) * (hh / 3.0);
-    h1 = (1.909859286 + (-1.145914713 + (0.294656958 + (-0.042070508 + (0.003785727 -
-          0.000207183 * yy) * yy) * yy) * yy) * yy) * yy;
+    const double th = hh * (1.0 / 3.0), yy = th * th;
+    j0 = horner({0.999999999, -2.249999879, 1.265623060, -0.316394552, 0.044460948, -0.003954479, 0.000212950}, yy);
+    j1 = horner({0.5, -0.562499992, 0.210937377, -0.039550040, 0.004447331, -0.000330547, 0.000015525}, yy) * hh;
+    h0 = horner({1.909859164, -1.909855001, 0.687514637, -0.126164557, 0.013828813, -0.000876918}, yy) * th;
+    h1 = horner({1.909859286, -1.145914713, 0.294656958, -0.042070508, 0.003785727, -0.000207183}, yy) * yy;
   } else {
-    const double y = 3.0 / hh, y2 = y * y, isq = 1.0 / sqrt(hh);
-    const double f0 = 0.79788454 + (-0.00553897 + (0.00099336 + (-0.00044346 + (0.00020445 -
-                      0.00004959 * y2) * y2) * y2) * y2) * y2;
-    const double t0 = hh - 0.25 * HG_PI + (-0.04166592 + (0.00239399 + (-0.00073984 + (0.00031099 -
-                      0.00007605 * y2) * y2) * y2) * y2) * y;
-    const double f1 = 0.79788459 + (0.01662008 + (-0.00187002 + (0.00068519 + (-0.00029440 +
-                      0.00006952 * y2) * y2) * y2) * y2) * y2;
-    const double t1 = hh - 0.75 * HG_PI + (0.12499895 + (-0.00605240 + (0.00135825 + (-0.00049616 +
-                      0.00011531 * y2) * y2) * y2) * y2) * y;
+    const double y = 3.0 * ihh, y2 = y * y, isq = rsqrt_near(hh);
+    const double f0 = horner({0.79788454, -0.00553897, 0.00099336, -0.00044346, 0.00020445, -0.00004959}, y2) * isq;
+    const double t0 = fma(horner({-0.04166592, 0.00239399, -0.00073984, 0.00031099, -0.00007605}, y2), y,
+                          hh - 0.25 * HG_PI);
+    const double f1 = horner({0.79788459, 0.01662008, -0.00187002, 0.00068519, -0.00029440, 0.00006952}, y2) * isq;
+    const double t1 = fma(horner({0.12499895, -0.00605240, 0.00135825, -0.00049616, 0.00011531}, y2), y,
+                          hh - 0.75 * HG_PI);
     double s0, c0, s1, c1;
     sincos(t0, &s0, &c0);
     sincos(t1, &s1, &c1);
-    j0 = f0 * c0 * isq;
-    j1 = f1 * c1 * isq;
-    const double y0 = f0 * s0 * isq, y1 = f1 * s1 * isq;
-    h0 = 2.0 * (0.99999906 + (4.77228920 + (3.85542044 + 0.32303607 * y2) * y2) * y2) /
-             (HG_PI * hh * (1.0 + (4.88331068 + (4.28957333 + 0.52120508 * y2) * y2) * y2)) + y0;
-    h1 = 2.0 * (1.00000004 + (3.92205313 + (2.64893033 + 0.27450895 * y2) * y2) * y2) /
-             (HG_PI * (1.0 + (3.81095112 + (2.26216956 + 0.10885141 * y2) * y2) * y2)) + y1;
+    j0 = f0 * c0;
+    j1 = f1 * c1;
+    const double e0 = horner({1.0, 4.88331068, 4.28957333, 0.52120508}, y2);
+    const double e1 = horner({1.0, 3.81095112, 2.26216956, 0.10885141}, y2);
+    const double ie = rcp_any(e0 * e1) * (2.0 / HG_PI);  // both denominators in one reciprocal
+    h0 = fma(horner({0.99999906, 4.77228920, 3.85542044, 0.32303607}, y2) * (ie * e1), ihh, f0 * s0);
+    h1 = fma(horner({1.00000004, 3.92205313, 2.64893033, 0.27450895}, y2), ie * e0, f1 * s1);
   }
   const double tpe = 2.0 * HG_PI * ev;
-  gf = make_double2(l0 + tpe * h0, -tpe * j0);
-  const double ps = (beta + hh) / (dd - vv) - 2.0 * beta + 2.0 * ev * dd - hh;
-  const double qs = emd * (1.0 - beta) * (1.0 + dd / dd3);
-  rr = beta * poly_da(rho) - (1.0 - alpha) * poly_db(rho) +
-       beta * (1.0 - beta) * rho * (1.0 - 2.0 * rho) * poly_dc(rho);
-  const double ls = 2.0 * ps / dd3 - 4.0 * qs + 2.0 * (rho * omr3 * rr);
-  gfh = make_double2(ls + tpe * (2.0 / HG_PI - h1), tpe * j1);
+  gf = make_double2(fma(tpe, h0, l0), -tpe * j0);
+  const double ps = fma(beta + hh, rcp_any(lam), fma(2.0 * ev, dd, fma(-2.0, beta, -hh)));
+  const double qs = emd * ob * fma(dd, id3, 1.0);
+  rr = fma(bob * rho * fma(-2.0, rho, 1.0), dc, fma(beta, da, -((1.0 - alpha) * db)));
+  const double ls = fma(2.0, fma(ps, id3, ro3 * rr), -4.0 * qs);
+  gfh = make_double2(fma(tpe, 2.0 / HG_PI - h1, ls), tpe * j1);
 }
 
 // INFGREEN3D (InfGreen_Appr.f90:104-186).  Source (xq,yq,zq), field (xp,yp,zp).
-HGD inline void inf_green(double xq, double yq, double zq, double xp, double yp,
-                                          double zp, double v, int flag, double2 g[4]) {
-  const double xpq = xq - xp, ypq = yq - yp, zpq = zp + zq;
-  const double rr = sqrt(xpq * xpq + ypq * ypq);
-  const double r = sqrt(rr * rr + (zp - zq) * (zp - zq));
-  const double r1 = sqrt(rr * rr + zpq * zpq);
-  const double ir1 = 1.0 / r1, ir13 = ir1 * ir1 * ir1;
-  const double ir = 1.0 / r, ir3 = ir * ir * ir;
+__device__ __forceinline__ void inf_green(double xq, double yq, double zq, double xp, double yp, double zp, double v,
+                                          double iv, int flag, double2 g[4]) {
+  const double xpq = xq - xp, ypq = yq - yp, zpq = zp + zq, zd = zq - zp;
+  const double h2 = fma(xpq, xpq, ypq * ypq);
+  const double irr = h2 > 0.0 ? rsqrt_near(h2) : 0.0, rr = h2 * irr;
+  const double q1 = fma(zpq, zpq, h2), ir1 = rsqrt_near(q1), ir13 = ir1 * ir1 * ir1;
   double sgn1 = 1.0;  // sign of the image term: -1 at the infinite-frequency limit
   if (fabs(v) < SPD(1.e-8) || fabs(v + 1.0) < SPD(1.e-8)) {
     if (!(fabs(v) < SPD(1.e-8))) sgn1 = -1.0;
     g[0] = make_double2(0.0, 0.0); g[1] = g[0]; g[2] = g[0]; g[3] = g[0];
   } else {
     double2 gf, gfh;
-    havelock(v * rr, v * zpq, gf, gfh);
+    const double is1 = copysign(ir1, v);
+    havelock(v * rr, v * zpq, fabs(v) * (q1 * ir1), -zpq * is1, rr * is1, irr * iv, gf, gfh);
     const double v2 = v * v;
     if (rr > SPD(1.e-6)) {
-      const double cx = -v2 * xpq / rr, cy = -v2 * ypq / rr;
+      const double c = -v2 * irr, cx = c * xpq, cy = c * ypq;
       g[1] = make_double2(gfh.x * cx, gfh.y * cx);
       g[2] = make_double2(gfh.x * cy, gfh.y * cy);
     } else {
@@ -210,17 +289,19 @@ HGD inline void inf_green(double xq, double yq, double zq, double xp, double yp,
       g[2] = make_double2(0.0, 0.0);
     }
     g[0] = make_double2(-v * gf.x, -v * gf.y);
-    g[3] = make_double2(-v2 * gf.x + 2.0 * v * ir1, -v2 * gf.y);
+    g[3] = make_double2(fma(2.0 * v, ir1, -v2 * gf.x), -v2 * gf.y);
   }
-  g[0].x += sgn1 * ir1;
-  g[1].x -= sgn1 * xpq * ir13;
-  g[2].x -= sgn1 * ypq * ir13;
-  g[3].x -= sgn1 * zpq * ir13;
+  const double i3 = sgn1 * ir13;
+  g[0].x = fma(sgn1, ir1, g[0].x);
+  g[1].x = fma(-xpq, i3, g[1].x);
+  g[2].x = fma(-ypq, i3, g[2].x);
+  g[3].x = fma(-zpq, i3, g[3].x);
   if (flag == 0) {
+    const double ir = rsqrt_near(fma(zd, zd, h2)), ir3 = ir * ir * ir;
     g[0].x += ir;
-    g[1].x -= xpq * ir3;
-    g[2].x -= ypq * ir3;
-    g[3].x -= (zq - zp) * ir3;
+    g[1].x = fma(-xpq, ir3, g[1].x);
+    g[2].x = fma(-ypq, ir3, g[2].x);
+    g[3].x = fma(-zd, ir3, g[3].x);
   }
 }
 
