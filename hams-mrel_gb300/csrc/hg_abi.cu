@@ -877,6 +877,9 @@ int solve_cols_once(hg_ctx* c, int c0, int c1) {
   return 0;
 }
 
+// Below this order the plain form's products with few columns run on the FP64 pipes.
+constexpr int kSmallOrder = 1024;
+
 int build_rhs(hg_ctx* c, int nbeta, const double* betas_h, bool modes) {
   int r = ensure_rhs(c, nbeta);
   if (r) return r;
@@ -891,9 +894,30 @@ int build_rhs(hg_ctx* c, int nbeta, const double* betas_h, bool modes) {
     CK(hg::launch_rhs_cols(c->st, c->n, c->dxyz.p, c->body_of.p, c->nbody, nbeta, c->W.p, c->Wz.p, c->n));
     CK(hg::resid_df(c->st, false, c->tn, nc, c->n, c->Sf.p, c->tn, c->Wz.p, c->n, nullptr, 0, 1.0, c->B.p, c->tn,
                     c->rws.p, c->rws.cap, false));
-  } else
-    CK(hg::launch_rhs<double2>(c->st, c->n, c->tn, c->S.p, c->tn, c->dxyz.p, c->body_of.p, c->nbody, nbeta, c->W.p,
-                               c->part.p, c->B.p, c->tn));
+  } else {
+    // B = S [modes | headings]: digit-sliced on the tensor cores (their digits in the LU's workspace,
+    // which the plain form keeps nothing in after the factorisation), below their order on the FP64
+    // pipes; one thread per row (launch_rhs) takes 4.2 ms against about 1 ms at 6048 panels, 0.6 ms
+    // against 0.02 ms at 384
+    const int nc = 6 * c->nbody + nbeta;
+    const size_t zb = c->o.lu_tensor != 0 && hg::zgemm_tc_supported() ? hg::zgemm_tc_work_bytes(c->tn, nc, c->n) : 0;
+    const bool small = c->n < kSmallOrder, ztc = !small && zb && c->luws.cap >= zb;
+    if (small || ztc) {
+      CK(c->Wz.ensure((size_t)c->n * nc));
+      CK(hg::launch_rhs_cols(c->st, c->n, c->dxyz.p, c->body_of.p, c->nbody, nbeta, c->W.p, c->Wz.p, c->n));
+    }
+    if (small) {
+      CK(hg::zskinny(c->st, c->tn, nc, c->n, 1.0, c->S.p, c->tn, c->Wz.p, c->n, 0.0, c->B.p, c->tn));
+    } else if (ztc) {
+      k_negate<<<256, 256, 0, c->st>>>((long)c->n * nc, c->Wz.p, c->Wz.p);
+      CK(cudaMemsetAsync(c->B.p, 0, (size_t)c->tn * nc * sizeof(double2), c->st));
+      CK(hg::zgemm_tc(c->st, c->tn, nc, c->n, c->S.p, c->tn, c->Wz.p, c->n, c->B.p, c->tn, c->luws.p, c->luws.cap,
+                      c->status.p));
+    } else {
+      CK(hg::launch_rhs<double2>(c->st, c->n, c->tn, c->S.p, c->tn, c->dxyz.p, c->body_of.p, c->nbody, nbeta, c->W.p,
+                                 c->part.p, c->B.p, c->tn));
+    }
+  }
   (void)modes;
   return 0;
 }

@@ -559,6 +559,59 @@ k_zupdate(int m, int n, int k, const double2* __restrict__ A, long lda, const do
 // tensor-core products.
 constexpr long kZupdMax = 400000;
 
+// C = beta C + alpha A B (beta 0 or 1, alpha +1 or -1) for few columns on the
+// FP64 pipes: 4 x 8 entries of C per CTA, the inner dimension dealt out over
+// 64 threads per row and added at the end.  A tile that takes the whole inner
+// dimension by itself (k_gemm) leaves a right-hand side of a few hundred rows
+// to two or three SMs: 143 us for 128 x 7 x 256.
+__global__ void __launch_bounds__(256)
+k_zskinny(int m, int n, int k, double alpha, double beta, const double2* __restrict__ A, long lda,
+          const double2* __restrict__ B, long ldb, double2* __restrict__ C, long ldc) {
+  __shared__ double2 red[8][4][8];
+  const int r = threadIdx.x & 3, sl = threadIdx.x >> 2, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int gr = blockIdx.x * 4 + r, c0 = blockIdx.y * 8;
+  double2 acc[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) acc[j] = make_double2(0.0, 0.0);
+  if (gr < m) {
+    for (int l = sl; l < k; l += 64) {
+      const double2 a = A[gr + (long)l * lda];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        if (c0 + j < n) {
+          const double2 b = B[l + (long)(c0 + j) * ldb];
+          acc[j].x = fma(-a.y, b.y, fma(a.x, b.x, acc[j].x));
+          acc[j].y = fma(a.y, b.x, fma(a.x, b.y, acc[j].y));
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+#pragma unroll
+    for (int off = 4; off < 32; off <<= 1) {
+      acc[j].x += __shfl_xor_sync(0xffffffffu, acc[j].x, off);
+      acc[j].y += __shfl_xor_sync(0xffffffffu, acc[j].y, off);
+    }
+    if (lane < 4) red[warp][r][j] = acc[j];
+  }
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    const int rr = threadIdx.x & 3, j = threadIdx.x >> 2, row = blockIdx.x * 4 + rr;
+    double2 t = red[0][rr][j];
+#pragma unroll
+    for (int w = 1; w < 8; ++w) {
+      t.x += red[w][rr][j].x;
+      t.y += red[w][rr][j].y;
+    }
+    if (row < m && c0 + j < n) {
+      double2* c = C + row + (long)(c0 + j) * ldc;
+      const double2 o = beta != 0.0 ? *c : make_double2(0.0, 0.0);
+      *c = make_double2(fma(alpha, t.x, o.x), fma(alpha, t.y, o.y));
+    }
+  }
+}
+
 // Columns [c0, c1) of A through one level of right-looking blocking with
 // 32-wide panels (pivots applied only inside [c0, c1)).  With aux, the
 // update of the columns beyond the next panel runs on aux->side (see getrf).
@@ -709,6 +762,11 @@ __global__ void k_u12_operands(int nb, const double2* __restrict__ X, const doub
   Lf[o] = r > c ? A11[r + (long)c * lda] : make_double2(r == c ? 1.0 : 0.0, 0.0);
 }
 
+}  // namespace
+cudaError_t trsm_blocks_z(cudaStream_t st, bool upper, const double2* A, long lda, int jb, double2* X, long ldx, int ncols,
+                          bool eye);
+namespace {
+
 // Two-level complex128 LU: 256-wide outer panels by the 32-wide loop (panels
 // on the FP64 pipes, their updates inside the outer panel on the tensor
 // cores), then U12 = L11^-1 A12 and A22 -= L21 U12, all products as exact
@@ -738,7 +796,7 @@ cudaError_t getrf_z_tc(cudaStream_t st, bool use_cluster, int n, double2* A, lon
     double2* A11 = A + K + (long)K * lda;
     double2* A12 = A + K + (long)(K + jbo) * lda;
     k_eye_z<<<eg, 128, 0, st>>>(jbo, X, kOuterNB);
-    e = trsm_cols<double>(st, false, A11, lda, jbo, X, kOuterNB, jbo);
+    e = trsm_blocks_z(st, false, A11, lda, jbo, X, kOuterNB, jbo, true);
     if (e != cudaSuccess) return e;
     k_u12_operands<<<eg, 128, 0, st>>>(jbo, X, A11, lda, M, Xn, Lf, kOuterNB);
     e = cudaMemcpy2DAsync(W, (size_t)kOuterNB * sizeof(double2), A12, (size_t)lda * sizeof(double2),
@@ -870,6 +928,86 @@ cudaError_t getrs_inv(cudaStream_t st, int n, int nrhs, const float2* LU, long l
   return cudaGetLastError();
 }
 
+// X = T^-1 X in complex128 for a triangle of at most 64 rows (unit lower, or
+// upper), one CTA per column.  A thread holds the real or the imaginary part
+// of one row: a step of the substitution is then two dependent fused
+// operations on each scheduler, one warp instruction of which occupies its
+// FP64 pipe for 64 cycles, and one barrier.  17 us (lower) and 31 us (upper)
+// for 64 rows; 16 rows at a time by one warp with shuffles took 48 and 41 us.
+constexpr int kSolveZ = 64;
+template <bool UPPER>
+__global__ void __launch_bounds__(2 * kSolveZ)
+k_trsm64_z(const double2* __restrict__ A, long lda, int w, double2* __restrict__ X, long ldx) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  double2* t = reinterpret_cast<double2*>(smem_raw);  // [w][kSolveZ], the needed triangle
+  __shared__ double xs[kSolveZ][2];
+  __shared__ double2 rd[kSolveZ];
+  const int row = threadIdx.x & (kSolveZ - 1), part = threadIdx.x / kSolveZ;
+  double* xc = reinterpret_cast<double*>(X + (long)blockIdx.x * ldx + row) + part;
+  double v = row < w ? *xc : 0.0;
+  for (int e = threadIdx.x; e < w * kSolveZ; e += 2 * kSolveZ) {
+    const int i = e % kSolveZ, j = e / kSolveZ;
+    if (i < w && (UPPER ? i <= j : i > j)) t[e] = A[i + (long)j * lda];
+  }
+  if (UPPER) {
+    __syncthreads();
+    if (part == 0 && row < w) rd[row] = crecip(t[row * kSolveZ + row]);
+  }
+  for (int q = 0; q < w; ++q) {
+    const int j = UPPER ? w - 1 - q : q;
+    if (row == j) xs[j][part] = v;
+    __syncthreads();  // also the triangle and the reciprocals on the first step
+    double xr = xs[j][0], xi = xs[j][1];
+    if (UPPER) {
+      const double2 r = rd[j];
+      const double yr = fma(-xi, r.y, xr * r.x);
+      xi = fma(xi, r.x, xr * r.y);
+      xr = yr;
+      if (row == j) v = part ? xi : xr;
+    }
+    if (row < w && (UPPER ? row < j : row > j)) {
+      const double2 l = t[j * kSolveZ + row];
+      v = part ? fma(-l.y, xr, fma(-l.x, xi, v)) : fma(l.y, xi, fma(-l.x, xr, v));
+    }
+  }
+  if (row < w) *xc = v;
+}
+
+cudaError_t trsm64_z(cudaStream_t st, bool upper, const double2* A, long lda, int w, double2* X, long ldx, int ncols) {
+  if (w <= 0 || ncols <= 0) return cudaSuccess;
+  const size_t smem = (size_t)kSolveZ * kSolveZ * sizeof(double2);
+  auto kern = upper ? k_trsm64_z<true> : k_trsm64_z<false>;
+  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  kern<<<ncols, 2 * kSolveZ, smem, st>>>(A, lda, w, X, ldx);
+  return cudaGetLastError();
+}
+
+cudaError_t zskinny(cudaStream_t st, int m, int n, int k, double alpha, const double2* A, long lda, const double2* B,
+                    long ldb, double beta, double2* C, long ldc) {
+  if (m <= 0 || n <= 0) return cudaSuccess;
+  k_zskinny<<<dim3((m + 3) / 4, (n + 7) / 8), 256, 0, st>>>(m, n, k, alpha, beta, A, lda, B, ldb, C, ldc);
+  return cudaGetLastError();
+}
+
+// X = T^-1 X by kSolveZ rows at a time: the triangles, and their updates of the
+// rows still to solve.  eye: X is the identity on entry and the triangle lower,
+// so the columns right of a step's rows are still zero in them.
+cudaError_t trsm_blocks_z(cudaStream_t st, bool upper, const double2* A, long lda, int jb, double2* X, long ldx, int ncols,
+                          bool eye) {
+  const int steps = (jb + kSolveZ - 1) / kSolveZ;
+  for (int q = 0; q < steps; ++q) {
+    const int k = (upper ? steps - 1 - q : q) * kSolveZ, w = (jb - k < kSolveZ) ? jb - k : kSolveZ;
+    const int nc = eye ? (k + w < ncols ? k + w : ncols) : ncols;
+    cudaError_t e = trsm64_z(st, upper, A + k + (long)k * lda, lda, w, X + k, ldx, nc);
+    if (e != cudaSuccess) return e;
+    if (upper) e = zskinny(st, k, nc, w, -1.0, A + (long)k * lda, lda, X + k, ldx, 1.0, X, ldx);
+    else e = zskinny(st, jb - k - w, nc, w, -1.0, A + k + w + (long)k * lda, lda, X + k, ldx, 1.0, X + k + w, ldx);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+
 template <typename R>
 cudaError_t getrs(cudaStream_t st, int n, int nrhs, const typename cx<R>::T* LU, long lda, const int* ipiv,
                   typename cx<R>::T* B, long ldb, void* work, size_t work_bytes, int* status) {
@@ -879,7 +1017,19 @@ cudaError_t getrs(cudaStream_t st, int n, int nrhs, const typename cx<R>::T* LU,
   // complex128 block updates as exact digit products on the tensor cores
   const bool ztc = sizeof(R) == 8 && work && status && n > kSolveNB &&
                    work_bytes >= zgemm_tc_work_bytes(n, nrhs, kSolveNB) && zgemm_tc_supported();
+  // Complex128: the diagonal blocks themselves in steps of kSolveZ rows, their
+  // updates spread over the SMs (k_zskinny), since one CTA per column runs a
+  // whole block's triangle at its own SM's FP64 rate (190 us for 256 rows).
+  auto solve_block = [&](bool upper, const T* A_, int jb, T* X_) -> cudaError_t {
+    if constexpr (sizeof(R) == 8)
+      return trsm_blocks_z(st, upper, A_, lda, jb, X_, ldb, nrhs, false);
+    else
+      return trsm_cols<R>(st, upper, A_, lda, jb, X_, ldb, nrhs);
+  };
   auto update = [&](int m, int kk, const T* A_, const T* X_, T* C_) -> cudaError_t {
+    if (sizeof(R) == 8 && !ztc && n < kTcMinN)
+      return zskinny(st, m, nrhs, kk, -1.0, reinterpret_cast<const double2*>(A_), lda,
+                     reinterpret_cast<const double2*>(X_), ldb, 1.0, reinterpret_cast<double2*>(C_), ldb);
     if (ztc)
       return zgemm_tc(st, m, nrhs, kk, reinterpret_cast<const double2*>(A_), lda, reinterpret_cast<const double2*>(X_),
                       ldb, reinterpret_cast<double2*>(C_), ldb, work, work_bytes, status);
@@ -888,7 +1038,7 @@ cudaError_t getrs(cudaStream_t st, int n, int nrhs, const typename cx<R>::T* LU,
   k_laswp<T><<<(nrhs + 127) / 128, 128, 0, st>>>(B, ldb, nrhs, ipiv, 0, n, 0, 0);
   for (int k = 0; k < n; k += kSolveNB) {
     const int jb = (n - k < kSolveNB) ? n - k : kSolveNB;
-    cudaError_t e = trsm_cols<R>(st, false, LU + k + (long)k * lda, lda, jb, B + k, ldb, nrhs);
+    cudaError_t e = solve_block(false, LU + k + (long)k * lda, jb, B + k);
     if (e != cudaSuccess) return e;
     const int rest = n - k - jb;
     if (rest > 0) {
@@ -899,7 +1049,7 @@ cudaError_t getrs(cudaStream_t st, int n, int nrhs, const typename cx<R>::T* LU,
   const int last = ((n - 1) / kSolveNB) * kSolveNB;
   for (int k = last; k >= 0; k -= kSolveNB) {
     const int jb = (n - k < kSolveNB) ? n - k : kSolveNB;
-    cudaError_t e = trsm_cols<R>(st, true, LU + k + (long)k * lda, lda, jb, B + k, ldb, nrhs);
+    cudaError_t e = solve_block(true, LU + k + (long)k * lda, jb, B + k);
     if (e != cudaSuccess) return e;
     if (k > 0) {
       e = update(k, jb, LU + (long)k * lda, B + k, B);

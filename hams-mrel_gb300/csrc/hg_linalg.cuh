@@ -84,6 +84,11 @@ template <typename R>
 cudaError_t getrs(cudaStream_t st, int n, int nrhs, const typename cx<R>::T* LU, long lda, const int* ipiv,
                   typename cx<R>::T* B, long ldb, void* work = nullptr, size_t work_bytes = 0, int* status = nullptr);
 
+// C = beta C + alpha A B in complex128 on the FP64 pipes for few columns n (any
+// inner dimension k; beta 0 or 1).
+cudaError_t zskinny(cudaStream_t st, int m, int n, int k, double alpha, const double2* A, long lda, const double2* B,
+                    long ldb, double beta, double2* C, long ldc);
+
 size_t lu_work_bytes(int n, int tc_passes);
 size_t lu_work_bytes_z(int n);
 

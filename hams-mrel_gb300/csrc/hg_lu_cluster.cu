@@ -954,15 +954,11 @@ constexpr int kTrsmBlock = 256;
 
 template <typename T> struct TrsmSub;
 template <> struct TrsmSub<float2> { static constexpr int SB = 32; };
-template <> struct TrsmSub<double2> { static constexpr int SB = 16; };
 
 template <typename T>
 __device__ __forceinline__ void cp_elem(T* dst, const T* src, bool pred);
 template <> __device__ __forceinline__ void cp_elem<float2>(float2* dst, const float2* src, bool pred) {
   cp_async8(dst, src, pred);
-}
-template <> __device__ __forceinline__ void cp_elem<double2>(double2* dst, const double2* src, bool pred) {
-  cp_async16(dst, src, pred ? 16 : 0);
 }
 
 template <typename T>
@@ -1055,7 +1051,6 @@ cudaError_t trsm_cols(cudaStream_t st, bool upper, const typename cx<R>::T* A, l
   return cudaGetLastError();
 }
 template cudaError_t trsm_cols<float>(cudaStream_t, bool, const float2*, long, int, float2*, long, int);
-template cudaError_t trsm_cols<double>(cudaStream_t, bool, const double2*, long, int, double2*, long, int);
 
 // ---------------------------------------------------------------------------
 // Inverses of the diagonal blocks (order <= 256) of the complex64 factors:
