@@ -203,7 +203,7 @@ int keyed_fill(hg_ctx* c, int tn, int near_only, OUT* A, OUT* S, bool* done) {
     CK(e);
   }
   const cudaError_t e = hg::fin_keys_fill<FAST, OUT>(c->st, K, c->rec.p, c->fx.p, c->tnf, c->zlev.p, fin_state(c),
-                                                     c->o.grn_kind, A, S, tn, tn);
+                                                     c->o.grn_kind, A, S, tn, tn, &c->lu_aux);
   if (e == cudaErrorMemoryAllocation) {
     cudaGetLastError();
     K.release();

@@ -50,9 +50,9 @@ void FinKeys::release() {
 template cudaError_t fin_keys_build<0>(cudaStream_t, FinKeys&, const double*, const double*, int, int, int, double, int,
                                        const int*, const int*, int);
 template cudaError_t fin_keys_fill<0, double2>(cudaStream_t, FinKeys&, const double*, const double*, int, const double*,
-                                               const FinState&, int, double2*, double2*, long, int);
+                                               const FinState&, int, double2*, double2*, long, int, const LuAux*);
 template cudaError_t fin_keys_fill<0, float2>(cudaStream_t, FinKeys&, const double*, const double*, int, const double*,
-                                              const FinState&, int, float2*, float2*, long, int);
+                                              const FinState&, int, float2*, float2*, long, int, const LuAux*);
 
 cudaError_t launch_green_points_fin(cudaStream_t st, int npts, const double* pts, const int* flags, const FinState& fs,
                                     double* out) {

@@ -21,6 +21,6 @@ cudaError_t launch_green_fill_fin_fma(cudaStream_t st, const double* rec, const 
 template cudaError_t fin_keys_build<1>(cudaStream_t, FinKeys&, const double*, const double*, int, int, int, double, int,
                                        const int*, const int*, int);
 template cudaError_t fin_keys_fill<1, float2>(cudaStream_t, FinKeys&, const double*, const double*, int, const double*,
-                                              const FinState&, int, float2*, float2*, long, int);
+                                              const FinState&, int, float2*, float2*, long, int, const LuAux*);
 
 }  // namespace hg

@@ -29,6 +29,7 @@
 namespace hg {
 
 struct FinState;
+struct LuAux;
 
 // Bands of keys, in the order of their R: 0 LINTON, 1..7 PIDCOCK, 8..13
 // EIGENE (both by series length), 14 EIGEN.
@@ -81,9 +82,10 @@ cudaError_t fin_keys_build(cudaStream_t st, FinKeys& K, const double* rec, const
                            double h, int near_only, const int* zsrc, const int* zfld, int nlev);
 
 // Evaluate the keys at fs and write A and S of their pairs (the others are
-// left alone).
+// left alone).  aux: a side stream for the LINTON keys, which are few and long
+// (about a millisecond on a handful of SMs): they run beside the others.
 template <int FAST, typename OUT>
 cudaError_t fin_keys_fill(cudaStream_t st, FinKeys& K, const double* rec, const double* fx, int ldf, const double* zlev,
-                          const FinState& fs, int grn_kind, OUT* A, OUT* S, long lda, int ndiag);
+                          const FinState& fs, int grn_kind, OUT* A, OUT* S, long lda, int ndiag, const LuAux* aux);
 
 }  // namespace hg

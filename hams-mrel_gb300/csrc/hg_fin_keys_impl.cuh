@@ -4,6 +4,7 @@
 #pragma once
 #include "hg_fill_kernel.cuh"
 #include "hg_fin_keys.cuh"
+#include "hg_linalg.cuh"
 #include "hg_rcp.cuh"
 
 namespace hg {
@@ -172,10 +173,12 @@ struct ZTab {
   double* fld;    // cos of um (z + h)
   double* fldt;
   double2* hyp;   // cosh, sinh of wk (z + h)
+  double* term;   // kTermVals per term i (row i - 2)
   int nlev;
 };
 constexpr int kZRows = 100;
-size_t ztab_doubles(int nlev) { return (size_t)kZRows * nlev * 6 + (size_t)2 * nlev; }
+constexpr int kTermVals = 6;  // per term: um, the EIGENE / EIGEN coefficient pm, pm um, PIDCOCK's ac, umt
+size_t ztab_doubles(int nlev) { return (size_t)kZRows * nlev * 6 + (size_t)2 * nlev + (size_t)kZRows * kTermVals; }
 ZTab ztab_of(double* p, int nlev) {
   const size_t row = (size_t)kZRows * nlev;
   ZTab t;
@@ -184,8 +187,41 @@ ZTab ztab_of(double* p, int nlev) {
   t.hyp = reinterpret_cast<double2*>(p + 4 * row);
   t.fld = p + 4 * row + 2 * (size_t)nlev;
   t.fldt = t.fld + row;
+  t.term = t.fldt + row;
   t.nlev = nlev;
   return t;
+}
+
+// The two expressions of PIDCOCK's terms whose fused form matters.  The
+// extrapolation turns their last bit into differences far above single
+// precision, so the contracted build spells out the fused operations that the
+// contracted per-pair kernel (d_series_eps) takes; the plain build rounds
+// every product.
+// A coefficient (um^2 + v^2) / ((um^2 + v^2) h - v):
+template <int FAST>
+__device__ __forceinline__ double pid_ac(double um, double v, double h) {
+  if (!FAST) return (um * um + v * v) / ((um * um + v * v) * h - v);
+  const double t = fma(v, v, __dmul_rn(um, um));
+  return t / fma(t, h, -v);
+}
+// A difference a x - b y, the first product fused:
+template <int FAST>
+__device__ __forceinline__ double pid_diff(double a, double x, double b, double y) {
+  return FAST ? fma(a, x, -__dmul_rn(b, y)) : a * x - b * y;
+}
+
+// The per-term coefficients of the series.
+template <int FAST>
+__global__ void k_key_terms(FinState s, ZTab t) {
+  const int i = threadIdx.x + 2;
+  if (i > kZRows + 1 || i > s.nk) return;
+  const double um = s.wvn[i - 1], h = s.h, tkh = 2.0 * um * h, pm = 4.0 / (1.0 + sin(tkh) / tkh) / h;
+  double* o = t.term + (size_t)(i - 2) * kTermVals;
+  o[0] = um;
+  o[1] = pm;
+  o[2] = pm * um;
+  o[3] = pid_ac<FAST>(um, s.v, h);
+  o[4] = (i - 1) * HG_PI / h;
 }
 
 template <int FAST>
@@ -280,13 +316,17 @@ __device__ __forceinline__ void wynn_entries(const double* x, const double* old,
 
 // Limes (d_limes, hg_green.cuh) on s[0..n] and scratch a[] with stride STR,
 // the a and s steps of a level in one pass: a(i) needs s(i), s(i+1) and the
-// old a(i+1), s(i - 1) the new a(i - 1), a(i) and the old s(i).  Four entries
-// at a time: their reciprocals are independent, and with one warp per
-// scheduler (shared memory holds no more) their latency is hidden only by
-// each other.  |a| is compared as its bits (the order of non-negative doubles).
-// Against the FP64 reciprocals, one entry at a time: EIGENE sums of the
-// irregular 627-panel hull (368 k keys) 17.3 -> 9.1 ms, PIDCOCK sums of two
-// cylinders at h = 150 m (82 k keys) about 15 -> 7.9 ms.
+// old a(i+1), s(i - 1) the new a(i - 1), a(i) and the old s(i).  U entries at a
+// time: their reciprocals are independent, and with a few warps per scheduler
+// (shared memory holds no more) their latency is hidden mostly by each other.
+// Every level is walked in whole groups, from i = 0 (which has no s step) to
+// beyond its last entry (whose surplus is formed from what lies there and
+// dropped): single entries would cost a group's latency each, and short
+// series are mostly ends.  |a| is compared as its bits (the order of
+// non-negative doubles).
+// EIGENE sums of the irregular 627-panel hull (368 k keys): 17.3 ms entry by
+// entry with FP64 reciprocals, 9.1 ms four at a time with single entries at the
+// ends, 5.8 ms as here with the terms' coefficients tabulated.
 template <int STR>
 __device__ __forceinline__ double limes_pass(int n, double* __restrict__ s, double* __restrict__ a) {
   constexpr int U = 4;
@@ -297,75 +337,52 @@ __device__ __forceinline__ double limes_pass(int n, double* __restrict__ s, doub
     const int last = n - 2 * k + 1;
     double sv[U + 1], an[U + 1], sn[U], ao[U];
     sv[0] = s[0];
-    sv[1] = s[STR];
-    ao[0] = (k == 1) ? 0.0 : a[STR];
-    wynn_entries<1>(sv, ao, an);
-    a[0] = an[0];
-    sv[0] = sv[1];
-    int i = 1;
-    auto record = [&](int j) {  // true: the extrapolation has come to rest
-      const uint64_t m = rcp_bits(an[j]) & ~(1ull << 63);
-      if (m > a_max && m <= kInf) {
-        a_max = m;
-        rl = sn[j];
-        return sv[j] == sn[j];
-      }
-      return false;
-    };
-    for (; i + U - 1 <= last; i += U) {
+    an[0] = 0.0;
+    for (int i = 0; i <= last; i += U) {
 #pragma unroll
       for (int j = 0; j < U; ++j) {
-        sv[j + 1] = s[(i + 1 + j) * STR];
-        ao[j] = (k == 1) ? 0.0 : a[(i + 1 + j) * STR];
+        const int at = min(i + 1 + j, n) * STR;
+        sv[j + 1] = s[at];
+        ao[j] = (k == 1) ? 0.0 : a[at];
       }
       wynn_entries<U>(sv, ao, an + 1);
       wynn_entries<U>(an, sv, sn);
 #pragma unroll
       for (int j = 0; j < U; ++j) {
-        a[(i + j) * STR] = an[j + 1];
-        s[(i - 1 + j) * STR] = sn[j];
-        if (record(j)) return rl;
+        const int q = i + j;  // entry of a; q - 1 that of s
+        if (q <= last) a[q * STR] = an[j + 1];
+        if (q <= last && q > 0) {
+          s[(q - 1) * STR] = sn[j];
+          const uint64_t m = rcp_bits(an[j]) & ~(1ull << 63);
+          if (m > a_max && m <= kInf) {
+            a_max = m;
+            rl = sn[j];
+            if (sv[j] == sn[j]) return rl;  // the extrapolation has come to rest
+          }
+        }
       }
       sv[0] = sv[U];
       an[0] = an[U];
-    }
-    for (; i <= last; ++i) {
-      sv[1] = s[(i + 1) * STR];
-      ao[0] = (k == 1) ? 0.0 : a[(i + 1) * STR];
-      wynn_entries<1>(sv, ao, an + 1);
-      wynn_entries<1>(an, sv, sn);
-      a[i * STR] = an[1];
-      s[(i - 1) * STR] = sn[0];
-      if (record(0)) return rl;
-      sv[0] = sv[1];
-      an[0] = an[1];
     }
   }
   return rl;
 }
 
-// The two expressions of PIDCOCK's terms whose fused form matters.  The
-// extrapolation turns their last bit into differences far above single
-// precision, so the contracted build spells out the fused operations that the
-// contracted per-pair kernel (d_series_eps) takes; the plain build rounds
-// every product.
-// A coefficient (um^2 + v^2) / ((um^2 + v^2) h - v):
-template <int FAST>
-__device__ __forceinline__ double pid_ac(double um, double v, double h) {
-  if (!FAST) return (um * um + v * v) / ((um * um + v * v) * h - v);
-  const double t = fma(v, v, __dmul_rn(um, um));
-  return t / fma(t, h, -v);
-}
-// A difference a x - b y, the first product fused:
-template <int FAST>
-__device__ __forceinline__ double pid_diff(double a, double x, double b, double y) {
-  return FAST ? fma(a, x, -__dmul_rn(b, y)) : a * x - b * y;
+// x / h, correctly rounded, from rh = 1 / h correctly rounded: the first
+// residual correction brings the quotient within a unit of the last place,
+// the second rounds it (Markstein 1990).
+__device__ __forceinline__ double div_known(double x, double h, double rh) {
+  double q = x * rh;
+  q = fma(fma(-q, h, x), rh, q);
+  return fma(fma(-q, h, x), rh, q);
 }
 
 // One sum of one key per thread (warps of 32 keys of one sum: 0 G, 1 dG/dR,
 // 2 dG/dz): partial sums into shared memory, extrapolated there into
 // F[6 key + 2 sum].
-constexpr int kSerThreads = 128;
+constexpr int kSerThreads = 32;  // a warp per block: shared memory packs the most warps onto an SM
+constexpr size_t kSerSmemSM = (size_t)227 << 10;  // an SM's shared memory
+constexpr size_t kSerSmemMax = (size_t)2 * (kZRows + 1) * kSerThreads * sizeof(double);
 template <int FAST, bool PID>
 __global__ void __launch_bounds__(kSerThreads)
 k_key_series(FinState s, KeySegs g, int k0, int k1, const int4* __restrict__ keys, ZTab t, const double2* __restrict__ kt,
@@ -382,34 +399,32 @@ k_key_series(FinState s, KeySegs g, int k0, int k1, const int4* __restrict__ key
   const KeySeg& sg = seg_of(g, key.x);
   const double2* kr = kt + sg.base + (key.x - sg.r0);
   const long kstep = sg.len, kpid = (long)sg.rows * sg.len;
-  const double h = s.h, v = s.v;
+  const double h = s.h, rh = 1.0 / h;
   double sum = 0.0;
   sq[0] = 0.0;
   for (int i = 2; i <= nt; ++i) {
-    const double um = s.wvn[i - 1];
+    const double* tv = t.term + (size_t)(i - 2) * kTermVals;
     const size_t zr = (size_t)(i - 2) * t.nlev;
     const double2 kk = kr[(i - 2) * kstep];
     const double2 sc = t.src[zr + key.y];
     const double cp = t.fld[zr + key.z];
     const double k0 = kk.x, k1 = kk.y, su = sc.x, cu = sc.y;
     if (!PID) {
-      const double tkh = 2.0 * um * h, pm = 4.0 / (1.0 + sin(tkh) / tkh) / h;
-      if (q == 0) sum = sum + pm * k0 * cu * cp;
-      else if (q == 1) sum = sum - pm * um * k1 * cu * cp;
-      else sum = sum - pm * um * k0 * su * cp;
+      if (q == 0) sum = sum + tv[1] * k0 * cu * cp;
+      else if (q == 1) sum = sum - tv[2] * k1 * cu * cp;
+      else sum = sum - tv[2] * k0 * su * cp;
     } else {
-      const double umt = (i - 1) * HG_PI / h;
+      const double um = tv[0], ac = tv[3], umt = tv[4];
       const double2 kkt = kr[(i - 2) * kstep + kpid];
       const double2 sct = t.srct[zr + key.y];
       const double cpt = t.fldt[zr + key.z];
       const double k0t = kkt.x, k1t = kkt.y, st = sct.x, ct = sct.y;
-      const double ac = pid_ac<FAST>(um, v, h);
       if (q < 2) {
-        const double am = ac * cu * cp, amt = ct * cpt / h;
+        const double am = ac * cu * cp, amt = div_known(ct * cpt, h, rh);
         if (q == 0) sum = sum + pid_diff<FAST>(am, k0, amt, k0t);
         else sum = sum + pid_diff<FAST>(umt * amt, k1t, um * am, k1);
       } else {
-        const double dam = -(um * ac * su * cp), damt = -(umt * st * cpt / h);
+        const double dam = -(um * ac * su * cp), damt = -div_known(umt * st * cpt, h, rh);
         sum = sum - pid_diff<FAST>(damt, k0t, dam, k0);
       }
     }
@@ -454,15 +469,14 @@ k_key_finish(FinState s, KeySegs g, int k0, int k1, int pid_end, int eig0, const
     const KeySeg& sg = seg_of(g, key.x);
     const double2* kr = kt + sg.base + (key.x - sg.r0);
     for (int i = 2; i <= 10; ++i) {
-      const double km = s.wvn[i - 1], tkh = 2.0 * km * h;
-      const double pm = 4.0 / (1.0 + sin(tkh) / tkh) / h;
+      const double* tv = t.term + (size_t)(i - 2) * kTermVals;
       const size_t zr = (size_t)(i - 2) * t.nlev;
       const double2 kk = kr[(long)(i - 2) * sg.len];
       const double k0 = kk.x, k1 = kk.y;
       const double2 sc = t.src[zr + key.y];
       const double skzf = sc.x, ckzf = sc.y, ckzp = t.fld[zr + key.z];
-      const double rm1 = pm * k0 * ckzf * ckzp, rm2 = -(pm * km * k1 * ckzf * ckzp),
-                   rm3 = -(pm * km * k0 * skzf * ckzp);
+      const double rm1 = tv[1] * k0 * ckzf * ckzp, rm2 = -(tv[2] * k1 * ckzf * ckzp),
+                   rm3 = -(tv[2] * k0 * skzf * ckzp);
       gq[0] += rm1; gq[2] += rm2; gq[4] += rm3;
       if (fabs(rm1) < SPD(1.e-6) && fabs(rm2) < SPD(1.e-6) && fabs(rm3) < SPD(1.e-6)) break;
     }
@@ -710,8 +724,10 @@ cudaError_t fin_keys_build(cudaStream_t st, FinKeys& K, const double* rec, const
 
 template <int FAST, typename OUT>
 cudaError_t fin_keys_fill(cudaStream_t st, FinKeys& K, const double* rec, const double* fx, int ldf, const double* zlev,
-                          const FinState& fs, int grn_kind, OUT* A, OUT* S, long lda, int ndiag) {
+                          const FinState& fs, int grn_kind, OUT* A, OUT* S, long lda, int ndiag, const LuAux* aux) {
   if (K.np == 0) return cudaSuccess;
+  if (aux && (!aux->side || !aux->ev_main || !aux->ev_side)) aux = nullptr;
+  bool side = false;
   if (K.zt_cap < ztab_doubles(K.nlev)) {
     cudaFree(K.zt);
     K.zt = nullptr;
@@ -726,6 +742,7 @@ cudaError_t fin_keys_fill(cudaStream_t st, FinKeys& K, const double* rec, const 
     any_pid = any_pid || (q.bin >= kKeyPid0 && q.bin < kKeyEps0);
     most = bin_rows(q.bin) > most ? bin_rows(q.bin) : most;
   }
+  if (most > 0) k_key_terms<FAST><<<1, 128, 0, st>>>(fs, zt);
   if (most > 0)
     k_key_depths<FAST><<<dim3((K.nlev + 127) / 128, most), 128, 0, st>>>(fs, zlev, zt, any_pid ? 1 : 0);
   size_t gi = 0;
@@ -733,7 +750,15 @@ cudaError_t fin_keys_fill(cudaStream_t st, FinKeys& K, const double* rec, const 
     size_t ge = 0;
     while (ge < K.groups.size() && K.groups[ge].bin == 0) ++ge;
     const int nl = K.groups[ge - 1].k1;
-    k_key_linton<FAST><<<(nl + 3) / 4, 128, 0, st>>>(fs, nl, K.keys, K.rval, zlev, K.F);
+    cudaStream_t ls = st;
+    if (aux) {
+      KE(cudaEventRecord(aux->ev_main, st));
+      KE(cudaStreamWaitEvent(aux->side, aux->ev_main, 0));
+      ls = aux->side;
+      side = true;
+    }
+    k_key_linton<FAST><<<(nl + 3) / 4, 128, 0, ls>>>(fs, nl, K.keys, K.rval, zlev, K.F);
+    if (side) KE(cudaEventRecord(aux->ev_side, ls));
     gi = ge;
   }
   while (gi < K.groups.size()) {  // as many groups at a time as the table holds
@@ -763,32 +788,31 @@ cudaError_t fin_keys_fill(cudaStream_t st, FinKeys& K, const double* rec, const 
     k_key_bessel<FAST><<<dim3((r1 - r0 + 127) / 128, rows), 128, 0, st>>>(fs, g, r0, r1, K.rval, K.rnt, kt, K.jy);
     const int ka = K.groups[g0].k0, kb = K.groups[gi - 1].k1;
     int pid_end = ka, eig0 = ka;
-    int prows = 0, erows = 0;
-    for (size_t q = g0; q < gi; ++q) {
-      const KeyGroup& w = K.groups[q];
-      if (w.bin < kKeyEps0) {
-        pid_end = w.k1;
-        prows = bin_rows(w.bin) > prows ? bin_rows(w.bin) : prows;
-      } else if (w.bin < kKeyEig) {
-        erows = bin_rows(w.bin) > erows ? bin_rows(w.bin) : erows;
+    // Each band with the shared memory its longest series needs, so that short series run with more warps
+    // on an SM; bands that fit the SMs together go in one launch, since each launch lasts at least as long
+    // as its longest extrapolation (fractions of a millisecond).
+    for (size_t q = g0; q < gi && K.groups[q].bin < kKeyEig;) {
+      const bool pid = K.groups[q].bin < kKeyEps0;
+      const int a = K.groups[q].k0, rw = bin_rows(K.groups[q].bin);
+      const size_t smem = (size_t)2 * (rw + 1) * kSerThreads * sizeof(double);
+      const long wave = 152L * (long)(kSerSmemSM / smem < 32 ? kSerSmemSM / smem : 32);
+      int b = K.groups[q].k1;
+      for (++q; q < gi && K.groups[q].bin < kKeyEig && (K.groups[q].bin < kKeyEps0) == pid; ++q) {
+        if (series_blocks(K.groups[q].k1 - a) > wave) break;
+        b = K.groups[q].k1;
       }
-      if (w.bin < kKeyEig) eig0 = w.k1;
+      auto kern = pid ? k_key_series<FAST, true> : k_key_series<FAST, false>;
+      // the attribute is the function's, not the launch's: the same value from every thread
+      KE(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSerSmemMax));
+      kern<<<series_blocks(b - a), kSerThreads, smem, st>>>(fs, g, a, b, K.keys, zt, kt, rw, K.F);
+      if (pid) pid_end = b;
+      eig0 = b;
     }
-    if (pid_end > ka) {
-      const size_t smem = (size_t)2 * (prows + 1) * kSerThreads * sizeof(double);
-      KE(cudaFuncSetAttribute(k_key_series<FAST, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      k_key_series<FAST, true><<<series_blocks(pid_end - ka), kSerThreads, smem, st>>>(fs, g, ka, pid_end, K.keys, zt, kt, prows,
-                                                                               K.F);
-    }
-    if (eig0 > pid_end) {
-      const size_t smem = (size_t)2 * (erows + 1) * kSerThreads * sizeof(double);
-      KE(cudaFuncSetAttribute(k_key_series<FAST, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      k_key_series<FAST, false><<<series_blocks(eig0 - pid_end), kSerThreads, smem, st>>>(fs, g, pid_end, eig0, K.keys, zt, kt,
-                                                                                  erows, K.F);
-    }
+    if (pid_end > eig0) eig0 = pid_end;
     k_key_finish<FAST><<<(kb - ka + 127) / 128, 128, 0, st>>>(fs, g, ka, kb, pid_end, eig0, K.keys, K.rval, zlev, K.jy, zt,
                                                              kt, K.F);
   }
+  if (side) KE(cudaStreamWaitEvent(st, aux->ev_side, 0));
   long fb = ((long)K.np + 127) / 128;
   if (fb > 152L * 64) fb = 152L * 64;
   k_key_fill<FAST, OUT><<<(unsigned)fb, 128, 0, st>>>(rec, fx, ldf, K.tn, K.np, K.pidx, K.pkey, K.F, fs, grn_kind, A, S, lda,

@@ -87,7 +87,7 @@ constexpr int kNodeRows = 54;            // terms of the longest EIGENE series
 struct NodeWork {
   static constexpr size_t F = 0;
   static constexpr size_t zt = F + (size_t)6 * kNodeR * kNodeKeys;
-  static constexpr size_t kt = zt + (size_t)kZRows * kNodeLev * 6 + (size_t)2 * kNodeLev;
+  static constexpr size_t kt = zt + (size_t)kZRows * (kNodeLev * 6 + kTermVals) + (size_t)2 * kNodeLev;
   static constexpr size_t keys = kt + (size_t)2 * kNodeR * kNodeRows;
   static constexpr size_t jy = keys + (size_t)2 * kNodeR * kNodeKeys;
   static constexpr size_t rval = jy + (size_t)4 * kNodeR;
@@ -180,12 +180,13 @@ cudaError_t node_build(cudaStream_t st, const FinState& fs, const FinTab& T, dou
   g.s[0] = KeySeg{0, kFinSegN[2], kNodeRows, 0, 0};
   g.s[1] = KeySeg{kFinSegN[2], kFinSegN[3], 9, 0, (long)kNodeRows * kFinSegN[2]};
   k_node_keys<<<dim3((kNodeKeys + 127) / 128, kNodeR), 128, 0, st>>>(fs, T, rval, rnt, zlev, keys);
+  k_key_terms<1><<<1, 128, 0, st>>>(fs, zt);
   k_key_depths<1><<<dim3((kNodeLev + 127) / 128, kNodeRows), 128, 0, st>>>(fs, zlev, zt, 0);
   k_key_bessel<1><<<dim3((kNodeR + 127) / 128, kNodeRows), 128, 0, st>>>(fs, g, 0, kNodeR, rval, rnt, kt, jy);
   const int ne = kFinSegN[2] * kNodeKeys, nk = kNodeR * kNodeKeys;
   const size_t smem = (size_t)2 * (kNodeRows + 1) * kSerThreads * sizeof(double);
   const cudaError_t e =
-      cudaFuncSetAttribute(k_key_series<1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      cudaFuncSetAttribute(k_key_series<1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSerSmemMax);
   if (e != cudaSuccess) return e;
   k_key_series<1, false><<<series_blocks(ne), kSerThreads, smem, st>>>(fs, g, 0, ne, keys, zt, kt, kNodeRows, F);
   k_key_finish<1><<<(nk + 127) / 128, 128, 0, st>>>(fs, g, 0, nk, 0, ne, keys, rval, zlev, jy, zt, kt, F);
