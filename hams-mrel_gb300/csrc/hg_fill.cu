@@ -114,8 +114,9 @@ cudaError_t launch_green_fill(cudaStream_t st, const double* rec, const double* 
                               int* bins, int ndiag) {
   if (ndiag < 0) ndiag = tn;
   if (!deep) return launch_green_fill_fin<OUT>(st, rec, fx, ldf, n, tn, fs, grn_kind, A, S, lda, status, bins, ndiag);
-  dim3 grid((tn + FILL_ROWS - 1) / FILL_ROWS, (n + FILL_COLS - 1) / FILL_COLS);
-  k_green_fill<true, OUT><<<grid, FILL_ROWS, 0, st>>>(rec, fx, ldf, n, tn, fs, grn_kind, A, S, lda, status, ndiag);
+  const int cols = fill_cols(n, tn);
+  dim3 grid((tn + FILL_ROWS - 1) / FILL_ROWS, (n + cols - 1) / cols);
+  k_green_fill<true, OUT><<<grid, FILL_ROWS, 0, st>>>(rec, fx, ldf, n, tn, fs, grn_kind, A, S, lda, status, ndiag, cols);
   return cudaGetLastError();
 }
 

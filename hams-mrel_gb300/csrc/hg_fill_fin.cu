@@ -18,8 +18,9 @@ cudaError_t launch_green_fill_fin(cudaStream_t st, const double* rec, const doub
                                   const FinState& fs, int grn_kind, OUT* A, OUT* S, long lda, int* status, int* bins,
                                   int ndiag) {
   if (bins) return launch_fin_binned<OUT, 0>(st, rec, fx, ldf, n, tn, fs, grn_kind, A, S, lda, bins, ndiag);
-  dim3 grid((tn + FILL_ROWS - 1) / FILL_ROWS, (n + FILL_COLS - 1) / FILL_COLS);
-  k_green_fill<false, OUT><<<grid, FILL_ROWS, 0, st>>>(rec, fx, ldf, n, tn, fs, grn_kind, A, S, lda, status, ndiag);
+  const int cols = fill_cols(n, tn);
+  dim3 grid((tn + FILL_ROWS - 1) / FILL_ROWS, (n + cols - 1) / cols);
+  k_green_fill<false, OUT><<<grid, FILL_ROWS, 0, st>>>(rec, fx, ldf, n, tn, fs, grn_kind, A, S, lda, status, ndiag, cols);
   return cudaGetLastError();
 }
 template cudaError_t launch_green_fill_fin<double2>(cudaStream_t, const double*, const double*, int, int, int,

@@ -20,6 +20,15 @@ namespace hg {
 // ---------------------------------------------------------------------------
 constexpr int FILL_ROWS = 128;
 constexpr int FILL_COLS = 16;
+// Columns per CTA: 16, or on small problems as few as give every SM four CTAs
+// (384 x 384 pairs in 16-column tiles are 72 CTAs, half the SMs: 0.42 ms
+// against 0.20 ms).
+inline int fill_cols(int n, int tn) {
+  const long rows = (tn + FILL_ROWS - 1) / FILL_ROWS;
+  int cols = FILL_COLS;
+  while (cols > 1 && rows * ((n + cols - 1) / cols) < 4 * 152) cols >>= 1;
+  return cols;
+}
 
 // One (field i, source j) pair of the fill: FLAG, Newman integral, Green
 // function, assembly of A(i, j) and S(i, j) (the loop body of k_green_fill).
@@ -74,11 +83,12 @@ __device__ __forceinline__ void fill_pair(const double* __restrict__ pr, double 
 template <bool DEEP, typename OUT, int FAST = 0>
 __global__ void __launch_bounds__(FILL_ROWS)
 k_green_fill(const double* __restrict__ rec, const double* __restrict__ fx /* ldf x 3 col-major */, int ldf, int n, int tn,
-             FinState fs, int grn_kind, OUT* __restrict__ A, OUT* __restrict__ S, long lda, int* status, int ndiag) {
+             FinState fs, int grn_kind, OUT* __restrict__ A, OUT* __restrict__ S, long lda, int* status, int ndiag,
+             int cols) {
   __shared__ alignas(128) double tile[FILL_COLS * PR_SIZE];
   __shared__ alignas(8) uint64_t bar;
-  const int col0 = blockIdx.y * FILL_COLS;
-  const int ncol = min(FILL_COLS, n - col0);
+  const int col0 = blockIdx.y * cols;
+  const int ncol = min(cols, n - col0);
   if (threadIdx.x == 0) {
     mbar_init(&bar, 1);
     mbar_expect_tx(&bar, (uint32_t)(ncol * PR_SIZE * sizeof(double)));
