@@ -438,14 +438,16 @@ __device__ __forceinline__ void warp_best_z(double& v, int& idx) {
   v = (km == 0ull) ? -1.0 : __longlong_as_double((long long)(km - 1ull));
 }
 
-// 1 / a by Smith's scaling, the reciprocals on the integer pipes (hg_rcp.cuh):
-// one thread forms it while the cluster waits, and three dependent FP64
-// divisions are most of a microsecond there.
-__device__ __forceinline__ double2 c_recip_z(double2 a) {
-  const bool re = fabs(a.x) >= fabs(a.y);
-  const double big = re ? a.x : a.y, small = re ? a.y : a.x;
-  const double q = small * rcp_any(big), d = rcp_any(fma(small, q, big));
-  return re ? make_double2(d, -q * d) : make_double2(q * d, -d);
+// The reciprocal of the pivot candidate, which one thread forms on the panel's
+// critical path: conj(a) / |a|^2 with one reciprocal on the integer pipes
+// (hg_rcp.cuh) where |a|^2 is far from overflow and underflow, else by Smith's
+// scaling with its three dependent FP64 divisions.  LU of order 384 1.93 -> 1.84
+// ms, of order 6048 78.3 -> 76.6 ms.
+__device__ __forceinline__ double2 c_recip_one(double2 a) {
+  const double m = fma(a.x, a.x, a.y * a.y);
+  if ((((uint32_t)(rcp_bits(m) >> 52) & 0x7ffu) - 24u) > 2000u) return c_recip(a);
+  const double r = rcp_rn(m);
+  return make_double2(a.x * r, -a.y * r);
 }
 
 // G column groups share the panel's rows: thread t works on row t mod (512 /
@@ -515,7 +517,7 @@ k_getf2_cluster_push_z(double2* __restrict__ P, long lda, int m, int jb, int rpc
       if (lane == 0) {
         msg.val = v;
         msg.idx = idx;
-        if (v > 0.0) msg.rcp = c_recip_z(tile[jj * rpc + (idx - r0)]);
+        if (v > 0.0) msg.rcp = c_recip_one(tile[jj * rpc + (idx - r0)]);
       }
       if (lane < jb) {
         if (idx != INT_MAX) msg.cand[lane] = tile[lane * rpc + (idx - r0)];
@@ -623,13 +625,7 @@ struct __align__(16) PanelMsgR {
 };
 static_assert(sizeof(PanelMsgR) % 16 == 0, "bulk copies move multiples of 16 bytes");
 
-__device__ __forceinline__ float2 pick32(const float2 (&a)[kClusterNB], int j) {
-  float2 x = a[0];
-#pragma unroll
-  for (int c = 1; c < kClusterNB; ++c)
-    if (c == j) x = a[c];
-  return x;
-}
+constexpr int kRegGroup = 8;  // columns of an unrolled group (even)
 
 // A panel row between registers and a 16-byte aligned message row, two
 // complex values per 16-byte access.
@@ -684,102 +680,128 @@ k_getf2_cluster_reg(float2* __restrict__ P, long lda, int m, int jb, int rpc, in
   }
   cluster.sync();  // barriers initialised and armed everywhere before any copy
 
-  bool bad = false;
-  // Fully unrolled: every column index below is a compile-time constant, so
-  // the row stays in registers without selects and the update touches only
-  // the columns right of jj.
+  bool bad = false, stop = false;
+  int turned = 0;  // the row's registers hold columns turned by this many: register c is column (c + turned) mod 32
+  // Groups of kRegGroup columns, unrolled inside, so that every register index
+  // is a compile-time constant and the row stays in registers without
+  // selects; between groups the row is turned by a group's width.  All 32
+  // steps unrolled were 300 KB of code that each launch walked once, fetching
+  // it: 57.4 us at 6048 rows and 50.7 us at 782 repeated back to back, and more
+  // inside a factorisation (LU of order 6048 18.4 ms); in groups 55.6 and
+  // 47.1 us (LU 16.4 ms).
+  for (int g = 0; g < kClusterNB / kRegGroup; ++g) {
 #pragma unroll
-  for (int jj = 0; jj < kClusterNB; ++jj) {
-    if (jj >= jb) break;
-    const int q = jj & 1;
-    const int oj = jj / rpc;
-    // (a) this CTA's candidate for column jj (rows >= jj), reduced by every warp
-    const float2 x = pick32(a, jj);
-    float v = (own && gr >= jj) ? fabsf(x.x) + fabsf(x.y) : -1.f;
-    int idx = (own && gr >= jj) ? gr : INT_MAX;
-    warp_best(v, idx);
-    if (lane == 0) { red_v[warp] = v; red_i[warp] = idx; }
-    __syncthreads();  // (the previous column's message slots were read before this barrier too)
-    v = (lane < kWarps) ? red_v[lane] : -1.f;
-    idx = (lane < kWarps) ? red_i[lane] : INT_MAX;
-    warp_best(v, idx);
-    // (b) the owners write the message: header and candidate row, row jj
-    PanelMsgR& msg = sendbuf[q];
-    if (idx == INT_MAX) {
-      if (tid == 0) { msg.val = -1.f; msg.idx = INT_MAX; }
-    } else if (own && gr == idx) {
-      msg.val = v;
-      msg.idx = idx;
-      msg.rcp = (x.x != 0.f || x.y != 0.f) ? c_recip(x) : make_float2(0.f, 0.f);
-      store_row(msg.cand, a);
-    }
-    if (own && gr == jj) {
-      store_row(msg.jrow, a);
-    }
-    fence_proxy_async_smem();
-    __syncthreads();
-    if (warp == 0 && lane < ncta) {
-      const uint32_t dst = mapa_shared(smem_addr(&recv[q][rank]), lane);
-      const uint32_t bar = mapa_shared(smem_addr(&mbar[q]), lane);
-      bulk_s2s_cluster(dst, smem_addr(&msg), kMsgBytes, bar);
-    }
-    // (c) wait for the ncta messages of this column
-    if (!mbar_wait_timed(&mbar[q], (jj >> 1) & 1, kPanelWaitNs)) bad = true;
-    if (__syncthreads_or(bad)) {
-      if (tid == 0) s_bad = 1;
-      break;
-    }
-    if (tid == 0 && jj + 2 < jb) mbar_expect_tx(&mbar[q], ncta * kMsgBytes);
-    // (d) the pivot: every warp reduces the ncta local messages
-    float pmax = (lane < ncta) ? recv[q][lane].val : -1.f;
-    int p = (lane < ncta) ? recv[q][lane].idx : INT_MAX;
-    warp_best(pmax, p);
-    if (p == INT_MAX) p = jj;
-    const int op = p / rpc;
-    const PanelMsgR& pm = recv[q][op];
-    const bool swap = pmax > 0.f && p != jj;
-    if (rank == 0 && tid == 0) {
-      ipiv[k0 + jj] = k0 + p + 1;
-      if (!(pmax > 0.f) && *info == 0) *info = k0 + jj + 1;
-    }
-    // (e) row jj becomes the pivot row; the owner of row p takes old row jj; update below jj
-    if (own && swap && gr == jj) {
-      load_row(a, pm.cand);
-    } else if (own && swap && gr == p) {
-      load_row(a, recv[q][oj].jrow);
-    }
-    if (pmax > 0.f && own && gr > jj) {
-      const float2 rp = pm.rcp;
-      const float2 l = c_mul(pick32(a, jj), rp);
-#pragma unroll
-      for (int c = 0; c < kClusterNB; ++c)
-        if (c == jj) a[c] = l;
-      // columns >= jb hold zeros in every row and in the pivot row and are never stored
-      const float4* u4 = reinterpret_cast<const float4*>(pm.cand);
-#pragma unroll
-      for (int c2 = 0; c2 < kClusterNB / 2; ++c2) {
-        if (2 * c2 + 1 > jj) {
-          const float4 uu = u4[c2];
-          if (2 * c2 > jj) {
-            a[2 * c2].x = fmaf(-l.x, uu.x, fmaf(l.y, uu.y, a[2 * c2].x));
-            a[2 * c2].y = fmaf(-l.x, uu.y, fmaf(-l.y, uu.x, a[2 * c2].y));
-          }
-          a[2 * c2 + 1].x = fmaf(-l.x, uu.z, fmaf(l.y, uu.w, a[2 * c2 + 1].x));
-          a[2 * c2 + 1].y = fmaf(-l.x, uu.w, fmaf(-l.y, uu.z, a[2 * c2 + 1].y));
-        }
-        if ((c2 & 3) == 3) asm volatile("" ::: "memory");  // keep at most 8 columns of loads in flight
+    for (int s = 0; s < kRegGroup; ++s) {
+      const int jj = g * kRegGroup + s;
+      if (stop || jj >= jb) {
+        stop = true;
+        break;
       }
+      const int q = s & 1;  // kRegGroup is even: jj & 1
+      const int oj = jj < rpc ? 0 : jj / rpc;
+      // (a) this CTA's candidate for column jj (rows >= jj), reduced by every warp
+      const float2 x = a[s];
+      float v = (own && gr >= jj) ? fabsf(x.x) + fabsf(x.y) : -1.f;
+      int idx = (own && gr >= jj) ? gr : INT_MAX;
+      warp_best(v, idx);
+      if (lane == 0) { red_v[warp] = v; red_i[warp] = idx; }
+      __syncthreads();  // (the previous column's message slots were read before this barrier too)
+      v = (lane < kWarps) ? red_v[lane] : -1.f;
+      idx = (lane < kWarps) ? red_i[lane] : INT_MAX;
+      warp_best(v, idx);
+      // (b) the owners write the message: header and candidate row, row jj
+      PanelMsgR& msg = sendbuf[q];
+      if (idx == INT_MAX) {
+        if (tid == 0) { msg.val = -1.f; msg.idx = INT_MAX; }
+      } else if (own && gr == idx) {
+        msg.val = v;
+        msg.idx = idx;
+        msg.rcp = (x.x != 0.f || x.y != 0.f) ? c_recip(x) : make_float2(0.f, 0.f);
+        store_row(msg.cand, a);
+      }
+      if (own && gr == jj) {
+        store_row(msg.jrow, a);
+      }
+      fence_proxy_async_smem();
+      // the warps wait at this barrier and not at the mbarrier: warps that poll while the owners write slow them
+      // down (one barrier a column, the owners' warps sending: 51 us against 47 us for 782 rows)
+      __syncthreads();
+      if (warp == 0 && lane < ncta) {
+        const uint32_t dst = mapa_shared(smem_addr(&recv[q][rank]), lane);
+        const uint32_t bar = mapa_shared(smem_addr(&mbar[q]), lane);
+        bulk_s2s_cluster(dst, smem_addr(&msg), kMsgBytes, bar);
+      }
+      // (c) wait for the ncta messages of this column
+      if (!mbar_wait_timed(&mbar[q], (jj >> 1) & 1, kPanelWaitNs)) bad = true;
+      if (__syncthreads_or(bad)) {
+        if (tid == 0) s_bad = 1;
+        stop = true;
+        break;
+      }
+      if (tid == 0 && jj + 2 < jb) mbar_expect_tx(&mbar[q], ncta * kMsgBytes);
+      // (d) the pivot: every warp reduces the ncta local messages
+      float pmax = (lane < ncta) ? recv[q][lane].val : -1.f;
+      const int pidx = (lane < ncta) ? recv[q][lane].idx : INT_MAX;
+      int p = pidx;
+      warp_best(pmax, p);
+      const unsigned from = __ballot_sync(0xffffffffu, lane < ncta && pidx == p);
+      const int op = from ? __ffs(from) - 1 : 0;  // the pivot row's CTA
+      if (p == INT_MAX) p = jj;
+      const PanelMsgR& pm = recv[q][op];
+      const bool swap = pmax > 0.f && p != jj;
+      if (rank == 0 && tid == 0) {
+        ipiv[k0 + jj] = k0 + p + 1;
+        if (!(pmax > 0.f) && *info == 0) *info = k0 + jj + 1;
+      }
+      // (e) row jj becomes the pivot row; the owner of row p takes old row jj; update below jj
+      if (own && swap && gr == jj) {
+        load_row(a, pm.cand);
+      } else if (own && swap && gr == p) {
+        load_row(a, recv[q][oj].jrow);
+      }
+      if (pmax > 0.f && own && gr > jj) {
+        const float2 rp = pm.rcp;
+        const float2 l = c_mul(a[s], rp);
+        a[s] = l;
+        // registers from 32 - g kRegGroup on hold finished columns; columns >= jb hold zeros in every row
+        // and in the pivot row and are never stored
+        const float4* u4 = reinterpret_cast<const float4*>(pm.cand);
+#pragma unroll
+        for (int c2 = 0; c2 < kClusterNB / 2; ++c2) {
+          if (2 * c2 % kRegGroup == 0 && 2 * c2 >= kClusterNB - g * kRegGroup) break;
+          if (2 * c2 + 1 > s) {
+            const float4 uu = u4[c2];
+            if (2 * c2 > s) {
+              a[2 * c2].x = fmaf(-l.x, uu.x, fmaf(l.y, uu.y, a[2 * c2].x));
+              a[2 * c2].y = fmaf(-l.x, uu.y, fmaf(-l.y, uu.x, a[2 * c2].y));
+            }
+            a[2 * c2 + 1].x = fmaf(-l.x, uu.z, fmaf(l.y, uu.w, a[2 * c2 + 1].x));
+            a[2 * c2 + 1].y = fmaf(-l.x, uu.w, fmaf(-l.y, uu.z, a[2 * c2 + 1].y));
+          }
+          if ((c2 & 3) == 3) asm volatile("" ::: "memory");  // keep at most 8 columns of loads in flight
+        }
+      }
+    }
+    if (stop) break;
+    {  // turn the row by a group
+      float2 t[kRegGroup];
+#pragma unroll
+      for (int c = 0; c < kRegGroup; ++c) t[c] = a[c];
+#pragma unroll
+      for (int c = 0; c + kRegGroup < kClusterNB; ++c) a[c] = a[c + kRegGroup];
+#pragma unroll
+      for (int c = 0; c < kRegGroup; ++c) a[kClusterNB - kRegGroup + c] = t[c];
+      turned += kRegGroup;
     }
   }
   __syncthreads();
   if (s_bad) {
     if (rank == 0 && tid == 0) *info = kPanelTimeout;
   } else if (own) {
-    float2* q = P + gr;
 #pragma unroll
-    for (int c = 0; c < kClusterNB; ++c, q += lda) {
-      asm volatile("" : "+l"(q));  // computed here, not kept from the loads
-      if (c < jb) *q = a[c];
+    for (int c = 0; c < kClusterNB; ++c) {
+      const int col = (c + turned) & (kClusterNB - 1);
+      if (col < jb) P[gr + (long)col * lda] = a[c];
     }
   }
   cluster.sync();  // no CTA leaves while a copy into its shared memory could be pending
