@@ -450,17 +450,17 @@ __device__ __forceinline__ double2 c_recip_one(double2 a) {
   return make_double2(a.x * r, -a.y * r);
 }
 
-// G column groups share the panel's rows: thread t works on row t mod (512 /
-// G) and columns t / (512 / G), + G, + 2 G, ...  The update is bound by the
+// G column groups share the panel's rows: thread t of NT works on row t mod (NT
+// / G) and columns t / (NT / G), + G, + 2 G, ...  The update is bound by the
 // FP64 pipe of the scheduler a warp sits on (one warp instruction takes 64
 // cycles there), so a short panel, whose rows would fill only a few warps,
 // spreads its columns over the others.  The thread that updates column jj + 1
 // takes its entry's |re| + |im| for the next pivot search from the register.
-template <int G>
-__global__ void __launch_bounds__(kClusterThreads, 1)
+template <int G, int NT>
+__global__ void __launch_bounds__(NT, 1)
 k_getf2_cluster_push_z(double2* __restrict__ P, long lda, int m, int jb, int rpc, int* __restrict__ ipiv, int k0,
                        int* __restrict__ info) {
-  constexpr int kWarps = kClusterThreads / 32, RT = kClusterThreads / G, NC = kPanelNBZ / G;
+  constexpr int kWarps = NT / 32, RT = NT / G, NC = kPanelNBZ / G;
   cg::cluster_group cluster = cg::this_cluster();
   const int rank = (int)cluster.block_rank();
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -893,26 +893,17 @@ cudaError_t panel_cluster<float>(cudaStream_t st, float2* P, long lda, int m, in
 }
 // Double precision: the pushed-candidate panel for panels of at most 16
 // columns whose tile fits beside its message buffers, else the loading panel.
-template <>
-cudaError_t panel_cluster<double>(cudaStream_t st, double2* P, long lda, int m, int jb, int* ipiv, int k0,
-                                  int* info) {
-  const int rpc = (m + kClusterCTAs - 1) / kClusterCTAs;
-  const size_t smem = (size_t)rpc * jb * sizeof(double2);
-  if (jb > kPanelNBZ || smem > (size_t)(kPanelSmemMax - kPushStaticSmem))
-    return panel_cluster_smem<double>(st, P, lda, m, jb, ipiv, k0, info);
-  // column groups: as many as leave every row of a CTA a thread
-  auto kern = k_getf2_cluster_push_z<1>;
-  if (rpc <= 32) kern = k_getf2_cluster_push_z<16>;
-  else if (rpc <= 64) kern = k_getf2_cluster_push_z<8>;
-  else if (rpc <= 128) kern = k_getf2_cluster_push_z<4>;
-  else if (rpc <= 256) kern = k_getf2_cluster_push_z<2>;
+template <int G, int NT>
+static cudaError_t launch_push_z(cudaStream_t st, size_t smem, double2* P, long lda, int m, int jb, int rpc, int* ipiv,
+                                 int k0, int* info) {
+  auto kern = k_getf2_cluster_push_z<G, NT>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kPanelSmemMax - kPushStaticSmem);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(kClusterCTAs, 1, 1);
-  cfg.blockDim = dim3(kClusterThreads, 1, 1);
+  cfg.blockDim = dim3(NT, 1, 1);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
@@ -925,6 +916,23 @@ cudaError_t panel_cluster<double>(cudaStream_t st, double2* P, long lda, int m, 
   return cudaLaunchKernelEx(&cfg, kern, P, lda, m, jb, rpc, ipiv, k0, info);
 }
 
+template <>
+cudaError_t panel_cluster<double>(cudaStream_t st, double2* P, long lda, int m, int jb, int* ipiv, int k0,
+                                  int* info) {
+  const int rpc = (m + kClusterCTAs - 1) / kClusterCTAs;
+  const size_t smem = (size_t)rpc * jb * sizeof(double2);
+  if (jb > kPanelNBZ || smem > (size_t)(kPanelSmemMax - kPushStaticSmem))
+    return panel_cluster_smem<double>(st, P, lda, m, jb, ipiv, k0, info);
+  // As many threads as the rows of a CTA need, and column groups while the rows are few: warps beyond that
+  // only wait, and their polls and barriers slow the others (512 threads in 16, 8, 4 and 2 groups: LU of order
+  // 384 1.84 ms, of 1536 12.6 ms; so 1.58 and 11.9 ms)
+  if (rpc <= 32) return launch_push_z<4, 128>(st, smem, P, lda, m, jb, rpc, ipiv, k0, info);
+  if (rpc <= 64) return launch_push_z<4, 256>(st, smem, P, lda, m, jb, rpc, ipiv, k0, info);
+  if (rpc <= 128) return launch_push_z<2, 256>(st, smem, P, lda, m, jb, rpc, ipiv, k0, info);
+  if (rpc <= 256) return launch_push_z<1, 256>(st, smem, P, lda, m, jb, rpc, ipiv, k0, info);
+  if (rpc <= 384) return launch_push_z<1, 384>(st, smem, P, lda, m, jb, rpc, ipiv, k0, info);
+  return launch_push_z<1, 512>(st, smem, P, lda, m, jb, rpc, ipiv, k0, info);
+}
 
 // Whether a 16-CTA cluster with the given dynamic shared memory can run here.
 template <typename R>
