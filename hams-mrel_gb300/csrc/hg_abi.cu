@@ -109,6 +109,8 @@ struct hg_ctx {
   DevBuf<double> gpts;                   // workspace of hg_green_points
   DevBuf<double> fpx;
   DevBuf<int> fonb;
+  DevBuf<float4> fplane;                 // panel planes and reaches of the on-body test
+  DevBuf<float> freach;
   DevBuf<double2> fA, fS, fW, fWn, fout, fout2;  // fWn: -fW, for the tensor-core products
   DevBuf<float2> fAf, fSf;
   int inner_its = 0;                     // GMRES iterations of the last solve
@@ -1473,6 +1475,9 @@ int hg_field_points(hg_ctx* c, int npts, const double* xyz, int kind, int isol, 
   const int ldc = (chunk + 1) & ~1;  // even leading dimension: 16-byte aligned columns of complex64
   CK(c->fpx.ensure((size_t)chunk * 3));
   CK(c->fonb.ensure(chunk));
+  CK(c->fplane.ensure(n));
+  CK(c->freach.ensure(n));
+  CK(hg::launch_field_planes(c->st, n, c->ntnd, c->nodes.p, c->ncon.p, c->dxyz.p, c->pnsz.p, c->fplane.p, c->freach.p));
   CK(c->fW.ensure((size_t)n * ncol));
   CK(c->fout.ensure((size_t)chunk * ncol));
   if (fast) {
@@ -1506,7 +1511,7 @@ int hg_field_points(hg_ctx* c, int npts, const double* xyz, int kind, int isol, 
       for (int k = 0; k < 3; ++k) hx[p + (size_t)k * m] = xyz[3 * (size_t)(p0 + p) + k];
     CK(cudaMemcpyAsync(c->fpx.p, hx.data(), (size_t)m * 3 * sizeof(double), cudaMemcpyHostToDevice, c->st));
     CK(hg::launch_field_on_body(c->st, m, c->fpx.p, m, n, c->ntnd, c->nodes.p, c->ncon.p, c->ncn.p, c->dxyz.p,
-                                c->pnsz.p, c->fonb.p));
+                                c->pnsz.p, c->fplane.p, c->freach.p, c->fonb.p));
     // rows = field points, no free term: A rows = DUM2, S rows = DUM1
     if (fast) {
       const int ldm = (m + 1) & ~1;

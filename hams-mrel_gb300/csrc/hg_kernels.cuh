@@ -87,9 +87,12 @@ cudaError_t launch_rhs_cols(cudaStream_t st, int n, const double* dxyz_p, const 
 // Field points (hg_field.cu): onb[p] = 1 where point p (npts x 3 column-major,
 // leading dimension ldp) lies on a panel; the finishing pass of the field
 // potentials acc (npts x ncol, columns >= nrad are diffraction headings).
+// launch_field_planes: the n panels' planes and reaches, which rule out most panels.
+cudaError_t launch_field_planes(cudaStream_t st, int n, int ntnd, const double* nodes, const int* ncon, const double* dxyz,
+                                const double* pnsz, float4* plane, float* reach);
 cudaError_t launch_field_on_body(cudaStream_t st, int npts, const double* px, int ldp, int n, int ntnd,
                                  const double* nodes, const int* ncon, const int* ncn, const double* dxyz,
-                                 const double* pnsz, int* onb);
+                                 const double* pnsz, const float4* plane, const float* reach, int* onb);
 cudaError_t launch_field_finish(cudaStream_t st, int npts, int ncol, int nrad, double2* acc, long lda, const int* onb,
                                 const double* px, int ldp, const double* betas, double v, double wk, double w1,
                                 double h, double g, double rho, int isol, int kind);
