@@ -28,7 +28,9 @@ __global__ void k_field_planes(int n, int ntnd, const double* __restrict__ nodes
   const int a0 = ncon[j] - 1;
   const double c = -(nodes[a0] * e0 + nodes[a0 + ntnd] * e1 + nodes[a0 + 2 * (size_t)ntnd] * e2);
   plane[j] = make_float4((float)e0, (float)e1, (float)e2, (float)c);
-  reach[j] = (float)(1.001 * fmax(1.0e-6, 1.0e-3 * pnsz[j]) + kPlaneErr * fabs(c));
+  // a normal that is not of unit length takes the test itself: the error bound is for |n| = 1
+  const bool unit = fabs(e0) <= 1.01 && fabs(e1) <= 1.01 && fabs(e2) <= 1.01;
+  reach[j] = unit ? (float)(1.001 * fmax(1.0e-6, 1.0e-3 * pnsz[j]) + kPlaneErr * fabs(c)) : INFINITY;
 }
 
 // Is point (x, y, z) on panel j's surface?  The test of
