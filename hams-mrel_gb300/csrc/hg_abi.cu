@@ -1758,9 +1758,10 @@ size_t hg_solve_footprint(int precision, int n, int nl, int nbody, int nbeta, in
   size_t b = 0;
   // mesh: node and panel arrays, 288-byte panel records, field points
   b += nn * (4 * sizeof(int) + 12 * sizeof(double) + 36 * sizeof(double)) + (nn + nl) * 3 * sizeof(double);
-  // finite depth: one int per pair for the cost-binned fill; in the mixed form also the near pairs'
+  // finite depth: one int per pair for the cost-binned fill; in the mixed form also the pairs'
   // map (pair index and key slot, 8 bytes per pair, and the keys, 16 bytes each, at most one per pair; their
-  // values are 48 bytes per distinct key)
+  // values are 48 bytes per distinct key).  The plain form's keys are not counted: they are built only
+  // into a quarter of the memory left free, and without them the cost-binned fill runs.
   b += sizeof(int) * tn * nn;
   if (precision == HG_PREC_MIXED) b += 24 * tn * nn;
   // right-hand sides, solutions, source weights, split-K workspace

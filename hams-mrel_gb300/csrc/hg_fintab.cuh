@@ -22,8 +22,9 @@
 // are cell-centred (W = 0 is never a node); the U nodes are uniform in
 // t = log(1 + |U|/u0), shifted by half a step (U = 0 is never a node).
 // Pairs interpolate both tables bicubically (Catmull-Rom) in single precision.
-// Below R/h = 0.05 the fill evaluates the pairs again per pair in FP64
-// (launch_fin_near): LINTON's and PIDCOCK's values are not smooth in R.
+// Below R/h = 0.05 the fill evaluates the pairs again in FP64 (per distinct
+// geometry, fin_keys_fill; per pair, launch_fin_near, when the keys do not
+// fit): LINTON's and PIDCOCK's values are not smooth in R.
 // The propagating-wave term of F (the k0 mode: p0 (-Y0, J0)(k0 R) with
 // p0 = pi/N0 cosh(k0(zq+h)) cosh(k0(zp+h)), and its derivatives; the
 // d_prop_part of FinGreen3D.f90:281-362) oscillates on the wavelength scale

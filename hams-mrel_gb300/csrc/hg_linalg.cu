@@ -1,6 +1,7 @@
 // Blocked complex LU with partial pivoting and triangular solves.
 //
-// getrf: right-looking, panel width NB = 32.  Per panel: the panel
+// getrf: right-looking, panel width NB = 32 (16 for complex128 with an update
+// kernel of its own, see factor_columns).  Per panel: the panel
 // factorisation (16-CTA cluster kernel, or one CTA when a cluster does not
 // fit: pivot = max |re|+|im| as LAPACK's IZAMAX, row swaps, reciprocal
 // scaling, rank-1 updates), the row interchanges applied to the columns
