@@ -601,19 +601,39 @@ def _launch_count(n, prec, sweeps=1, nd=30, nbeta=8, lu_tensor=2):
     """Kernels the library launches per frequency-solve, from its launch
     sequence (checked against the ncu launch list of one solve)."""
     nb, nbo = 32, 256
+
+    def steps64(jb):  # a complex128 triangle 64 rows at a time: solves, and updates of the rows still to solve
+        q = (jb + 63) // 64
+        return 2 * q - 1
+
+    def blocks64(update):  # forward and backward over the 256-row blocks, the interchanges first
+        sizes = [min(nbo, n - k) for k in range(0, n, nbo)]
+        return 1 + 2 * sum(steps64(jb) for jb in sizes) + 2 * update * (len(sizes) - 1)
+
     if prec == 0 and n >= 1024 and lu_tensor != 0:
         # FP64 form on the tensor cores: each sliced product is 3 kernels (A's digits, B's digits,
-        # the product).  Per outer panel of jbo columns: p = jbo / 16 panels, their interchanges
-        # and L11 solves (when jbo > 16), p - 1 inner products, the other columns' interchanges; where
-        # columns remain: I, L11^-1, the U12 operands, three U12 products and the trailing one.
+        # the product), in passes of 256 of its inner dimension.  Per outer panel of jbo columns: p =
+        # jbo / 16 panels, their interchanges and L11 solves (when jbo > 16), p - 1 inner updates (one
+        # kernel up to 400 000 entries, a sliced product beyond), the other columns' interchanges;
+        # where columns remain: I, L11^-1 by 64 rows, the U12 operands, three U12 products and the
+        # trailing one.
         lu = 0
         for k in range(0, n, nbo):
             jbo = min(nbo, n - k)
             p = (jbo + 15) // 16
-            lu += p + (p if jbo > 16 else 0) + 3 * (p - 1) + 1 + (15 if n - k - jbo > 0 else 0)
-        blocks = (n + nbo - 1) // nbo
-        getrs = 1 + 2 * blocks + 3 * 2 * (blocks - 1)
-        return 1 + lu + 3 + getrs + 1  # fill, LU, incident / source columns / S W, solves, forces
+            lu += p + (p if jbo > 16 else 0) + 1
+            for c in range(k, k + jbo, 16):
+                rest = k + jbo - c - 16
+                if rest > 0:
+                    lu += 1 if (n - c - 16) * rest <= 400000 else 3
+            if n - k - jbo > 0:
+                lu += 2 + steps64(jbo) + 12
+        rhs = 3 + 3 * ((n + 255) // 256)  # incident, source columns, their sign, S W
+        return 1 + lu + rhs + blocks64(3) + 1  # fill, LU, right-hand sides, solves, forces
+    if prec == 0 and n < 1024:
+        p = (n + 15) // 16  # 16-wide panels, their interchanges, the updates between them
+        return 1 + (p + (p if n > 16 else 0) + p - 1) + 3 + blocks64(1) + 1
+
     def inner(jb, split=False):  # 32-wide panels: panel + fused interchanges / L11 solve, then the update
         p = (jb + nb - 1) // nb   # while columns remain (the FP64 form splits it: next panel's columns, the rest)
         return 2 * p + ((2 * p - 3 if p >= 2 else 0) if split else p - 1)
@@ -633,7 +653,7 @@ def _launch_count(n, prec, sweeps=1, nd=30, nbeta=8, lu_tensor=2):
     fill = 2 if prec == 1 else 1  # mixed deep water: the FP32 tile kernel and the self/adjacent-pair kernel
     forces = 1
     if prec == 0:
-        return fill + lu + 3 + getrs + forces      # incident weights, source columns, S W product
+        return fill + lu + 3 + blocks64(1) + forces  # incident weights, S W product in two kernels
     # mixed: RHS (incident, source columns, S W as a split product: 3 kernels);
     # 1 + sweeps solves, each followed by a residual check (product, split,
     # reduce) and bracketed by conversions; column norms of B and of each residual
