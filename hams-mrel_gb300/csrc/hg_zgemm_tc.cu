@@ -122,13 +122,30 @@ __device__ __forceinline__ double oz_scale2(double v, int sc) {
   return ldexp(v, sc);
 }
 
+// The kZD digits of two neighbouring entries, a word each (p even: kp is, and
+// k where the caller adds it).
+__device__ __forceinline__ void oz_store2(uint16_t* p, size_t slice, const uint16_t* d0, const uint16_t* d1) {
+#pragma unroll
+  for (int s = 0; s < kZD; ++s)
+    *reinterpret_cast<uint32_t*>(p + s * slice) = (uint32_t)d0[s] | ((uint32_t)d1[s] << 16);
+}
+
 // A's digits: [kZD][mp][kp] BF16 rows (K fastest), row i holding Ar(i, :) at
 // 0..k-1 and Ai(i, :) at k..2k-1, zero beyond (rows m..mp-1, K 2k..kp-1);
 // ex[i] the row's exponent.  The operand is A (m x k, A[i + p lda]) or, with
 // TRANS, the transpose of the k x m matrix A (A[p + i lda]: its rows are A's
-// columns).  One CTA per 32 rows: their largest entries first, then 32 x 32
+// columns).  A row block is 32 rows: their largest entries first, then 32 x 32
 // tiles through shared memory (transposed for A, direct for TRANS), so that
-// the reads of A and the digit writes are both coalesced.
+// the reads of A and the digit writes are both coalesced.  The tiles of a row
+// block go to gridDim.y CTAs, each of which looks for the largest entries
+// itself (from L2): with one CTA a row block the kernel waited on its loads, 8
+// CTAs for a 256-row operand and about one an SM for the matrix's rows.  Even k:
+// two entries a thread, so that the 2-byte digits leave as words.  In the LU
+// and solves of order 6048: A's digits 7.1 -> 3.5 ms, B's 3.2 -> 2.6 ms, LU
+// 75.4 -> 72.9 ms (73.1 with one CTA a row block), solves 15.0 -> 13.5 ms (14.0);
+// 2, 8 and 16 CTAs an SM the same to 0.1 ms.
+constexpr int kZSliceCtas = 4;
+
 template <bool TRANS>
 __global__ void __launch_bounds__(256) k_zoz_slice_a(int m, int k, int mp, int kp, const double2* __restrict__ A,
                                                      long lda, int* __restrict__ ex, uint16_t* __restrict__ D) {
@@ -141,6 +158,7 @@ __global__ void __launch_bounds__(256) k_zoz_slice_a(int m, int k, int mp, int k
       const int i = i0 + r;
       unsigned long long amax = 0;
       if (i < m)
+#pragma unroll 8
         for (int p = tx; p < k; p += 32) {
           const double2 a = A[p + (long)i * lda];
           amax = max(amax, max(oz_abs_bits(a.x), oz_abs_bits(a.y)));
@@ -150,7 +168,7 @@ __global__ void __launch_bounds__(256) k_zoz_slice_a(int m, int k, int mp, int k
       if (tx == 0) {
         const int e = oz_exp_bits(amax);
         es[r] = e;
-        if (i < mp) ex[i] = e;
+        if (i < mp && blockIdx.y == 0) ex[i] = e;
       }
     }
     __syncthreads();
@@ -158,6 +176,7 @@ __global__ void __launch_bounds__(256) k_zoz_slice_a(int m, int k, int mp, int k
     unsigned long long amax = 0;
     const int i = i0 + tx;
     if (i < m)
+#pragma unroll 8
       for (int p = ty; p < k; p += 8) {
         const double2 a = A[i + (long)p * lda];
         amax = max(amax, max(oz_abs_bits(a.x), oz_abs_bits(a.y)));
@@ -168,12 +187,12 @@ __global__ void __launch_bounds__(256) k_zoz_slice_a(int m, int k, int mp, int k
       for (int r = 1; r < 8; ++r) amax = max(amax, red[r][tx]);
       const int e = oz_exp_bits(amax);
       es[tx] = e;
-      if (i < mp) ex[i] = e;
+      if (i < mp && blockIdx.y == 0) ex[i] = e;
     }
     __syncthreads();
   }
   const size_t slice = (size_t)mp * kp;
-  for (int p0 = 0; p0 < k; p0 += 32) {
+  for (int p0 = 32 * blockIdx.y; p0 < k; p0 += 32 * gridDim.y) {
     for (int r = ty; r < 32; r += 8) {
       if (TRANS) {  // t[r][tx] = op(i0 + r, p0 + tx)
         const int i = i0 + r, p = p0 + tx;
@@ -184,6 +203,24 @@ __global__ void __launch_bounds__(256) k_zoz_slice_a(int m, int k, int mp, int k
       }
     }
     __syncthreads();
+    if (k % 2 == 0) {  // two entries a thread, half a warp a row
+#pragma unroll 1
+      for (int r = ty + 8 * (tx >> 4); r < 32; r += 16) {
+        const int i = i0 + r, q = 2 * (tx & 15), p = p0 + q;
+        if (i >= mp || p >= k) continue;
+        const double2 a = TRANS ? t[r][q] : t[q][r], b = TRANS ? t[r][q + 1] : t[q + 1][r];
+        uint16_t d0[kZD], d1[kZD];
+        uint16_t* row = D + (size_t)i * kp + p;
+        oz_digits_d(a.x, es[r], d0);
+        oz_digits_d(b.x, es[r], d1);
+        oz_store2(row, slice, d0, d1);
+        oz_digits_d(a.y, es[r], d0);
+        oz_digits_d(b.y, es[r], d1);
+        oz_store2(row + k, slice, d0, d1);
+      }
+      __syncthreads();
+      continue;
+    }
     for (int r = ty; r < 32; r += 8) {
       const int i = i0 + r, p = p0 + tx;
       if (i >= mp || p >= k) continue;
@@ -201,7 +238,7 @@ __global__ void __launch_bounds__(256) k_zoz_slice_a(int m, int k, int mp, int k
     __syncthreads();
   }
   const int w = kp - 2 * k;
-  if (w > 0)
+  if (w > 0 && blockIdx.y == 0)
     for (int e = ty * 32 + tx; e < kZD * 32 * w; e += 256) {
       const int c = e % w, r = (e / w) % 32, s = e / (w * 32);
       if (i0 + r < mp) D[s * slice + (size_t)(i0 + r) * kp + 2 * k + c] = 0;
@@ -232,7 +269,26 @@ __global__ void __launch_bounds__(256) k_zoz_slice_b(int k, int n, int np, int k
   const size_t slice = (size_t)np * kp;
   uint16_t* re = G + (size_t)(2 * j) * kp;
   uint16_t* im = re + kp;
-  for (int p = lane; p < k; p += 32) {
+  if (k % 2 == 0) {  // two entries a thread
+    for (int p = 2 * lane; p < k; p += 64) {
+      uint16_t r0[kZD], r1[kZD], i0[kZD], i1[kZD];
+      const double2 y = live ? col[p] : make_double2(0.0, 0.0), z = live ? col[p + 1] : make_double2(0.0, 0.0);
+      oz_digits_d(y.x, f, r0);
+      oz_digits_d(z.x, f, r1);
+      oz_store2(re + p, slice, r0, r1);
+      oz_store2(im + k + p, slice, r0, r1);
+      oz_digits_d(y.y, f, i0);
+      oz_digits_d(z.y, f, i1);
+      oz_store2(im + p, slice, i0, i1);
+#pragma unroll
+      for (int s = 0; s < kZD; ++s) {
+        i0[s] ^= 0x8000u;
+        i1[s] ^= 0x8000u;
+      }
+      oz_store2(re + k + p, slice, i0, i1);
+    }
+  }
+  for (int p = k % 2 == 0 ? k : lane; p < k; p += 32) {
     uint16_t dr[kZD], di[kZD];
     const double2 y = live ? col[p] : make_double2(0.0, 0.0);
     oz_digits_d(y.x, f, dr);
@@ -477,10 +533,13 @@ cudaError_t zgemm_tc(cudaStream_t st, int m, int n, int k, const double2* A, lon
     uint16_t* Bd = reinterpret_cast<uint16_t*>(w + lw.b_off);
     int* ex = reinterpret_cast<int*>(w + lw.ex_off);
     int* fx = reinterpret_cast<int*>(w + lw.fx_off);
+    // A's tiles over as many CTAs as give every SM kZSliceCtas, at most one each
+    const int rows = lw.mp / 32, want = (kZSliceCtas * (g_z_sms > 0 ? g_z_sms : 152) + rows - 1) / rows;
+    const dim3 ga(rows, std::min((kc + 31) / 32, want));
     if (transa)
-      k_zoz_slice_a<true><<<lw.mp / 32, dim3(32, 8), 0, st>>>(m, kc, lw.mp, lw.kp, A + k0, lda, ex, Ad);
+      k_zoz_slice_a<true><<<ga, dim3(32, 8), 0, st>>>(m, kc, lw.mp, lw.kp, A + k0, lda, ex, Ad);
     else
-      k_zoz_slice_a<false><<<lw.mp / 32, dim3(32, 8), 0, st>>>(m, kc, lw.mp, lw.kp, A + (long)k0 * lda, lda, ex, Ad);
+      k_zoz_slice_a<false><<<ga, dim3(32, 8), 0, st>>>(m, kc, lw.mp, lw.kp, A + (long)k0 * lda, lda, ex, Ad);
     k_zoz_slice_b<<<(lw.np / 2 + 7) / 8, 256, 0, st>>>(kc, n, lw.np, lw.kp, B + k0, ldb, fx, Bd);
     CUtensorMap ma, mb;
     if (!oz_map(&ma, Ad, lw.kp, kZD * lw.mp, kZTM) || !oz_map(&mb, Bd, lw.kp, kZD * lw.np, kZTN))
