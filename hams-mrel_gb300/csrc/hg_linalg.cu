@@ -939,8 +939,13 @@ cudaError_t getrs_inv(cudaStream_t st, int n, int nrhs, const float2* LU, long l
 // upper), one CTA per column.  A thread holds the real or the imaginary part
 // of one row: a step of the substitution is then two dependent fused
 // operations on each scheduler, one warp instruction of which occupies its
-// FP64 pipe for 64 cycles, and one barrier.  17 us (lower) and 31 us (upper)
-// for 64 rows; 16 rows at a time by one warp with shuffles took 48 and 41 us.
+// FP64 pipe for 64 cycles, and one barrier.  An upper triangle's columns are
+// divided by their diagonal first, all at once, and the solution at the end, so
+// that its steps are the lower one's: 18 us (lower) and 22 us (upper) for 64
+// rows, 31 us with the product by the reciprocal inside each step; 16 rows at a
+// time by one warp with shuffles took 48 and 41 us.  Forward errors of random
+// and collocation-like systems of order 384 against extended precision are the
+// same to 1 % either way.
 constexpr int kSolveZ = 64;
 template <bool UPPER>
 __global__ void __launch_bounds__(2 * kSolveZ)
@@ -959,25 +964,32 @@ k_trsm64_z(const double2* __restrict__ A, long lda, int w, double2* __restrict__
   if (UPPER) {
     __syncthreads();
     if (part == 0 && row < w) rd[row] = crecip(t[row * kSolveZ + row]);
+    __syncthreads();
+    // columns p and w - 1 - p together have w - 1 entries above the diagonal
+    for (int p = part; 2 * p <= w - 1; p += 2) {
+      const int j = row < p ? p : w - 1 - p, i = row < p ? row : row - p;
+      if (row >= w - 1 || (2 * p == w - 1 && row >= p)) continue;
+      const double2 a = t[j * kSolveZ + i], r = rd[j];
+      t[j * kSolveZ + i] = make_double2(fma(-a.y, r.y, a.x * r.x), fma(a.y, r.x, a.x * r.y));
+    }
   }
   for (int q = 0; q < w; ++q) {
     const int j = UPPER ? w - 1 - q : q;
     if (row == j) xs[j][part] = v;
-    __syncthreads();  // also the triangle and the reciprocals on the first step
-    double xr = xs[j][0], xi = xs[j][1];
-    if (UPPER) {
-      const double2 r = rd[j];
-      const double yr = fma(-xi, r.y, xr * r.x);
-      xi = fma(xi, r.x, xr * r.y);
-      xr = yr;
-      if (row == j) v = part ? xi : xr;
-    }
+    __syncthreads();  // also the triangle on the first step
+    const double xr = xs[j][0], xi = xs[j][1];
     if (row < w && (UPPER ? row < j : row > j)) {
       const double2 l = t[j * kSolveZ + row];
       v = part ? fma(-l.y, xr, fma(-l.x, xi, v)) : fma(l.y, xi, fma(-l.x, xr, v));
     }
   }
-  if (row < w) *xc = v;
+  if (row >= w) return;
+  if (UPPER) {
+    const double xr = xs[row][0], xi = xs[row][1];
+    const double2 r = rd[row];
+    v = part ? fma(xi, r.x, xr * r.y) : fma(-xi, r.y, xr * r.x);
+  }
+  *xc = v;
 }
 
 cudaError_t trsm64_z(cudaStream_t st, bool upper, const double2* A, long lda, int w, double2* X, long ldx, int ncols) {
