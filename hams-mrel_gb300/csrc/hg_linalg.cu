@@ -520,7 +520,12 @@ cudaError_t panel(cudaStream_t st, bool use_cluster, int n, typename cx<R>::T* A
 // complex128 panels) on the FP64 pipes: a 16 x 16 tile of C per CTA of 64
 // threads, operands staged once.  With two FP64 operations a clock and SM the
 // product is bound by that pipe, and small tiles are what spreads it evenly
-// over the SMs.
+// over the SMs.  The product is summed by itself and subtracted at the end, one
+// rounding at C's size: C's largest entries are the diagonal's 2 pi, and
+// summing into C rounded them 32 times an update.  Forward error of
+// collocation-like systems of order 627 with that 1.2e-15, so (and with one
+// rounding a step in k_trsm64_z) 4.6e-16; the solve at order 384 2.31 and 2.34
+// ms.
 constexpr int kZupdT = 16, kZupdK = 16;
 __global__ void __launch_bounds__(64)
 k_zupdate(int m, int n, int k, const double2* __restrict__ A, long lda, const double2* __restrict__ B, long ldb,
@@ -528,13 +533,14 @@ k_zupdate(int m, int n, int k, const double2* __restrict__ A, long lda, const do
   __shared__ double2 as[kZupdK][kZupdT], bs[kZupdK][kZupdT + 1];
   const int m0 = blockIdx.x * kZupdT, n0 = blockIdx.y * kZupdT;
   const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3;  // rows tx, tx + 8; columns ty, ty + 8
-  double2 c[2][2];
+  double2 c[2][2], p[2][2];
 #pragma unroll
   for (int j = 0; j < 2; ++j)
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
       const int r = m0 + tx + 8 * i, q = n0 + ty + 8 * j;
       c[i][j] = (r < m && q < n) ? C[r + (long)q * ldc] : make_double2(0.0, 0.0);
+      p[i][j] = make_double2(0.0, 0.0);
     }
 #pragma unroll
   for (int e = threadIdx.x; e < kZupdK * kZupdT; e += 64) {
@@ -550,8 +556,8 @@ k_zupdate(int m, int n, int k, const double2* __restrict__ A, long lda, const do
     for (int i = 0; i < 2; ++i)
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
-        c[i][j].x = fma(a[i].y, b[j].y, fma(-a[i].x, b[j].x, c[i][j].x));
-        c[i][j].y = fma(-a[i].y, b[j].x, fma(-a[i].x, b[j].y, c[i][j].y));
+        p[i][j].x = fma(-a[i].y, b[j].y, fma(a[i].x, b[j].x, p[i][j].x));
+        p[i][j].y = fma(a[i].y, b[j].x, fma(a[i].x, b[j].y, p[i][j].y));
       }
   }
 #pragma unroll
@@ -559,7 +565,7 @@ k_zupdate(int m, int n, int k, const double2* __restrict__ A, long lda, const do
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
       const int r = m0 + tx + 8 * i, q = n0 + ty + 8 * j;
-      if (r < m && q < n) C[r + (long)q * ldc] = c[i][j];
+      if (r < m && q < n) C[r + (long)q * ldc] = make_double2(c[i][j].x - p[i][j].x, c[i][j].y - p[i][j].y);
     }
 }
 // Up to this many entries of C the update runs there, beyond it as sliced
@@ -937,15 +943,16 @@ cudaError_t getrs_inv(cudaStream_t st, int n, int nrhs, const float2* LU, long l
 
 // X = T^-1 X in complex128 for a triangle of at most 64 rows (unit lower, or
 // upper), one CTA per column.  A thread holds the real or the imaginary part
-// of one row: a step of the substitution is then two dependent fused
-// operations on each scheduler, one warp instruction of which occupies its
-// FP64 pipe for 64 cycles, and one barrier.  An upper triangle's columns are
+// of one row: a step of the substitution is then a product of its own and a
+// difference (one rounding at the row's size) on each scheduler, one warp
+// instruction of which occupies its FP64 pipe for 64 cycles, and one barrier.  An upper triangle's columns are
 // divided by their diagonal first, all at once, and the solution at the end, so
-// that its steps are the lower one's: 18 us (lower) and 22 us (upper) for 64
-// rows, 31 us with the product by the reciprocal inside each step; 16 rows at a
-// time by one warp with shuffles took 48 and 41 us.  Forward errors of random
-// and collocation-like systems of order 384 against extended precision are the
-// same to 1 % either way.
+// that its steps are the lower one's: 20 us (lower) and 24 us (upper) for 64
+// rows; with two roundings a step in place of one 18 and 22 us, with the
+// product by the reciprocal inside each step of the upper triangle 31 us, and 16
+// rows at a time by one warp with shuffles 48 and 41 us.  The scaling leaves
+// forward errors of random and collocation-like systems of order 384 the same to
+// 1 %.
 constexpr int kSolveZ = 64;
 template <bool UPPER>
 __global__ void __launch_bounds__(2 * kSolveZ)
@@ -980,7 +987,7 @@ k_trsm64_z(const double2* __restrict__ A, long lda, int w, double2* __restrict__
     const double xr = xs[j][0], xi = xs[j][1];
     if (row < w && (UPPER ? row < j : row > j)) {
       const double2 l = t[j * kSolveZ + row];
-      v = part ? fma(-l.y, xr, fma(-l.x, xi, v)) : fma(l.y, xi, fma(-l.x, xr, v));
+      v -= part ? fma(l.y, xr, l.x * xi) : fma(-l.y, xi, l.x * xr);  // one rounding at v's size
     }
   }
   if (row >= w) return;

@@ -456,7 +456,11 @@ __device__ __forceinline__ double2 c_recip_one(double2 a) {
 // cycles there), so a short panel, whose rows would fill only a few warps,
 // spreads its columns over the others.  The thread that updates column jj + 1
 // takes its entry's |re| + |im| for the next pivot search from the register.
-template <int G, int NT>
+// ONE: an update rounds once at the entry's size, with a third FP64 operation
+// (the product, its sum, the difference); else twice.  Inside a panel that is
+// 16 roundings at most, which the order's other n / 16 outweigh except in small
+// systems: see kOneRounding.
+template <int G, int NT, bool ONE>
 __global__ void __launch_bounds__(NT, 1)
 k_getf2_cluster_push_z(double2* __restrict__ P, long lda, int m, int jb, int rpc, int* __restrict__ ipiv, int k0,
                        int* __restrict__ info) {
@@ -581,8 +585,12 @@ k_getf2_cluster_push_z(double2* __restrict__ P, long lda, int m, int jb, int rpc
         const int c = g + t * G;
         if (c > jj && c < jb) {
           const double2 u = prow[c];
-          a[t].x = fma(l.y, u.y, fma(-l.x, u.x, a[t].x));
-          a[t].y = fma(-l.y, u.x, fma(-l.x, u.y, a[t].y));
+          if (ONE) {
+            a[t] = c_sub(a[t], c_mul(l, u));
+          } else {
+            a[t].x = fma(l.y, u.y, fma(-l.x, u.x, a[t].x));
+            a[t].y = fma(-l.y, u.x, fma(-l.x, u.y, a[t].y));
+          }
           tile[c * rpc + r] = a[t];
           if (c == jj + 1) consider(a[t], gr);
         } else if (c == jj) {
@@ -891,12 +899,20 @@ cudaError_t panel_cluster<float>(cudaStream_t st, float2* P, long lda, int m, in
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, k_getf2_cluster_push, P, lda, m, jb, rpc, ipiv, k0, info);
 }
+// Largest order whose complex128 panels round an update once.  Forward errors of
+// collocation-like systems (geometric mean, 1e-16) with one and two roundings:
+// order 8 1.70 and 1.90, 24 2.63 and 2.83, 48 3.57 and 3.77, 150 4.00 and 4.12,
+// 627 4.47 and 4.60; with 32-wide panels and column-wise triangular solves 1.69,
+// 2.74, 3.65, 6.14 and 7.52.  At order 384 a solve takes 2.38 and 2.34 ms, at
+// 6048 123.9 and 118.4 ms.
+constexpr int kOneRounding = 96;
+
 // Double precision: the pushed-candidate panel for panels of at most 16
 // columns whose tile fits beside its message buffers, else the loading panel.
-template <int G, int NT>
+template <int G, int NT, bool ONE = false>
 static cudaError_t launch_push_z(cudaStream_t st, size_t smem, double2* P, long lda, int m, int jb, int rpc, int* ipiv,
                                  int k0, int* info) {
-  auto kern = k_getf2_cluster_push_z<G, NT>;
+  auto kern = k_getf2_cluster_push_z<G, NT, ONE>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kPanelSmemMax - kPushStaticSmem);
@@ -926,6 +942,7 @@ cudaError_t panel_cluster<double>(cudaStream_t st, double2* P, long lda, int m, 
   // As many threads as the rows of a CTA need, and column groups while the rows are few: warps beyond that
   // only wait, and their polls and barriers slow the others (512 threads in 16, 8, 4 and 2 groups: LU of order
   // 384 1.84 ms, of 1536 12.6 ms; so 1.58 and 11.9 ms)
+  if (k0 + m <= kOneRounding) return launch_push_z<4, 128, true>(st, smem, P, lda, m, jb, rpc, ipiv, k0, info);
   if (rpc <= 32) return launch_push_z<4, 128>(st, smem, P, lda, m, jb, rpc, ipiv, k0, info);
   if (rpc <= 64) return launch_push_z<4, 256>(st, smem, P, lda, m, jb, rpc, ipiv, k0, info);
   if (rpc <= 128) return launch_push_z<2, 256>(st, smem, P, lda, m, jb, rpc, ipiv, k0, info);
