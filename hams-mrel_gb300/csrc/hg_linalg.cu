@@ -953,7 +953,22 @@ cudaError_t getrs_inv(cudaStream_t st, int n, int nrhs, const float2* LU, long l
 // rows at a time by one warp with shuffles 48 and 41 us.  The scaling leaves
 // forward errors of random and collocation-like systems of order 384 the same to
 // 1 %.
+// A triangle in which a scaled entry would leave the range of doubles (a
+// diagonal some 10^280 away from an entry of its column) keeps its columns and
+// takes the product inside each step.
 constexpr int kSolveZ = 64;
+
+// a r stays clear of overflow and underflow (or a is zero).
+__device__ __forceinline__ bool scales_safely(double2 a, double2 r) {
+  auto top = [](double2 z) {
+    const int x = __double2hiint(z.x) & 0x7fffffff, y = __double2hiint(z.y) & 0x7fffffff;
+    return max(x, y) >> 20;  // biased exponent of the larger part
+  };
+  if (a.x == 0.0 && a.y == 0.0) return true;
+  const int ea = top(a), er = top(r), e = ea + er - 2 * 1023;
+  return ea > 0 && ea < 2047 && er > 0 && er < 2047 && e > -940 && e < 1000;
+}
+
 template <bool UPPER>
 __global__ void __launch_bounds__(2 * kSolveZ)
 k_trsm64_z(const double2* __restrict__ A, long lda, int w, double2* __restrict__ X, long ldx) {
@@ -968,12 +983,20 @@ k_trsm64_z(const double2* __restrict__ A, long lda, int w, double2* __restrict__
     const int i = e % kSolveZ, j = e / kSolveZ;
     if (i < w && (UPPER ? i <= j : i > j)) t[e] = A[i + (long)j * lda];
   }
+  bool plain = !UPPER;
   if (UPPER) {
     __syncthreads();
     if (part == 0 && row < w) rd[row] = crecip(t[row * kSolveZ + row]);
     __syncthreads();
     // columns p and w - 1 - p together have w - 1 entries above the diagonal
+    bool wide = false;
     for (int p = part; 2 * p <= w - 1; p += 2) {
+      const int j = row < p ? p : w - 1 - p, i = row < p ? row : row - p;
+      if (row >= w - 1 || (2 * p == w - 1 && row >= p)) continue;
+      wide = wide || !scales_safely(t[j * kSolveZ + i], rd[j]);
+    }
+    plain = __syncthreads_or(wide);
+    for (int p = part; 2 * p <= w - 1 && !plain; p += 2) {
       const int j = row < p ? p : w - 1 - p, i = row < p ? row : row - p;
       if (row >= w - 1 || (2 * p == w - 1 && row >= p)) continue;
       const double2 a = t[j * kSolveZ + i], r = rd[j];
@@ -984,7 +1007,13 @@ k_trsm64_z(const double2* __restrict__ A, long lda, int w, double2* __restrict__
     const int j = UPPER ? w - 1 - q : q;
     if (row == j) xs[j][part] = v;
     __syncthreads();  // also the triangle on the first step
-    const double xr = xs[j][0], xi = xs[j][1];
+    double xr = xs[j][0], xi = xs[j][1];
+    if (UPPER && plain) {
+      const double2 r = rd[j];
+      const double y = fma(-xi, r.y, xr * r.x);
+      xi = fma(xi, r.x, xr * r.y);
+      xr = y;
+    }
     if (row < w && (UPPER ? row < j : row > j)) {
       const double2 l = t[j * kSolveZ + row];
       v -= part ? fma(l.y, xr, l.x * xi) : fma(-l.y, xi, l.x * xr);  // one rounding at v's size

@@ -33,3 +33,20 @@ def test_solve_of_collocation_like_systems():
         errs.append(np.linalg.norm((x - y).astype(complex)) / np.linalg.norm(y.astype(complex)))
     s.close()
     assert np.exp(np.mean(np.log(errs))) <= 8.4 * U, errs
+
+
+# the last column's diagonal entry so far from its other entries that their quotient leaves the range of doubles
+@pytest.mark.parametrize("n", [2, 64, 130])
+@pytest.mark.parametrize("diag,entry", [(1e-300, 1e10), (1e300, 1e-10), (1e-300 + 1e-300j, -1e12j)])
+def test_graded_triangle(n, diag, entry):
+    a = np.eye(n, dtype=complex) * min(1.0, abs(entry))
+    a[:-1, -1], a[-1, -1] = entry, diag
+    b = np.full((n, 3), a[0, 0] + entry)
+    b[-1] = diag
+    s = g.load_package().hamsgpu.Solver()
+    x, _, info = s.gesv(a, b)[2:]
+    s.close()
+    # x = 1 throughout; each b was rounded once at |entry| and the entry's product is rounded there again, so rows
+    # above the last carry up to 4 units of |entry| / |diagonal| of their own
+    bound = np.full(n, 4 * 2 * U * max(1.0, abs(entry)) + 8 * U)
+    assert info == 0 and (np.abs(x - 1.0).max(axis=1) <= bound).all()
