@@ -116,7 +116,10 @@ cudaError_t launch_green_fill(cudaStream_t st, const double* rec, const double* 
   if (!deep) return launch_green_fill_fin<OUT>(st, rec, fx, ldf, n, tn, fs, grn_kind, A, S, lda, status, bins, ndiag);
   const int cols = fill_cols(n, tn);
   dim3 grid((tn + FILL_ROWS - 1) / FILL_ROWS, (n + cols - 1) / cols);
-  k_green_fill<true, OUT><<<grid, FILL_ROWS, 0, st>>>(rec, fx, ldf, n, tn, fs, grn_kind, A, S, lda, status, ndiag, cols);
+  auto kern = k_green_fill<true, OUT, 0, kNewmanRef>;
+  if constexpr (sizeof(OUT) == sizeof(double2))
+    if (grn_kind != 4) kern = k_green_fill<true, OUT, 0, kNewmanFused>;
+  kern<<<grid, FILL_ROWS, 0, st>>>(rec, fx, ldf, n, tn, fs, grn_kind, A, S, lda, status, ndiag, cols);
   return cudaGetLastError();
 }
 

@@ -15,7 +15,7 @@ namespace hg {
 // so every warp store of A/S is 32 consecutive complex entries of one column.
 // Bound by the FP64 pipe in deep water, plain form: 46.6 ms for 6048 x 6048
 // pairs before their arithmetic was cut to fewer FP64 operations
-// (hg_green.cuh), 31.7 ms with it; 0.68 and 0.42 ms for 384 x 384, where every
+// (hg_green.cuh), 32.8 ms with it; 0.68 and 0.42 ms for 384 x 384, where every
 // pair takes the panel integral.
 // ---------------------------------------------------------------------------
 constexpr int FILL_ROWS = 128;
@@ -36,7 +36,15 @@ inline int fill_cols(int n, int tn) {
 // and get the free term 2 pi on the diagonal; field points (ndiag = 0) none.
 // fpre (finite depth): FINGREEN3D's region-method values at this pair when
 // already evaluated (fin_green).  iv (deep water): 1 / fs.v.
-template <bool DEEP, typename OUT>
+// NM: the panel integral's form.  Entries rounded to single precision (stored so,
+// or grn_kind 4) keep the reference's order of operations, the others take the
+// fused one; kNewmanByKind decides by grn_kind, with a call for the former whose
+// stack frame the kernels of the main path do without (deep water, 6048 panels:
+// 34.2 ms with the call in the kernel, 32.8 without).
+enum { kNewmanFused, kNewmanRef, kNewmanByKind };
+template <typename OUT>
+constexpr int newman_form() { return sizeof(OUT) == sizeof(double2) ? kNewmanByKind : kNewmanRef; }
+template <bool DEEP, typename OUT, int NM = newman_form<OUT>()>
 __device__ __forceinline__ void fill_pair(const double* __restrict__ pr, double xp, double yp, double zp, int i, int j,
                                           const FinState& fs, int grn_kind, OUT* __restrict__ A,
                                           OUT* __restrict__ S, long lda, int ndiag, const double* fpre = nullptr,
@@ -49,8 +57,9 @@ __device__ __forceinline__ void fill_pair(const double* __restrict__ pr, double 
   if (fabs(rsq - l2) <= 1e-14 * l2) flag = (sqrt(rsq) <= lim) ? 1 : 0;
   double sij = 0.0, d0 = 0.0, d1 = 0.0, d2 = 0.0;
   if (flag) {
-    if (sizeof(OUT) == sizeof(double2)) newman_pair(pr, xp, yp, zp, sij, d0, d1, d2);
-    else newman_pair_ref(pr, xp, yp, zp, sij, d0, d1, d2);
+    if (NM == kNewmanRef) newman_pair_ref(pr, xp, yp, zp, sij, d0, d1, d2);
+    else if (NM == kNewmanByKind && grn_kind == 4) newman_pair_ref_call(pr, xp, yp, zp, sij, d0, d1, d2);
+    else newman_pair(pr, xp, yp, zp, sij, d0, d1, d2);
   }
   double2 g[4];
   if (DEEP) inf_green(xq, yq, zq, xp, yp, zp, fs.v, iv, flag, g);
@@ -80,7 +89,7 @@ __device__ __forceinline__ void fill_pair(const double* __restrict__ pr, double 
 // FAST distinguishes the instantiation compiled with fused multiply-adds
 // (the mixed form's finite-depth fill) from the one compiled without; the
 // code is the same.
-template <bool DEEP, typename OUT, int FAST = 0>
+template <bool DEEP, typename OUT, int FAST = 0, int NM = newman_form<OUT>()>
 __global__ void __launch_bounds__(FILL_ROWS)
 k_green_fill(const double* __restrict__ rec, const double* __restrict__ fx /* ldf x 3 col-major */, int ldf, int n, int tn,
              FinState fs, int grn_kind, OUT* __restrict__ A, OUT* __restrict__ S, long lda, int* status, int ndiag,
@@ -105,7 +114,7 @@ k_green_fill(const double* __restrict__ rec, const double* __restrict__ fx /* ld
   const double xp = fx[i], yp = fx[i + ldf], zp = fx[i + 2 * (size_t)ldf];
   const double iv = DEEP ? 1.0 / fs.v : 0.0;
   for (int jj = 0; jj < ncol; ++jj)
-    fill_pair<DEEP, OUT>(tile + jj * PR_SIZE, xp, yp, zp, i, col0 + jj, fs, grn_kind, A, S, lda, ndiag, nullptr, iv);
+    fill_pair<DEEP, OUT, NM>(tile + jj * PR_SIZE, xp, yp, zp, i, col0 + jj, fs, grn_kind, A, S, lda, ndiag, nullptr, iv);
 }
 
 // ---------------------------------------------------------------------------

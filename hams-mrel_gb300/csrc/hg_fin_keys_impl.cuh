@@ -573,7 +573,7 @@ k_key_linton(FinState s, int nk, const int4* __restrict__ keys, const double* __
   }
 }
 
-template <int FAST, typename OUT>
+template <int FAST, typename OUT, int NM>
 __global__ void __launch_bounds__(128)
 k_key_fill(const double* __restrict__ rec, const double* __restrict__ fx, int ldf, int tn, long np,
            const int* __restrict__ pidx, const int* __restrict__ pkey, const double* __restrict__ F, FinState fs,
@@ -581,7 +581,7 @@ k_key_fill(const double* __restrict__ rec, const double* __restrict__ fx, int ld
   for (long k = blockIdx.x * (long)blockDim.x + threadIdx.x; k < np; k += (long)gridDim.x * blockDim.x) {
     const int p = pidx ? pidx[k] : (int)k;
     const int i = p % tn, j = p / tn;
-    fill_pair<false, OUT>(rec + (size_t)j * PR_SIZE, fx[i], fx[i + ldf], fx[i + 2 * (size_t)ldf], i, j, fs, grn_kind, A, S,
+    fill_pair<false, OUT, NM>(rec + (size_t)j * PR_SIZE, fx[i], fx[i + ldf], fx[i + 2 * (size_t)ldf], i, j, fs, grn_kind, A, S,
                           lda, ndiag, F + 6 * (size_t)pkey[k]);
   }
 }
@@ -815,8 +815,10 @@ cudaError_t fin_keys_fill(cudaStream_t st, FinKeys& K, const double* rec, const 
   if (side) KE(cudaStreamWaitEvent(st, aux->ev_side, 0));
   long fb = ((long)K.np + 127) / 128;
   if (fb > 152L * 64) fb = 152L * 64;
-  k_key_fill<FAST, OUT><<<(unsigned)fb, 128, 0, st>>>(rec, fx, ldf, K.tn, K.np, K.pidx, K.pkey, K.F, fs, grn_kind, A, S, lda,
-                                                     ndiag);
+  auto fill = k_key_fill<FAST, OUT, kNewmanRef>;
+  if constexpr (sizeof(OUT) == sizeof(double2))
+    if (grn_kind != 4) fill = k_key_fill<FAST, OUT, kNewmanFused>;
+  fill<<<(unsigned)fb, 128, 0, st>>>(rec, fx, ldf, K.tn, K.np, K.pidx, K.pkey, K.F, fs, grn_kind, A, S, lda, ndiag);
   return cudaGetLastError();
 }
 

@@ -99,6 +99,12 @@ __device__ __forceinline__ void newman_pair_ref(const double* __restrict__ pr, d
   d2 = sg * (pr[PR_UI + 2] * sxt + pr[PR_UJ + 2] * syt + pr[PR_UK + 2] * szt);
 }
 
+// The same out of line, for kernels that take it only for one option.
+static __device__ __noinline__ void newman_pair_ref_call(const double* __restrict__ pr, double xf0, double xf1, double xf2,
+                                                         double& sij, double& d0, double& d1, double& d2) {
+  newman_pair_ref(pr, xf0, xf1, xf2, sij, d0, d1, d2);
+}
+
 // The angles' sum edge by edge (x, y, z in the panel's frame).
 static __device__ __noinline__ double newman_angles(const double* __restrict__ pr, double x, double y, double z) {
   const int nv = (int)pr[PR_NCN];
