@@ -15,7 +15,7 @@ namespace hg {
 // so every warp store of A/S is 32 consecutive complex entries of one column.
 // Bound by the FP64 pipe in deep water, plain form: 46.6 ms for 6048 x 6048
 // pairs before their arithmetic was cut to fewer FP64 operations
-// (hg_green.cuh), 32.8 ms with it; 0.68 and 0.42 ms for 384 x 384, where every
+// (hg_green.cuh), 33.6 ms with it; 0.68 and 0.42 ms for 384 x 384, where every
 // pair takes the panel integral.
 // ---------------------------------------------------------------------------
 constexpr int FILL_ROWS = 128;
@@ -40,7 +40,7 @@ inline int fill_cols(int n, int tn) {
 // or grn_kind 4) keep the reference's order of operations, the others take the
 // fused one; kNewmanByKind decides by grn_kind, with a call for the former whose
 // stack frame the kernels of the main path do without (deep water, 6048 panels:
-// 34.2 ms with the call in the kernel, 32.8 without).
+// 35.2 ms with the call in the kernel, 33.7 without).
 enum { kNewmanFused, kNewmanRef, kNewmanByKind };
 template <typename OUT>
 constexpr int newman_form() { return sizeof(OUT) == sizeof(double2) ? kNewmanByKind : kNewmanRef; }

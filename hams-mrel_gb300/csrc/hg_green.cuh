@@ -21,8 +21,12 @@
 
 #ifdef __CUDACC__
 #define HGD __host__ __device__
+#define HGD_INL __host__ __device__ __forceinline__
+#define HGD_CALL static __host__ __device__ __noinline__
 #else
 #define HGD
+#define HGD_INL inline
+#define HGD_CALL static inline
 #endif
 
 namespace hg {
@@ -51,7 +55,7 @@ namespace hg {
 // where a last bit of the double now and then moves the stored value by one
 // unit (outputs by up to 2e-8 near an irregular frequency).
 // ===================================================================
-__device__ __forceinline__ void newman_pair_ref(const double* __restrict__ pr, double xf0, double xf1,
+HGD_INL void newman_pair_ref(const double* __restrict__ pr, double xf0, double xf1,
                                             double xf2, double& sij, double& d0, double& d1,
                                             double& d2) {
   const double p0 = xf0 - pr[PR_PO], p1 = xf1 - pr[PR_PO + 1], p2 = xf2 - pr[PR_PO + 2];
@@ -100,13 +104,13 @@ __device__ __forceinline__ void newman_pair_ref(const double* __restrict__ pr, d
 }
 
 // The same out of line, for kernels that take it only for one option.
-static __device__ __noinline__ void newman_pair_ref_call(const double* __restrict__ pr, double xf0, double xf1, double xf2,
+HGD_CALL void newman_pair_ref_call(const double* __restrict__ pr, double xf0, double xf1, double xf2,
                                                          double& sij, double& d0, double& d1, double& d2) {
   newman_pair_ref(pr, xf0, xf1, xf2, sij, d0, d1, d2);
 }
 
 // The angles' sum edge by edge (x, y, z in the panel's frame).
-static __device__ __noinline__ double newman_angles(const double* __restrict__ pr, double x, double y, double z) {
+HGD_CALL double newman_angles(const double* __restrict__ pr, double x, double y, double z) {
   const int nv = (int)pr[PR_NCN];
   double szt = 0.0;
   for (int e = 0; e < nv; ++e) {
@@ -121,7 +125,7 @@ static __device__ __noinline__ double newman_angles(const double* __restrict__ p
   return szt;
 }
 
-__device__ __forceinline__ void newman_pair(const double* __restrict__ pr, double xf0, double xf1, double xf2,
+HGD_INL void newman_pair(const double* __restrict__ pr, double xf0, double xf1, double xf2,
                                             double& sij, double& d0, double& d1, double& d2) {
   const double p0 = xf0 - pr[PR_PO], p1 = xf1 - pr[PR_PO + 1], p2 = xf2 - pr[PR_PO + 2];
   const double x = fma(pr[PR_UI + 2], p2, fma(pr[PR_UI + 1], p1, pr[PR_UI] * p0));
@@ -197,11 +201,11 @@ __device__ __forceinline__ void newman_pair(const double* __restrict__ pr, doubl
 // ===================================================================
 // Deep water.  As above FP64 operations are what counts: Horner steps are
 // fused, the nine divisions left of some thirty-five are reciprocals on the
-// integer pipes, and the distances' square roots come with their reciprocals
-// (measured at 6048 panels: see k_green_fill).
+// integer pipes, and the distances' square roots come from their reciprocals
+// and are rounded by one residual (measured at 6048 panels: see k_green_fill).
 // ===================================================================
 template <int N>
-__device__ __forceinline__ double horner(const double (&c)[N], double t) {
+HGD_INL double horner(const double (&c)[N], double t) {
   double g = c[N - 1];
 #pragma unroll
   for (int k = N - 2; k >= 0; --k) g = fma(g, t, c[k]);
@@ -209,13 +213,19 @@ __device__ __forceinline__ double horner(const double (&c)[N], double t) {
 }
 
 // Havelock wave term GF and its horizontal derivative GFh at the
-// non-dimensional horizontal distance hh = v*R and depth vv = v*(z+zeta):
-// dd = |(hh, vv)|, alpha = -vv / dd, beta = hh / dd, ihh = 1 / hh (used
-// beyond 3).
-__device__ __forceinline__ void havelock(double hh, double vv, double dd, double alpha, double beta, double ihh,
-                                         double2& gf, double2& gfh) {
+// non-dimensional horizontal distance hh = v*R and depth vv = v*(z+zeta);
+// idd = 1 / |(hh, vv)| to a few units, ihh = 1 / hh (used beyond 3).  dd is the
+// rounded root of the rounded hh^2 + vv^2, so that it equals -vv above the source:
+// GFh is what is left there of terms of the size of exp(vv) and exp(-dd), and
+// 1 - alpha is formed from dd + vv for the same reason.  (With dd taken from R
+// and z + zeta the horizontal derivatives of near-vertical pairs were 1.6 times
+// as far off, 2.0e-13 of their size against 1.2e-13.)
+HGD_INL void havelock(double hh, double vv, double idd, double ihh, double2& gf, double2& gfh) {
   const double gama = 0.5772156649;
-  const double omr = rcp_any(1.0 + dd), rho = dd * omr;  // rho = dd / (1 + dd), omr = 1 - rho
+  const double dd = root_of(fma(hh, hh, vv * vv), idd), alpha = -vv * idd, oma = (dd + vv) * idd, beta = hh * idd;
+  const double opd = 1.0 + dd, omr = rcp_any(opd);  // 1 - rho
+  double rho = dd * omr;
+  rho = fma(fma(-rho, opd, dd), omr, rho);  // dd / (1 + dd), rounded
   const double ev = exp(vv), emd = exp(-dd);
   const double id3 = rcp_any(fma(dd * dd, dd, 1.0));
   const double ro3 = rho * (omr * omr * omr), ob = 1.0 - beta, lam = dd - vv;
@@ -265,17 +275,17 @@ __device__ __forceinline__ void havelock(double hh, double vv, double dd, double
   gf = make_double2(fma(tpe, h0, l0), -tpe * j0);
   const double ps = fma(beta + hh, rcp_any(lam), fma(2.0 * ev, dd, fma(-2.0, beta, -hh)));
   const double qs = emd * ob * fma(dd, id3, 1.0);
-  rr = fma(bob * rho * fma(-2.0, rho, 1.0), dc, fma(beta, da, -((1.0 - alpha) * db)));
+  rr = fma(bob * rho * fma(-2.0, rho, 1.0), dc, fma(beta, da, -(oma * db)));
   const double ls = fma(2.0, fma(ps, id3, ro3 * rr), -4.0 * qs);
   gfh = make_double2(fma(tpe, 2.0 / HG_PI - h1, ls), tpe * j1);
 }
 
 // INFGREEN3D (InfGreen_Appr.f90:104-186).  Source (xq,yq,zq), field (xp,yp,zp).
-__device__ __forceinline__ void inf_green(double xq, double yq, double zq, double xp, double yp, double zp, double v,
+HGD_INL void inf_green(double xq, double yq, double zq, double xp, double yp, double zp, double v,
                                           double iv, int flag, double2 g[4]) {
   const double xpq = xq - xp, ypq = yq - yp, zpq = zp + zq, zd = zq - zp;
   const double h2 = fma(xpq, xpq, ypq * ypq);
-  const double irr = h2 > 0.0 ? rsqrt_near(h2) : 0.0, rr = h2 * irr;
+  const double irr = h2 > 0.0 ? rsqrt_near(h2) : 0.0, rr = root_of(h2, irr);
   const double q1 = fma(zpq, zpq, h2), ir1 = rsqrt_near(q1), ir13 = ir1 * ir1 * ir1;
   double sgn1 = 1.0;  // sign of the image term: -1 at the infinite-frequency limit
   if (fabs(v) < SPD(1.e-8) || fabs(v + 1.0) < SPD(1.e-8)) {
@@ -283,8 +293,7 @@ __device__ __forceinline__ void inf_green(double xq, double yq, double zq, doubl
     g[0] = make_double2(0.0, 0.0); g[1] = g[0]; g[2] = g[0]; g[3] = g[0];
   } else {
     double2 gf, gfh;
-    const double is1 = copysign(ir1, v);
-    havelock(v * rr, v * zpq, fabs(v) * (q1 * ir1), -zpq * is1, rr * is1, irr * iv, gf, gfh);
+    havelock(v * rr, v * zpq, fabs(iv) * ir1, irr * iv, gf, gfh);
     const double v2 = v * v;
     if (rr > SPD(1.e-6)) {
       const double c = -v2 * irr, cx = c * xpq, cy = c * ypq;

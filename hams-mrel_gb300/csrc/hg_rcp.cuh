@@ -14,6 +14,7 @@
 // (checked against it over random and boundary significands); rcp_in_range
 // says which those are.
 #pragma once
+#include <math.h>
 #include <stdint.h>
 #include <string.h>
 
@@ -97,23 +98,33 @@ HG_HD double rcp_rn(double x) {
 // 1 / x for any x.
 HG_HD double rcp_any(double x) { return rcp_in_range(rcp_bits(x)) ? rcp_rn(x) : 1.0 / x; }
 
-#ifdef __CUDACC__
-// 1 / sqrt(x), x >= 0, within about a unit of the last place: a single-precision
-// seed (22 bits) and one third-order step in FP64, five FP64 operations against
-// about twenty for 1.0 / sqrt(x).  Outside the seed's range the latter.
-__device__ __forceinline__ double rsqrt_near(double x) {
+HG_HD float rsqrt_seed(float f) {
 #ifdef __CUDA_ARCH__
-  const uint32_t hi = (uint32_t)(rcp_bits(x) >> 32);
-  if (hi - 0x38500000u >= 0x0f500000u) return 1.0 / sqrt(x);  // below 2^-122, above 2^122, NaN
-  const float f = (float)x;
   float r;
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(f));
-  const double y = (double)r, e = fma(-x * y, y, 1.0);
-  return fma(fma(e, 0.375, 0.5) * e, y, y);
+  return r;
 #else
-  return 1.0;
+  return 1.0f / sqrtf(f);
 #endif
 }
-#endif
+
+// 1 / sqrt(x), x >= 0, within a unit of the last place: a single-precision
+// seed (22 bits) and one step of Householder's third-order iteration (1970) for
+// 1 / y^2 - x, y (1 + e / 2 + 3 e^2 / 8) with e = 1 - x y^2, five FP64
+// operations against about twenty for 1.0 / sqrt(x).  Outside the seed's range
+// the latter.
+HG_HD double rsqrt_near(double x) {
+  const uint32_t hi = (uint32_t)(rcp_bits(x) >> 32);
+  if (hi - 0x38500000u >= 0x0f500000u) return 1.0 / sqrt(x);  // below 2^-122, above 2^122, NaN
+  const double y = (double)rsqrt_seed((float)x), e = fma(-x * y, y, 1.0);
+  return fma(fma(e, 0.375, 0.5) * e, y, y);
+}
+
+// sqrt(x) from ix near 1 / sqrt(x) (0 for x = 0): half the exact residual of
+// x ix, times ix, rounds it (Markstein 1990).  Exact roots come out exactly.
+HG_HD double root_of(double x, double ix) {
+  const double r = x * ix;
+  return fma(fma(-r, r, x), 0.5 * ix, r);
+}
 
 }  // namespace hg
