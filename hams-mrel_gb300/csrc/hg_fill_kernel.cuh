@@ -15,7 +15,7 @@ namespace hg {
 // so every warp store of A/S is 32 consecutive complex entries of one column.
 // Bound by the FP64 pipe in deep water, plain form: 46.6 ms for 6048 x 6048
 // pairs before their arithmetic was cut to fewer FP64 operations
-// (hg_green.cuh), 33.6 ms with it; 0.68 and 0.42 ms for 384 x 384, where every
+// (hg_green.cuh), 33.7 ms with it; 0.68 and 0.42 ms for 384 x 384, where every
 // pair takes the panel integral.
 // ---------------------------------------------------------------------------
 constexpr int FILL_ROWS = 128;

@@ -44,11 +44,11 @@ namespace hg {
 //
 // GB300's FP64 pipe (two operations a clock and SM) bounds every caller, so
 // the work is arranged to spend few of them: vertex terms are formed once and
-// shared by the two edges that meet there, distances come from one
-// reciprocal square root, 1 / l and 1 / (s - l) run on the integer pipes
-// (hg_rcp.cuh), and the edges' angles are added as the argument of one complex
-// product: one atan2 instead of four, its multiple of 2 pi taken from the four
-// single-precision angles.
+// shared by the two edges that meet there, distances are one rounded root each,
+// 1 / l and 1 / (s - l) run on the integer pipes (hg_rcp.cuh) and each quotient
+// takes one residual, and the edges' angles are added as the argument of one
+// complex product: one atan2 instead of four, its multiple of 2 pi taken from
+// the four single-precision angles.
 //
 // newman_pair is the form of the complex128 matrices; newman_pair_ref, in the
 // reference's order of operations, that of entries rounded to single precision,
@@ -138,7 +138,7 @@ HGD_INL void newman_pair(const double* __restrict__ pr, double xf0, double xf1, 
   // vertex terms: offset, p = dx^2 + z^2, q = dx dy, distance r
   double dx = pr[PR_KSI] - x, dy = pr[PR_ETA] - y;
   double va = fma(dx, dx, z2), vq = dx * dy, vr = fma(dy, dy, va);
-  vr = vr > 0.0 ? vr * rsqrt_near(vr) : 0.0;
+  vr = sqrt_near(vr);
   const double fdx = dx, fdy = dy, fa = va, fq = vq, fr = vr;
   double st = 0.0, sxt = 0.0, syt = 0.0, szt = 0.0;
   double zr = 1.0, zi = 0.0;        // product of the edges' complex numbers
@@ -157,7 +157,7 @@ HGD_INL void newman_pair(const double* __restrict__ pr, double xf0, double xf1, 
       wa = fma(ex, ex, z2);
       wq = ex * ey;
       wr = fma(ey, ey, wa);
-      wr = wr > 0.0 ? wr * rsqrt_near(wr) : 0.0;
+      wr = sqrt_near(wr);
     }
     const double l = pr[PR_L + e];
     if (tri || !(fabs(l) < 1.0e-8)) {
@@ -175,7 +175,10 @@ HGD_INL void newman_pair(const double* __restrict__ pr, double xf0, double xf1, 
       }
       const double s = vr + wr, gap = s - l;
       if (!(fabs(gap) < 1.0e-6)) {
-        const double lg = log((s + l) * rcp_any(gap)) * rcp_any(l);
+        // both quotients rounded once: far from the panel the edges' logarithms cancel to the square of its
+        // angle, and what their arguments are off by is left over
+        const double ig = rcp_any(gap), top = s + l, q = top * ig, lq = log(fma(fma(-q, gap, top), ig, q));
+        const double il = rcp_any(l), l0 = lq * il, lg = fma(fma(-l0, l, lq), il, l0);
         sxt = fma(-deta, lg, sxt);
         syt = fma(dksi, lg, syt);
         st = fma(fma(dksi, dy, -(deta * dx)), lg, st);  // deta (x - ksi) - dksi (y - eta)

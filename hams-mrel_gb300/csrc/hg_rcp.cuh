@@ -127,4 +127,18 @@ HG_HD double root_of(double x, double ix) {
   return fma(fma(-r, r, x), 0.5 * ix, r);
 }
 
+// sqrt(x), x >= 0, rounded the same way, where its reciprocal is not needed: one
+// coupled Newton step (Goldschmidt 1964) on the seed's root and half reciprocal,
+// then the residual, seven FP64 operations.
+HG_HD double sqrt_near(double x) {
+  const uint32_t hi = (uint32_t)(rcp_bits(x) >> 32);
+  if (hi - 0x38500000u >= 0x0f500000u) return sqrt(x);
+  const double y = (double)rsqrt_seed((float)x);
+  double g = x * y, h = 0.5 * y;
+  const double r = fma(-g, h, 0.5);
+  g = fma(g, r, g);
+  h = fma(h, r, h);
+  return fma(fma(-g, g, x), h, g);
+}
+
 }  // namespace hg

@@ -1,4 +1,5 @@
-"""Rounding of the deep-water Green function (hg_green.cuh, compiled for the host) against extended precision: no further
+"""Rounding of the deep-water Green function and of Newman's panel integral
+(hg_green.cuh, compiled for the host) against extended precision: no further
 from it than the formulas written out in double precision, on average over
 the pairs of a mesh's distances.  The averages are over some 10^5 pairs each
 and fluctuate by about a per cent."""
@@ -75,8 +76,64 @@ template <class T> void green(const double* q, const double* p, double v_, int f
     o[0] += is; o[2] -= dx * s3; o[4] -= dy * s3; o[6] -= dz * s3;
   }
 }
+// Newman's integral as the formulas stand.
+template <class T> void newman(const double* pr, const double* f, T o[4]) {
+  T p[3], c[3];
+  for (int k = 0; k < 3; ++k) p[k] = (T)f[k] - pr[PR_PO + k];
+  for (int a = 0; a < 3; ++a) c[a] = pr[PR_UI + 3 * a] * p[0] + pr[PR_UI + 3 * a + 1] * p[1] + pr[PR_UI + 3 * a + 2] * p[2];
+  const T x = c[0], y = c[1], z = c[2];
+  const int nv = (int)pr[PR_NCN];
+  T st = 0, sx = 0, sy = 0, sz = 0;
+  for (int e = 0; e < nv; ++e) {
+    const int n = (e + 1) % nv;
+    const T k1 = pr[PR_KSI + e], e1 = pr[PR_ETA + e], k2 = pr[PR_KSI + n], e2 = pr[PR_ETA + n], l = pr[PR_L + e];
+    const T dk = k2 - k1, de = e2 - e1;
+    const T r1 = sqrt((k1 - x) * (k1 - x) + (e1 - y) * (e1 - y) + z * z), r2 = sqrt((k2 - x) * (k2 - x) + (e2 - y) * (e2 - y) + z * z);
+    const T b1 = de * ((k1 - x) * (k1 - x) + z * z) - dk * (k1 - x) * (e1 - y), a1 = r1 * z * dk;
+    const T b2 = de * ((k2 - x) * (k2 - x) + z * z) - dk * (k2 - x) * (e2 - y), a2 = r2 * z * dk;
+    if (!(std::abs((double)z) < 1e-6)) sz += atan2(b1 * a2 - b2 * a1, a1 * a2 + b1 * b2);
+    const T s = r1 + r2;
+    if (std::abs((double)(s - l)) < 1e-6) continue;
+    const T lg = log((s + l) / (s - l));
+    sx -= de / l * lg; sy += dk / l * lg; st += (de * (x - k1) - dk * (y - e1)) / l * lg;
+  }
+  const T sg = nv == 3 ? 1 : -1;
+  o[0] = sg * (st - z * sz);
+  for (int k = 0; k < 3; ++k) o[1 + k] = sg * (pr[PR_UI + k] * sx + pr[PR_UJ + k] * sy + pr[PR_UK + k] * sz);
+}
+
 static std::mt19937_64 gen(5);
 static double uni(double a, double b) { return std::uniform_real_distribution<double>(a, b)(gen); }
+static double nrm() { return std::normal_distribution<double>()(gen); }
+static void direction(double d[3]) {
+  double n = 0;
+  for (int k = 0; k < 3; ++k) { d[k] = nrm(); n += d[k] * d[k]; }
+  for (int k = 0; k < 3; ++k) d[k] /= std::sqrt(n);
+}
+// a planar panel of about `size` in a random frame
+static void panel(double pr[PR_SIZE], bool tri, double size) {
+  double a[3], b[3], dot = 0, n = 0;
+  direction(a); direction(b);
+  for (int k = 0; k < 3; ++k) dot += a[k] * b[k];
+  for (int k = 0; k < 3; ++k) { b[k] -= dot * a[k]; n += b[k] * b[k]; }
+  for (int k = 0; k < 3; ++k) b[k] /= std::sqrt(n);
+  for (int k = 0; k < 3; ++k) {
+    pr[PR_PO + k] = size * uni(-10, 10);
+    pr[PR_UI + k] = a[k]; pr[PR_UJ + k] = b[k];
+    pr[PR_UK + k] = a[(k + 1) % 3] * b[(k + 2) % 3] - a[(k + 2) % 3] * b[(k + 1) % 3];
+  }
+  const double w = uni(0.15, 0.65), h = uni(0.15, 0.65), sx[4] = {1, -1, -1, 1}, sy[4] = {1, 1, -1, -1};
+  const int nv = tri ? 3 : 4;
+  pr[PR_NCN] = nv;
+  for (int e = 0; e < nv; ++e) {
+    pr[PR_KSI + e] = size * (sx[e] * w + uni(-.05, .05));
+    pr[PR_ETA + e] = size * (sy[e] * h + uni(-.05, .05));
+  }
+  for (int e = 0; e < nv; ++e) {
+    const int x = (e + 1) % nv;
+    pr[PR_L + e] = std::hypot(pr[PR_KSI + x] - pr[PR_KSI + e], pr[PR_ETA + x] - pr[PR_ETA + e]);
+  }
+}
 
 int main() {
   // relative errors of G, of its horizontal and of its vertical derivative, ours and the double formula's
@@ -108,6 +165,33 @@ int main() {
     }
     for (int m = 0; m < 3; ++m) std::printf("green%d_%d %.6g %.6g\n", band, m, e[m][0], e[m][1]);
   }
+  // the same of the integral and its gradient
+  for (int band = 0; band < 5; ++band) {  // the panel's own point, then distances in panel sizes
+    double e[2][2] = {};
+    const double lo[] = {0, 0.3, 1.5, 5, 15}, hi[] = {0, 1.5, 5, 15, 50};
+    for (int k = 0; k < 100000; ++k) {
+      double pr[PR_SIZE] = {}, f[3], u[3], o[4], d[4];
+      ld x[4];
+      panel(pr, k % 4 == 3, 1.0);
+      direction(u);
+      const double r = band ? lo[band] * std::pow(hi[band] / lo[band], uni(0, 1)) : 0.0;
+      for (int c = 0; c < 3; ++c) f[c] = pr[PR_PO + c] + r * u[c];
+      newman_pair(pr, f[0], f[1], f[2], o[0], o[1], o[2], o[3]);
+      newman<double>(pr, f, d);
+      newman<ld>(pr, f, x);
+      e[0][0] += std::abs((double)((o[0] - x[0]) / x[0]));
+      e[0][1] += std::abs((double)((d[0] - x[0]) / x[0]));
+      double s = 0, a = 0, b = 0;
+      for (int c = 1; c < 4; ++c) {
+        s += (double)(x[c] * x[c]);
+        a += (double)((o[c] - x[c]) * (o[c] - x[c]));
+        b += (double)((d[c] - x[c]) * (d[c] - x[c]));
+      }
+      e[1][0] += std::sqrt(a / s);
+      e[1][1] += std::sqrt(b / s);
+    }
+    for (int m = 0; m < 2; ++m) std::printf("newman%d_%d %.6g %.6g\n", band, m, e[m][0], e[m][1]);
+  }
   return 0;
 }
 '''
@@ -128,7 +212,8 @@ def sums(tmp_path_factory):
 
 
 # a mean further off than the plain formula's by more than three of its own fluctuations is a loss
-@pytest.mark.parametrize("what", ["green%d_%d" % (b, m) for b in range(4) for m in range(3)])
+@pytest.mark.parametrize("what", ["green%d_%d" % (b, m) for b in range(4) for m in range(3)] +
+                         ["newman%d_%d" % (b, m) for b in range(5) for m in range(2)])
 def test_no_further_off_than_the_formula_in_double(sums, what):
     ours, plain = sums[what]
     assert ours <= 1.03 * plain
