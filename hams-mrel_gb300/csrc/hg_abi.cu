@@ -193,8 +193,8 @@ bool mixed(const hg_ctx* c) { return c->o.precision == HG_PREC_MIXED; }
 // Finite-depth A and S with the region methods evaluated once per distinct
 // (R, zq, zp): every pair, or with near_only those below R/h = 0.05 over what
 // A and S hold.  The keys are built on the first frequency of a mesh and depth
-// and kept.  *done = false where they do not fit (more than 2^27 pairs, or no
-// room in device memory): the caller takes the per-pair kernels.
+// and kept.  *done = false where they do not fit (more than 2^27 pairs to key, or
+// no room in device memory): the caller takes the per-pair kernels.
 template <int FAST, typename OUT>
 int keyed_fill(hg_ctx* c, int tn, int near_only, OUT* A, OUT* S, bool* done) {
   hg::FinKeys& K = c->fkeys;

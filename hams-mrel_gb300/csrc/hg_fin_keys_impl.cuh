@@ -620,7 +620,7 @@ cudaError_t keys_build_body(cudaStream_t st, FinKeys& K, const double* rec, cons
   int* cnt = nullptr;  // pair counter, then the cursors of the order of R
   KE(sc.get(&cnt, 1 + kPlaces));
   KE(cudaMemsetAsync(cnt, 0, (1 + kPlaces) * sizeof(int), st));
-  K.np = tn * n;
+  K.np = (int)((long long)tn * n);
   if (near_only) {
     k_key_pairs<FAST, false><<<g, 128, 0, st>>>(rec, fx, ldf, n, tn, h, 1, zsrc, zfld, nullptr, nullptr, 0, cnt, nullptr,
                                                 nullptr);
@@ -629,6 +629,7 @@ cudaError_t keys_build_body(cudaStream_t st, FinKeys& K, const double* rec, cons
     KE(cudaMemsetAsync(cnt, 0, sizeof(int), st));
   }
   if (K.np == 0) return cudaSuccess;
+  if (K.np > kKeyMaxPairs) return cudaErrorMemoryAllocation;
   size_t free_b = 0, total_b = 0;
   KE(cudaMemGetInfo(&free_b, &total_b));
   unsigned cap = 4096;
@@ -707,7 +708,7 @@ template <int FAST>
 cudaError_t fin_keys_build(cudaStream_t st, FinKeys& K, const double* rec, const double* fx, int ldf, int n, int tn,
                            double h, int near_only, const int* zsrc, const int* zfld, int nlev) {
   K.release();
-  if ((long long)tn * n > kKeyMaxPairs || nlev > kKeyMaxLevels) return cudaErrorMemoryAllocation;
+  if (!keys_index(tn, n, near_only, nlev)) return cudaErrorMemoryAllocation;
   const cudaError_t e = keys_build_body<FAST>(st, K, rec, fx, ldf, n, tn, h, near_only, zsrc, zfld);
   if (e != cudaSuccess) {
     K.release();
