@@ -194,26 +194,21 @@ bool mixed(const hg_ctx* c) { return c->o.precision == HG_PREC_MIXED; }
 // (R, zq, zp): every pair, or with near_only those below R/h = 0.05 over what
 // A and S hold.  The keys are built on the first frequency of a mesh and depth
 // and kept.  *done = false where they do not fit (more than 2^27 pairs to key, or
-// no room in device memory): the caller takes the per-pair kernels.
+// more memory than they may hold): the caller takes the per-pair kernels, and the
+// keys are not tried again before the next mesh, depth or limit.
 template <int FAST, typename OUT>
 int keyed_fill(hg_ctx* c, int tn, int near_only, OUT* A, OUT* S, bool* done) {
   hg::FinKeys& K = c->fkeys;
-  *done = false;
   if (K.tn != tn || K.h != c->h || K.near_only != near_only || K.fast != FAST) {
     const cudaError_t e = hg::fin_keys_build<FAST>(c->st, K, c->rec.p, c->fx.p, c->tnf, c->n, tn, c->h, near_only,
                                                    c->zsrc.p, c->zfld.p, c->nlev);
-    if (e == cudaErrorMemoryAllocation) return 0;
     CK(e);
   }
+  *done = K.fit;
+  if (!K.fit) return 0;
   const cudaError_t e = hg::fin_keys_fill<FAST, OUT>(c->st, K, c->rec.p, c->fx.p, c->tnf, c->zlev.p, fin_state(c),
                                                      c->o.grn_kind, A, S, tn, tn, &c->lu_aux);
-  if (e == cudaErrorMemoryAllocation) {
-    cudaGetLastError();
-    K.release();
-    return 0;
-  }
   CK(e);
-  *done = true;
   return 0;
 }
 
@@ -1221,6 +1216,32 @@ int hg_keep_matrices(hg_ctx* c, int keep) {
   return 0;
 }
 
+int hg_set_key_limit(hg_ctx* c, double bytes) {
+  if (!c) return -1;
+  if (std::isnan(bytes)) return fail(c, -2, "the limit is not a number");
+  c->fkeys.limit = bytes;
+  // keys within the limit stay; the others go, and those that did not fit are tried again
+  if (!c->fkeys.fit || (bytes >= 0.0 && (double)c->fkeys.peak > bytes)) {
+    CK(cudaSetDevice(c->o.device));
+    CK(cudaStreamSynchronize(c->st));
+    c->fkeys.release();
+  }
+  return 0;
+}
+
+int hg_key_info(const hg_ctx* c, double* info) {
+  if (!c) return -1;
+  if (!info) return -2;
+  const hg::FinKeys& K = c->fkeys;
+  info[0] = (double)K.bytes;
+  info[1] = (double)K.peak;
+  info[2] = (double)K.np;
+  info[3] = (double)K.nk;
+  info[4] = (double)K.passes;
+  info[5] = (double)K.builds;
+  return 0;
+}
+
 int hg_fill_factor(hg_ctx* c, int irsp) {
   if (!c) return -1;
   if (irsp != 0 && irsp != 1) return fail(c, -2, "irsp must be 0 or 1");
@@ -1647,6 +1668,8 @@ int hg_solve_sweep(hg_ctx* c, int nfreq, const double* v, const double* wk, cons
       sl->mnear_np = c->mnear_np;
       sl->mnear_tn = sweep_tn;
     }
+    const double share = c->fkeys.limit < 0.0 ? c->fkeys.limit : c->fkeys.limit / nslots;
+    if (sl->fkeys.limit != share) hg_set_key_limit(sl, share);
     for (;;) {
       const int i = next.fetch_add(1);
       if (i >= nfreq) break;
@@ -1760,8 +1783,8 @@ size_t hg_solve_footprint(int precision, int n, int nl, int nbody, int nbeta, in
   b += nn * (4 * sizeof(int) + 12 * sizeof(double) + 36 * sizeof(double)) + (nn + nl) * 3 * sizeof(double);
   // finite depth: one int per pair for the cost-binned fill; in the mixed form also the pairs'
   // map (pair index and key slot, 8 bytes per pair, and the keys, 16 bytes each, at most one per pair; their
-  // values are 48 bytes per distinct key).  The plain form's keys are not counted: they are built only
-  // into a quarter of the memory left free, and without them the cost-binned fill runs.
+  // values are 48 bytes per distinct key).  What the keys hold beyond that is not counted here: it is bounded
+  // by hg_set_key_limit, and without it the cost-binned fill runs.
   b += sizeof(int) * tn * nn;
   if (precision == HG_PREC_MIXED) b += 24 * tn * nn;
   // right-hand sides, solutions, source weights, split-K workspace

@@ -58,9 +58,12 @@ struct BesselJY {
   double2 j, y;  // orders 0 and 1
 };
 
-// The keys of one mesh and depth, and the scratch their evaluation uses.
+// The keys of one mesh and depth, and the scratch their evaluation uses.  tn, h,
+// near_only and fast say what they were built for; fit = false: they did not fit
+// in the memory they may hold, which is not tried again for the same.
 struct FinKeyData {
   int tn = -1, near_only = 0, fast = 0, nlev = 0;
+  bool fit = false;
   double h = 0.0;
   int np = 0, nr = 0, nk = 0;
   int* pidx = nullptr;     // near_only: pair index i + j tn of each listed pair
@@ -72,10 +75,14 @@ struct FinKeyData {
   double* zt = nullptr;    // per-depth tables
   double* kt = nullptr;    // Bessel tables of the groups in flight
   BesselJY* jy = nullptr;  // at wk R
-  size_t zt_cap = 0, kt_cap = 0;
+  size_t table = 0;            // bytes of kt
+  size_t bytes = 0, peak = 0;  // device memory held, and the most held while building
 };
 struct FinKeys : FinKeyData {
   std::vector<KeyGroup> groups;
+  double limit = -1.0;  // bytes they may hold, tables and the build's scratch included; < 0: see fin_keys_build
+  long builds = 0;      // builds tried
+  int passes = 0;       // passes of the last evaluation over its tables
   FinKeys() = default;
   FinKeys(const FinKeys&) = delete;
   FinKeys& operator=(const FinKeys&) = delete;
@@ -84,8 +91,10 @@ struct FinKeys : FinKeyData {
 };
 
 // Build the keys of the pairs (field row i < tn, source j < n): all of them, or
-// with near_only those below R/h = 0.05.  cudaErrorMemoryAllocation where they
-// do not fit (the caller takes the per-pair kernels).
+// with near_only those below R/h = 0.05, and everything their evaluation needs.
+// K.fit = false where they do not fit into K.limit bytes (by default a quarter
+// of the free device memory) or an allocation fails: the caller takes the
+// per-pair kernels.
 template <int FAST>
 cudaError_t fin_keys_build(cudaStream_t st, FinKeys& K, const double* rec, const double* fx, int ldf, int n, int tn,
                            double h, int near_only, const int* zsrc, const int* zfld, int nlev);

@@ -12,7 +12,8 @@ namespace {
 
 constexpr unsigned long long kKeyEmpty = ~0ull;
 constexpr int kZBits = 18;
-constexpr size_t kTableBudget = (size_t)256 << 20;  // bytes of Bessel tables in flight
+constexpr size_t kTableBudget = (size_t)256 << 20;  // bytes of Bessel tables in flight, or as few as
+constexpr size_t kTableLeast = (size_t)4 << 20;     // these where memory is short
 constexpr int kMaxSegs = 16;
 
 __device__ __forceinline__ unsigned key_hash(unsigned long long k, unsigned mask) {
@@ -156,6 +157,13 @@ __global__ void k_key_unique(const unsigned long long* __restrict__ tabk, unsign
     const unsigned zm = (1u << kZBits) - 1u;
     keys[at] = make_int4(r, (int)((key >> kZBits) & zm), (int)(key & zm), rnt[r]);
   }
+}
+
+// Occupied key slots.
+template <int FAST>
+__global__ void k_key_count(const unsigned long long* __restrict__ tabk, unsigned cap, int* __restrict__ count) {
+  const unsigned s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s < cap && tabk[s] != kKeyEmpty) bin_place(count, 0);
 }
 
 template <int FAST>
@@ -613,11 +621,18 @@ struct KeyScratch {  // build-time device memory, freed on every way out
 
 template <int FAST>
 cudaError_t keys_build_body(cudaStream_t st, FinKeys& K, const double* rec, const double* fx, int ldf, int n, int tn,
-                            double h, int near_only, const int* zsrc, const int* zfld) {
+                            double h, int near_only, const int* zsrc, const int* zfld, int nlev) {
   KeyScratch sc;
   const dim3 g((tn + 127) / 128, n);
   constexpr int kPlaces = kKeyBins * kKeySub;
+  double avail = K.limit;
+  if (avail < 0.0) {
+    size_t free_b = 0, total_b = 0;
+    KE(cudaMemGetInfo(&free_b, &total_b));
+    avail = (double)(free_b / 4);
+  }
   int* cnt = nullptr;  // pair counter, then the cursors of the order of R
+  if (avail < (double)(1 << 20)) return cudaErrorMemoryAllocation;
   KE(sc.get(&cnt, 1 + kPlaces));
   KE(cudaMemsetAsync(cnt, 0, (1 + kPlaces) * sizeof(int), st));
   K.np = (int)((long long)tn * n);
@@ -630,11 +645,11 @@ cudaError_t keys_build_body(cudaStream_t st, FinKeys& K, const double* rec, cons
   }
   if (K.np == 0) return cudaSuccess;
   if (K.np > kKeyMaxPairs) return cudaErrorMemoryAllocation;
-  size_t free_b = 0, total_b = 0;
-  KE(cudaMemGetInfo(&free_b, &total_b));
   unsigned cap = 4096;
   while (cap < 2u * (unsigned)K.np) cap <<= 1;
-  if ((size_t)24 * cap + (size_t)96 * K.np > free_b / 4) return cudaErrorMemoryAllocation;
+  const size_t small = sizeof(int) * (1 + kPlaces);  // and the groups' cursors, a few hundred bytes
+  const size_t scratch = (size_t)24 * cap + 2 * small, pairs = sizeof(int) * (size_t)K.np * (near_only ? 2 : 1);
+  if ((double)(scratch + pairs) > avail) return cudaErrorMemoryAllocation;
   unsigned long long *tabr = nullptr, *tabk = nullptr;
   int *slot2r = nullptr, *slot2k = nullptr;
   KE(sc.get(&tabr, cap));
@@ -647,9 +662,13 @@ cudaError_t keys_build_body(cudaStream_t st, FinKeys& K, const double* rec, cons
   KE(cudaMemsetAsync(tabk, 0xff, (size_t)cap * sizeof(*tabk), st));
   k_key_pairs<FAST, true><<<g, 128, 0, st>>>(rec, fx, ldf, n, tn, h, near_only, zsrc, zfld, tabr, tabk, cap - 1, cnt,
                                              K.pidx, K.pkey);
-  // distinct R by band
+  // distinct R by band, and the number of keys
   const unsigned cb = (cap + 255) / 256;
   std::vector<int> hc(kPlaces);
+  int nkeys = 0;
+  KE(cudaMemsetAsync(cnt, 0, sizeof(int), st));
+  k_key_count<FAST><<<cb, 256, 0, st>>>(tabk, cap, cnt);
+  KE(cudaMemcpyAsync(&nkeys, cnt, sizeof(int), cudaMemcpyDeviceToHost, st));
   k_key_r<FAST, false><<<cb, 256, 0, st>>>(tabr, cap, h, cnt + 1, nullptr, nullptr, nullptr);
   KE(cudaMemcpyAsync(hc.data(), cnt + 1, kPlaces * sizeof(int), cudaMemcpyDeviceToHost, st));
   KE(cudaStreamSynchronize(st));
@@ -660,6 +679,19 @@ cudaError_t keys_build_body(cudaStream_t st, FinKeys& K, const double* rec, cons
     K.nr += c;
     start[q / kKeySub + 1] = K.nr;
   }
+  // What stays: pairs, R, keys and their values, the tables.  The build's scratch is gone before the tables come.
+  const size_t keyed = pairs + (sizeof(double) + sizeof(int) + sizeof(BesselJY)) * (size_t)K.nr +
+                       (sizeof(int4) + 6 * sizeof(double)) * (size_t)nkeys;
+  const size_t fixed = keyed + ztab_doubles(nlev) * sizeof(double);
+  size_t whole = 0;
+  for (int b = 0; b < kKeyBins; ++b)
+    whole += (size_t)bin_rows(b) * bin_width(b) * sizeof(double2) * (start[b + 1] - start[b]);
+  const size_t least = whole < kTableLeast ? whole : kTableLeast;
+  if ((double)(scratch + keyed) > avail || (double)(fixed + least) > avail) return cudaErrorMemoryAllocation;
+  const size_t room = (size_t)(avail - (double)fixed), most = room < kTableBudget ? room : kTableBudget;
+  K.table = whole < most ? whole : most;
+  K.bytes = fixed + K.table;
+  K.peak = K.bytes > scratch + keyed ? K.bytes : scratch + keyed;
   KE(key_alloc(&K.rval, K.nr));
   KE(key_alloc(&K.rnt, K.nr));
   KE(key_alloc(&K.jy, K.nr));
@@ -669,7 +701,7 @@ cudaError_t keys_build_body(cudaStream_t st, FinKeys& K, const double* rec, cons
   std::vector<int> gend;
   for (int b = 0; b < kKeyBins; ++b) {
     const size_t per = (size_t)bin_rows(b) * bin_width(b) * sizeof(double2);
-    const int step = per ? (int)(kTableBudget / per) : 1 << 30;
+    const int step = per ? (int)(most / per) : 1 << 30;
     for (int r = start[b]; r < start[b + 1];) {
       const int e = (step < start[b + 1] - r) ? r + step : start[b + 1];
       K.groups.push_back(KeyGroup{b, r, e, 0, 0});
@@ -708,13 +740,19 @@ template <int FAST>
 cudaError_t fin_keys_build(cudaStream_t st, FinKeys& K, const double* rec, const double* fx, int ldf, int n, int tn,
                            double h, int near_only, const int* zsrc, const int* zfld, int nlev) {
   K.release();
-  if (!keys_index(tn, n, near_only, nlev)) return cudaErrorMemoryAllocation;
-  const cudaError_t e = keys_build_body<FAST>(st, K, rec, fx, ldf, n, tn, h, near_only, zsrc, zfld);
+  ++K.builds;
+  cudaError_t e = cudaErrorMemoryAllocation;
+  if (keys_index(tn, n, near_only, nlev)) {
+    e = keys_build_body<FAST>(st, K, rec, fx, ldf, n, tn, h, near_only, zsrc, zfld, nlev);
+    if (e == cudaSuccess && K.np > 0) e = key_alloc(&K.zt, ztab_doubles(nlev));
+    if (e == cudaSuccess && K.np > 0) e = key_alloc(&K.kt, K.table / sizeof(double));
+  }
   if (e != cudaSuccess) {
     K.release();
-    if (e == cudaErrorMemoryAllocation) cudaGetLastError();  // the per-pair kernels run instead
-    return e;
+    if (e != cudaErrorMemoryAllocation) return e;
+    cudaGetLastError();  // the per-pair kernels run instead
   }
+  K.fit = e == cudaSuccess;
   K.tn = tn;
   K.h = h;
   K.near_only = near_only;
@@ -726,16 +764,10 @@ cudaError_t fin_keys_build(cudaStream_t st, FinKeys& K, const double* rec, const
 template <int FAST, typename OUT>
 cudaError_t fin_keys_fill(cudaStream_t st, FinKeys& K, const double* rec, const double* fx, int ldf, const double* zlev,
                           const FinState& fs, int grn_kind, OUT* A, OUT* S, long lda, int ndiag, const LuAux* aux) {
+  K.passes = 0;
   if (K.np == 0) return cudaSuccess;
   if (aux && (!aux->side || !aux->ev_main || !aux->ev_side)) aux = nullptr;
   bool side = false;
-  if (K.zt_cap < ztab_doubles(K.nlev)) {
-    cudaFree(K.zt);
-    K.zt = nullptr;
-    K.zt_cap = 0;
-    KE(key_alloc(&K.zt, ztab_doubles(K.nlev)));
-    K.zt_cap = ztab_doubles(K.nlev);
-  }
   const ZTab zt = ztab_of(K.zt, K.nlev);
   bool any_pid = false;
   int most = 0;
@@ -767,22 +799,15 @@ cudaError_t fin_keys_fill(cudaStream_t st, FinKeys& K, const double* rec, const 
     size_t used = 0;
     const size_t g0 = gi;
     int rows = 0;
+    ++K.passes;
     while (gi < K.groups.size() && g.n < kMaxSegs) {
       const KeyGroup& q = K.groups[gi];
       const size_t cnt = (size_t)bin_rows(q.bin) * bin_width(q.bin) * (q.r1 - q.r0);
-      if (g.n && (used + cnt) * sizeof(double2) > kTableBudget) break;
+      if (g.n && (used + cnt) * sizeof(double2) > K.table) break;
       g.s[g.n++] = KeySeg{q.r0, q.r1 - q.r0, bin_rows(q.bin), bin_width(q.bin) == 2 ? 1 : 0, (long)used};
       used += cnt;
       rows = bin_rows(q.bin) > rows ? bin_rows(q.bin) : rows;
       ++gi;
-    }
-    if (K.kt_cap < used) {
-      KE(cudaStreamSynchronize(st));
-      cudaFree(K.kt);
-      K.kt = nullptr;
-      K.kt_cap = 0;
-      KE(key_alloc(&K.kt, 2 * used));
-      K.kt_cap = used;
     }
     double2* kt = reinterpret_cast<double2*>(K.kt);
     const int r0 = K.groups[g0].r0, r1 = K.groups[gi - 1].r1;

@@ -22,7 +22,8 @@ EXPORTS = [
     "hg_default_opts", "hg_create", "hg_destroy", "hg_last_error", "hg_set_mesh", "hg_set_frequency",
     "hg_fill_factor", "hg_solve_radiation", "hg_solve_all_headings", "hg_solve_diffraction", "hg_forces",
     "hg_solve_frequency", "hg_keep_matrices", "hg_get_matrix", "hg_green_points", "hg_refine_info",
-    "hg_stage_times", "hg_dispersion", "hg_wave_properties", "hg_panel_geometry", "hg_mark", "hg_elapsed",
+    "hg_set_key_limit", "hg_key_info", "hg_stage_times", "hg_dispersion", "hg_wave_properties",
+    "hg_panel_geometry", "hg_mark", "hg_elapsed",
     "hg_bench_gemm", "hg_green_points_noalloc", "hg_gesv", "hg_gemm_check",
     "hg_solve_sweep", "hg_gmres_iterations", "hg_solve_footprint", "hg_server_create", "hg_server_submit",
     "hg_server_wait", "hg_server_stats", "hg_server_last_error", "hg_server_destroy", "hg_field_points",
@@ -92,6 +93,8 @@ def load(build_if_missing: bool = True):
                                      c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int]
     L.hg_field_points.argtypes = [c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_int]
     L.hg_keep_matrices.argtypes = [c_void_p, c_int]
+    L.hg_set_key_limit.argtypes = [c_void_p, c_double]
+    L.hg_key_info.argtypes = [c_void_p, P(c_double)]
     L.hg_get_matrix.argtypes = [c_void_p, c_int, c_void_p, c_int]
     L.hg_green_points.argtypes = [c_void_p, c_int, c_void_p, c_void_p, c_void_p]
     L.hg_refine_info.argtypes = [c_void_p, P(c_int), P(c_double)]
@@ -266,6 +269,16 @@ class Solver:
 
     def keep_matrices(self, keep=True):
         self._check(self.L.hg_keep_matrices(self.h, 1 if keep else 0))
+
+    def set_key_limit(self, limit):
+        """Device bytes the finite-depth keys may hold; 0: none, negative: the default (hg_set_key_limit)."""
+        self._check(self.L.hg_set_key_limit(self.h, float(limit)))
+
+    def key_info(self):
+        """The finite-depth keys' memory and counts (hg_key_info)."""
+        a = (ctypes.c_double * 6)()
+        self._check(self.L.hg_key_info(self.h, a))
+        return dict(zip(("bytes", "peak", "pairs", "keys", "passes", "builds"), (int(x) for x in a)))
 
     def get_matrix(self, which, rows):
         out = np.zeros((rows, self.n), dtype=np.complex128, order="F")

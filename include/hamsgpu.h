@@ -219,6 +219,22 @@ int hg_solve_sweep(hg_ctx *ctx, int nfreq, const double *v, const double *wk, co
 size_t hg_solve_footprint(int precision, int n, int nl, int nbody, int nbeta, int irsp, int lu_tensor);
 
 /*
+ * Finite depth: the fill evaluates the Green function's series once per
+ * distinct (R, zq, zp) of a mesh and depth and keeps these keys, their values
+ * and tables in device memory beside the solve's own buffers (60 to 120 bytes a
+ * pair, of the mixed form from 1e6 pairs on a pair with R/h < 0.05; while they are
+ * built up to 212).  hg_set_key_limit says how many bytes they may hold at any
+ * time, of a sweep all its slots together: beyond it, and where an allocation
+ * fails, the pairs are evaluated one by one, with the same results.  0: always so.
+ * Negative (the default): a quarter of the device memory that is free when they
+ * are built.  hg_key_info: info[6] = bytes held, most bytes held while they were
+ * built, pairs keyed (0: pair by pair), keys, passes over the tables in the last
+ * keyed fill, builds tried in this context.
+ */
+int hg_set_key_limit(hg_ctx *ctx, double bytes);
+int hg_key_info(const hg_ctx *ctx, double *info);
+
+/*
  * Serving: continuous batching of frequency-solve requests (the serving form
  * of this path; the reference runs one request per process, HAMS_Prog).  A
  * request is a mesh (as hg_set_mesh), a depth, nfreq frequencies (wave state
