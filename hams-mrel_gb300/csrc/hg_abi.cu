@@ -43,7 +43,7 @@ struct DevBuf {
     if (p) cudaFree(p);
     p = nullptr;
     cap = 0;
-    cudaError_t e = cudaMalloc((void**)&p, (count ? count : 1) * sizeof(T));
+    cudaError_t e = hg::device_alloc((void**)&p, (count ? count : 1) * sizeof(T));
     if (e == cudaSuccess) cap = count;
     return e;
   }
@@ -199,6 +199,7 @@ bool mixed(const hg_ctx* c) { return c->o.precision == HG_PREC_MIXED; }
 template <int FAST, typename OUT>
 int keyed_fill(hg_ctx* c, int tn, int near_only, OUT* A, OUT* S, bool* done) {
   hg::FinKeys& K = c->fkeys;
+  std::lock_guard<std::mutex> lock(K.mu);
   if (K.tn != tn || K.h != c->h || K.near_only != near_only || K.fast != FAST) {
     const cudaError_t e = hg::fin_keys_build<FAST>(c->st, K, c->rec.p, c->fx.p, c->tnf, c->n, tn, c->h, near_only,
                                                    c->zsrc.p, c->zfld.p, c->nlev);
@@ -1179,6 +1180,7 @@ int hg_set_mesh(hg_ctx* c, int n, int ntnd, const double* nodes, const int* ncon
     CK(cudaMemcpyAsync(c->zlev.p, lev.data(), lev.size() * sizeof(double), cudaMemcpyHostToDevice, c->st));
     CK(cudaMemcpyAsync(c->zsrc.p, zi.data(), (size_t)n * sizeof(int), cudaMemcpyHostToDevice, c->st));
     CK(cudaMemcpyAsync(c->zfld.p, zi.data(), ((size_t)n + nl) * sizeof(int), cudaMemcpyHostToDevice, c->st));
+    std::lock_guard<std::mutex> lock(c->fkeys.mu);
     c->fkeys.release();  // the keys and the near-pair list belong to the previous mesh
     c->mnear_tn = -1;
   }
@@ -1219,6 +1221,7 @@ int hg_keep_matrices(hg_ctx* c, int keep) {
 int hg_set_key_limit(hg_ctx* c, double bytes) {
   if (!c) return -1;
   if (std::isnan(bytes)) return fail(c, -2, "the limit is not a number");
+  std::lock_guard<std::mutex> lock(c->fkeys.mu);
   c->fkeys.limit = bytes;
   // keys within the limit stay; the others go, and those that did not fit are tried again
   if (!c->fkeys.fit || (bytes >= 0.0 && (double)c->fkeys.peak > bytes)) {
@@ -1229,10 +1232,11 @@ int hg_set_key_limit(hg_ctx* c, double bytes) {
   return 0;
 }
 
-int hg_key_info(const hg_ctx* c, double* info) {
+int hg_key_info(hg_ctx* c, double* info) {
   if (!c) return -1;
-  if (!info) return -2;
-  const hg::FinKeys& K = c->fkeys;
+  if (!info) return fail(c, -2, "info is NULL");
+  hg::FinKeys& K = c->fkeys;
+  std::lock_guard<std::mutex> lock(K.mu);
   info[0] = (double)K.bytes;
   info[1] = (double)K.peak;
   info[2] = (double)K.np;

@@ -19,6 +19,11 @@ enum {
 // Single-precision literal of the Fortran source promoted to double.
 #define SPD(x) ((double)(float)(x))
 
+namespace hg {
+// cudaMalloc; where memory is short, once more after the finite-depth keys on the current device are given back.
+cudaError_t device_alloc(void** p, size_t bytes);
+}  // namespace hg
+
 struct zc {
   double re, im;
 };

@@ -7,6 +7,7 @@
 // arithmetic.  The mixed form, whose matrices are single precision, uses the
 // instantiation of hg_fill_fin_fma.cu instead (same code, contracted).
 #define HG_NO_CONTRACTION 1
+#include <algorithm>
 #include "hg_fin_keys_impl.cuh"
 
 namespace hg {
@@ -39,6 +40,64 @@ template cudaError_t launch_green_fill_fin<float2>(cudaStream_t, const double*, 
 cudaError_t launch_fin_near(cudaStream_t st, const double* rec, const double* fx, int ldf, int n, int tn,
                             const FinState& fs, int grn_kind, float2* A, float2* S, long lda, int* bins, int ndiag) {
   return launch_fin_binned<float2, 0>(st, rec, fx, ldf, n, tn, fs, grn_kind, A, S, lda, bins, ndiag, kFinNearBins);
+}
+
+namespace {
+// All keys of the process; never destroyed, since contexts may be closed while the process ends.
+struct KeyList {
+  std::mutex mu;
+  std::vector<FinKeys*> v;
+};
+KeyList& key_list() {
+  static KeyList* l = new KeyList;
+  return *l;
+}
+}  // namespace
+
+FinKeys::FinKeys() {
+  KeyList& l = key_list();
+  std::lock_guard<std::mutex> lock(l.mu);
+  l.v.push_back(this);
+}
+FinKeys::~FinKeys() {
+  {
+    KeyList& l = key_list();
+    std::lock_guard<std::mutex> lock(l.mu);
+    l.v.erase(std::find(l.v.begin(), l.v.end(), this));
+  }
+  release();
+}
+
+cudaError_t device_alloc(void** p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e != cudaErrorMemoryAllocation) return e;
+  cudaGetLastError();
+  int dev = -1;
+  bool given = false;
+  if (cudaGetDevice(&dev) != cudaSuccess) return e;
+  {
+    KeyList& l = key_list();
+    std::lock_guard<std::mutex> list(l.mu);
+    for (FinKeys* K : l.v) {
+      std::lock_guard<std::mutex> lock(K->mu);
+      if (K->device != dev || K->bytes == 0) continue;
+      const cudaError_t s = cudaDeviceSynchronize();  // evaluations still queued read them
+      if (s != cudaSuccess) return s;
+      // what they were built for stays noted, as not fitting
+      const int tn = K->tn, near_only = K->near_only, fast = K->fast;
+      const double h = K->h;
+      K->release();
+      K->tn = tn;
+      K->h = h;
+      K->near_only = near_only;
+      K->fast = fast;
+      given = true;
+    }
+  }
+  if (!given) return e;
+  e = cudaMalloc(p, bytes);
+  if (e == cudaErrorMemoryAllocation) cudaGetLastError();
+  return e;
 }
 
 void FinKeys::release() {

@@ -23,6 +23,7 @@
 // of the epsilon table fused into one pass.
 #pragma once
 #include <cuda_runtime.h>
+#include <mutex>
 #include <vector>
 #include "hg_common.cuh"
 
@@ -78,15 +79,22 @@ struct FinKeyData {
   size_t table = 0;            // bytes of kt
   size_t bytes = 0, peak = 0;  // device memory held, and the most held while building
 };
+// Keys only save time, so an allocation of this library that fails takes all of
+// the device's back (device_alloc) and is tried again: what a solve needs is there
+// whether or not another context's keys came first.  mu is held while keys are
+// built, evaluated (their launches queued) or given back; the list of all keys has
+// a lock of its own, taken before mu and never while holding one.
 struct FinKeys : FinKeyData {
+  std::mutex mu;
+  int device = -1;      // of the memory held
   std::vector<KeyGroup> groups;
   double limit = -1.0;  // bytes they may hold, tables and the build's scratch included; < 0: see fin_keys_build
   long builds = 0;      // builds tried
   int passes = 0;       // passes of the last evaluation over its tables
-  FinKeys() = default;
+  FinKeys();
   FinKeys(const FinKeys&) = delete;
   FinKeys& operator=(const FinKeys&) = delete;
-  ~FinKeys() { release(); }
+  ~FinKeys();
   void release();  // frees the device memory: no keys afterwards
 };
 

@@ -741,6 +741,7 @@ cudaError_t fin_keys_build(cudaStream_t st, FinKeys& K, const double* rec, const
                            double h, int near_only, const int* zsrc, const int* zfld, int nlev) {
   K.release();
   ++K.builds;
+  KE(cudaGetDevice(&K.device));
   cudaError_t e = cudaErrorMemoryAllocation;
   if (keys_index(tn, n, near_only, nlev)) {
     e = keys_build_body<FAST>(st, K, rec, fx, ldf, n, tn, h, near_only, zsrc, zfld, nlev);

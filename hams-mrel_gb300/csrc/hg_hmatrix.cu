@@ -334,7 +334,7 @@ struct DBuf {
     if (p) cudaFree(p);
     p = nullptr;
     cap = 0;
-    cudaError_t e = cudaMalloc((void**)&p, (count ? count : 1) * sizeof(T));
+    cudaError_t e = device_alloc((void**)&p, (count ? count : 1) * sizeof(T));
     if (e == cudaSuccess) cap = count;
     return e;
   }

@@ -227,12 +227,13 @@ size_t hg_solve_footprint(int precision, int n, int nl, int nbody, int nbeta, in
  * time, of a sweep all its slots together: beyond it, and where an allocation
  * fails, the pairs are evaluated one by one, with the same results.  0: always so.
  * Negative (the default): a quarter of the device memory that is free when they
- * are built.  hg_key_info: info[6] = bytes held, most bytes held while they were
+ * are built.  An allocation of any context that fails takes every context's keys
+ * on its device back and is tried again.  hg_key_info: info[6] = bytes held, most bytes held while they were
  * built, pairs keyed (0: pair by pair), keys, passes over the tables in the last
  * keyed fill, builds tried in this context.
  */
 int hg_set_key_limit(hg_ctx *ctx, double bytes);
-int hg_key_info(const hg_ctx *ctx, double *info);
+int hg_key_info(hg_ctx *ctx, double *info);
 
 /*
  * Serving: continuous batching of frequency-solve requests (the serving form

@@ -112,3 +112,26 @@ def test_sweep_without_keys():
         s.close()
     for a, b in zip(*out):
         assert np.array_equal(a, b)
+
+
+def test_a_failing_allocation_takes_the_keys_back():
+    """A call for more memory than any device has fails, but only after every context's keys went; they are not built
+    again for their mesh and depth, and the fill gives the same bits without them."""
+    pkg = g.load_package()
+    mesh = _mesh(pkg, "irregular")
+    a, b = (_solver(pkg, mesh, form, -1) for form in (0, 1))
+    want = [_fill(pkg, s, mesh, 1.2, 20.0) for s in (a, b)]
+    assert a.key_info()["bytes"] > 0 and b.key_info()["bytes"] > 0
+    other = pkg.hamsgpu.Solver()
+    n = 200000  # 640 GB of matrix: refused before anything is read
+    one, piv = np.zeros(2), np.zeros(1, dtype=np.int32)
+    rc = other.L.hg_gesv(other.h, 0, n, 0, one.ctypes.data, n, piv.ctypes.data, None, n, None, None)
+    assert rc < 0 and b"out of memory" in other.L.hg_last_error(other.h)
+    other.close()
+    for s, x in zip((a, b), want):
+        builds = s.key_info()["builds"]
+        assert s.key_info()["bytes"] == 0
+        y = _fill(pkg, s, mesh, 1.2, 20.0)
+        assert np.array_equal(x[0], y[0]) and np.array_equal(x[1], y[1])
+        assert s.key_info()["bytes"] == 0 and s.key_info()["builds"] == builds
+        s.close()
