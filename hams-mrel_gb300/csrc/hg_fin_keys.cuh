@@ -98,6 +98,10 @@ struct FinKeys : FinKeyData {
   void release();  // frees the device memory: no keys afterwards
 };
 
+// The most that the keys of tn x n pairs over nlev depths can hold, the build's
+// scratch included (0 where they are never keyed): every R and every key distinct.
+size_t fin_keys_bound(int tn, int n, int near_only, int nlev);
+
 // Build the keys of the pairs (field row i < tn, source j < n): all of them, or
 // with near_only those below R/h = 0.05, and everything their evaluation needs.
 // K.fit = false where they do not fit into K.limit bytes (by default a quarter

@@ -613,6 +613,21 @@ struct KeyScratch {  // build-time device memory, freed on every way out
   }
 };
 
+// Slots of a hash table for np keys, and the bytes of the build's scratch: two such tables and their maps, and the
+// cursors of the order of R.
+inline unsigned key_slots(int np) {
+  unsigned cap = 4096;
+  while (cap < 2u * (unsigned)np) cap <<= 1;
+  return cap;
+}
+constexpr int kPlaces = kKeyBins * kKeySub;
+inline size_t key_scratch_bytes(int np) { return (size_t)24 * key_slots(np) + 2 * sizeof(int) * (1 + kPlaces); }
+// Bytes of np listed pairs, nr distances and nk keys.
+inline size_t keyed_bytes(int np, int near_only, size_t nr, size_t nk) {
+  return sizeof(int) * (size_t)np * (near_only ? 2 : 1) + (sizeof(double) + sizeof(int) + sizeof(BesselJY)) * nr +
+         (sizeof(int4) + 6 * sizeof(double)) * nk;
+}
+
 #define KE(call)                          \
   do {                                    \
     const cudaError_t e_ = (call);        \
@@ -624,7 +639,6 @@ cudaError_t keys_build_body(cudaStream_t st, FinKeys& K, const double* rec, cons
                             double h, int near_only, const int* zsrc, const int* zfld, int nlev) {
   KeyScratch sc;
   const dim3 g((tn + 127) / 128, n);
-  constexpr int kPlaces = kKeyBins * kKeySub;
   double avail = K.limit;
   if (avail < 0.0) {
     size_t free_b = 0, total_b = 0;
@@ -645,11 +659,9 @@ cudaError_t keys_build_body(cudaStream_t st, FinKeys& K, const double* rec, cons
   }
   if (K.np == 0) return cudaSuccess;
   if (K.np > kKeyMaxPairs) return cudaErrorMemoryAllocation;
-  unsigned cap = 4096;
-  while (cap < 2u * (unsigned)K.np) cap <<= 1;
-  const size_t small = sizeof(int) * (1 + kPlaces);  // and the groups' cursors, a few hundred bytes
-  const size_t scratch = (size_t)24 * cap + 2 * small, pairs = sizeof(int) * (size_t)K.np * (near_only ? 2 : 1);
-  if ((double)(scratch + pairs) > avail) return cudaErrorMemoryAllocation;
+  const unsigned cap = key_slots(K.np);
+  const size_t scratch = key_scratch_bytes(K.np);
+  if ((double)(scratch + keyed_bytes(K.np, near_only, 0, 0)) > avail) return cudaErrorMemoryAllocation;
   unsigned long long *tabr = nullptr, *tabk = nullptr;
   int *slot2r = nullptr, *slot2k = nullptr;
   KE(sc.get(&tabr, cap));
@@ -680,8 +692,7 @@ cudaError_t keys_build_body(cudaStream_t st, FinKeys& K, const double* rec, cons
     start[q / kKeySub + 1] = K.nr;
   }
   // What stays: pairs, R, keys and their values, the tables.  The build's scratch is gone before the tables come.
-  const size_t keyed = pairs + (sizeof(double) + sizeof(int) + sizeof(BesselJY)) * (size_t)K.nr +
-                       (sizeof(int4) + 6 * sizeof(double)) * (size_t)nkeys;
+  const size_t keyed = keyed_bytes(K.np, near_only, K.nr, nkeys);
   const size_t fixed = keyed + ztab_doubles(nlev) * sizeof(double);
   size_t whole = 0;
   for (int b = 0; b < kKeyBins; ++b)

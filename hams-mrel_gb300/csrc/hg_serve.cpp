@@ -7,7 +7,8 @@
 // CUDA stream, driven by its own host thread), and:
 //   - admits queued requests in arrival order while the device memory they
 //     may hold stays within the budget: a request reserves
-//     min(nslots, nfreq) x hg_solve_footprint(its size) plus its mesh, and
+//     min(nslots, nfreq) x hg_solve_footprint(its size) plus its mesh, over a
+//     bottom also what the keys of its pairs may hold (see key_share), and
 //     gives the reservation back when its last frequency is done;
 //   - hands the frequencies of all admitted requests to whichever slot is
 //     free, preferring the request whose mesh the slot already holds (the
@@ -38,6 +39,7 @@
 
 namespace hg {
 size_t hmatrix_bytes_estimate(int n, const double* xyz, int nc);  // hg_hmatrix.cu
+size_t fin_keys_bound(int tn, int n, int near_only, int nlev);    // hg_fill_fin.cu
 }
 
 // Milliseconds from ref (an event recorded earlier on the context's device)
@@ -62,7 +64,8 @@ struct Request {
   std::vector<double> amas, bdmp, exfc;
   // state
   size_t reserve = 0;       // bytes reserved at admission
-  size_t slot_bytes = 0;    // one solve's footprint
+  size_t slot_bytes = 0;    // one solve's footprint, its keys included
+  size_t key_limit = 0;     // of which the keys may hold (hg_set_key_limit)
   int next = 0;             // next frequency to hand out
   int done = 0;             // frequencies finished
   int rc = 0;               // first error
@@ -189,7 +192,10 @@ void worker(hg_server* s, int k) {
       if (rc) msg = "creating a solve slot failed";
     }
     if (!rc && sl.mesh_of != r->id) {
-      rc = hg_set_mesh(sl.ctx, r->n, r->ntnd, r->nodes.data(), r->ncon.data(), r->ncn.data(), r->xyz.data(),
+      sl.mesh_of = -1;
+      rc = hg_set_key_limit(sl.ctx, (double)r->key_limit);
+      if (!rc)
+        rc = hg_set_mesh(sl.ctx, r->n, r->ntnd, r->nodes.data(), r->ncon.data(), r->ncn.data(), r->xyz.data(),
                        r->ds.data(), r->pnsz.data(), r->dxyz.data(), r->nl, r->nl ? r->lid.data() : nullptr,
                        r->nbody, r->ranges.data());
       if (rc) msg = hg_last_error(sl.ctx);
@@ -223,6 +229,31 @@ void worker(hg_server* s, int k) {
       finish_unit(s, r);
     }
   }
+}
+
+// Bytes beyond hg_solve_footprint that a request's slots may each hold for their
+// keys, and in *limit all that the keys may hold: up to everything that keys of its
+// size can come to (fin_keys_bound), as far as that leaves every slot of the server
+// an equal part of the budget.  hg_solve_footprint counts 4 bytes a pair for the
+// pair-by-pair fill, in the mixed form 24 more, which keys use instead.  A request
+// over a bottom that fits the budget without this extra is admitted without it, and
+// its pairs are evaluated one by one where the keys then do not fit.
+size_t key_share(const hg_opts& o, const hg_request& q, size_t base, size_t mesh, size_t budget, int nslots, size_t* limit) {
+  *limit = 0;
+  if (!(q.h > 0.0)) return 0;
+  const long long rows = (long long)q.n + (q.irsp == 1 ? q.nl : 0), pairs = rows * q.n;
+  const bool mixed = o.precision == HG_PREC_MIXED;
+  const bool near_only = mixed && o.grn_kind == 8 && (o.fin_table == 1 || (o.fin_table < 0 && pairs >= 1000000LL));
+  std::vector<double> z(q.xyz_p + 2 * (size_t)q.n, q.xyz_p + 3 * (size_t)q.n);
+  if (q.nl > 0) z.insert(z.end(), q.lid_xyz_p + 2 * (size_t)q.nl, q.lid_xyz_p + 3 * (size_t)q.nl);
+  std::sort(z.begin(), z.end());
+  const int nlev = (int)(std::unique(z.begin(), z.end()) - z.begin());
+  const size_t counted = (size_t)pairs * (mixed ? 28 : 4);
+  const size_t bound = rows <= 2147483647LL ? hg::fin_keys_bound((int)rows, q.n, near_only ? 1 : 0, nlev) : 0;
+  const size_t part = (budget - std::min(budget, mesh)) / nslots;
+  const size_t extra = std::min(bound > counted ? bound - counted : 0, part > base ? part - base : 0);
+  *limit = std::min(bound, counted + extra);
+  return extra;
 }
 
 template <typename T>
@@ -342,7 +373,10 @@ int hg_server_submit(hg_server* s, const hg_request* q, long long* ticket) {
   r->exfc.assign((size_t)q->nfreq * (q->nbeta > 0 ? q->nbeta : 0) * nd * 2, 0.0);
   r->slot_bytes = hg_solve_footprint(s->opts.precision, q->n, q->nl, q->nbody, q->nbeta, q->irsp, s->opts.lu_tensor) +
                   iter_bytes(s->opts, *q);
-  r->reserve = (size_t)std::min(s->nslots, q->nfreq) * r->slot_bytes + mesh_bytes(*r);
+  const size_t used = (size_t)std::min(s->nslots, q->nfreq), mesh = mesh_bytes(*r);
+  if (used * r->slot_bytes + mesh <= s->budget)
+    r->slot_bytes += key_share(s->opts, *q, r->slot_bytes, mesh, s->budget, s->nslots, &r->key_limit);
+  r->reserve = used * r->slot_bytes + mesh;
   if (r->reserve > s->budget) {
     s->err = "request needs " + std::to_string(r->reserve) + " bytes of device memory, above the budget of " +
              std::to_string(s->budget);

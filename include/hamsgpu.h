@@ -247,7 +247,9 @@ int hg_key_info(hg_ctx *ctx, double *info);
  * device.  Admission: requests are admitted in arrival order while the
  * reserved device memory, min(nslots, nfreq) x hg_solve_footprint + mesh per
  * admitted request, stays within budget_bytes; a request larger than the
- * budget is rejected by hg_server_submit (-3).  Each result equals that of
+ * budget is rejected by hg_server_submit (-3).  Over a bottom a request reserves
+ * more per solve for its keys (hg_set_key_limit): what they can come to at most,
+ * but no more than leaves each slot budget_bytes / nslots.  Each result equals that of
  * hg_solve_frequency on a single context (same kernels, same order).
  *   hg_server_wait: blocks (timeout_s <= 0) or waits up to timeout_s seconds
  *     (returns 1 if the request is not finished); copies amas, bdmp
