@@ -108,16 +108,20 @@ HG_HD float rsqrt_seed(float f) {
 #endif
 }
 
+// Where the seed and the steps' products are normal: 2^-122 to 2^122.
+HG_HD bool rsqrt_in_range(double x) { return (uint32_t)(rcp_bits(x) >> 32) - 0x38500000u < 0x0f500000u; }
+
 // 1 / sqrt(x), x >= 0, within a unit of the last place: a single-precision
 // seed (22 bits) and one step of Householder's third-order iteration (1970) for
 // 1 / y^2 - x, y (1 + e / 2 + 3 e^2 / 8) with e = 1 - x y^2, five FP64
 // operations against about twenty for 1.0 / sqrt(x).  Outside the seed's range
 // the latter.
-HG_HD double rsqrt_near(double x) {
-  const uint32_t hi = (uint32_t)(rcp_bits(x) >> 32);
-  if (hi - 0x38500000u >= 0x0f500000u) return 1.0 / sqrt(x);  // below 2^-122, above 2^122, NaN
-  const double y = (double)rsqrt_seed((float)x), e = fma(-x * y, y, 1.0);
+HG_HD double rsqrt_from_seed(double x, double y) {
+  const double e = fma(-x * y, y, 1.0);
   return fma(fma(e, 0.375, 0.5) * e, y, y);
+}
+HG_HD double rsqrt_near(double x) {
+  return rsqrt_in_range(x) ? rsqrt_from_seed(x, (double)rsqrt_seed((float)x)) : 1.0 / sqrt(x);
 }
 
 // sqrt(x) from ix near 1 / sqrt(x) (0 for x = 0): half the exact residual of
@@ -130,15 +134,13 @@ HG_HD double root_of(double x, double ix) {
 // sqrt(x), x >= 0, rounded the same way, where its reciprocal is not needed: one
 // coupled Newton step (Goldschmidt 1964) on the seed's root and half reciprocal,
 // then the residual, seven FP64 operations.
-HG_HD double sqrt_near(double x) {
-  const uint32_t hi = (uint32_t)(rcp_bits(x) >> 32);
-  if (hi - 0x38500000u >= 0x0f500000u) return sqrt(x);
-  const double y = (double)rsqrt_seed((float)x);
+HG_HD double sqrt_from_seed(double x, double y) {
   double g = x * y, h = 0.5 * y;
   const double r = fma(-g, h, 0.5);
   g = fma(g, r, g);
   h = fma(h, r, h);
   return fma(fma(-g, g, x), h, g);
 }
+HG_HD double sqrt_near(double x) { return rsqrt_in_range(x) ? sqrt_from_seed(x, (double)rsqrt_seed((float)x)) : sqrt(x); }
 
 }  // namespace hg
