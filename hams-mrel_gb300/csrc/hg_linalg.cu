@@ -947,7 +947,7 @@ cudaError_t getrs_inv(cudaStream_t st, int n, int nrhs, const float2* LU, long l
 // difference (one rounding at the row's size) on each scheduler, one warp
 // instruction of which occupies its FP64 pipe for 64 cycles, and one barrier.  An upper triangle's columns are
 // divided by their diagonal first, all at once, and the solution at the end, so
-// that its steps are the lower one's: 20 us (lower) and 24 us (upper) for 64
+// that its steps are the lower one's: 20 us (lower) and 27 us (upper) for 64
 // rows; with two roundings a step in place of one 18 and 22 us, with the
 // product by the reciprocal inside each step of the upper triangle 31 us, and 16
 // rows at a time by one warp with shuffles 48 and 41 us.  The scaling leaves
@@ -955,7 +955,8 @@ cudaError_t getrs_inv(cudaStream_t st, int n, int nrhs, const float2* LU, long l
 // 1 %.
 // A triangle in which a scaled entry would leave the range of doubles (a
 // diagonal some 10^280 away from an entry of its column) keeps its columns and
-// takes the product inside each step.
+// takes the product inside each step, in a loop of its own (as a branch inside
+// the steps it took every triangle 36 us).
 constexpr int kSolveZ = 64;
 
 // a r stays clear of overflow and underflow (or a is zero).
@@ -979,44 +980,48 @@ k_trsm64_z(const double2* __restrict__ A, long lda, int w, double2* __restrict__
   const int row = threadIdx.x & (kSolveZ - 1), part = threadIdx.x / kSolveZ;
   double* xc = reinterpret_cast<double*>(X + (long)blockIdx.x * ldx + row) + part;
   double v = row < w ? *xc : 0.0;
-  for (int e = threadIdx.x; e < w * kSolveZ; e += 2 * kSolveZ) {
-    const int i = e % kSolveZ, j = e / kSolveZ;
-    if (i < w && (UPPER ? i <= j : i > j)) t[e] = A[i + (long)j * lda];
-  }
-  bool plain = !UPPER;
+  auto load = [&]() {
+    for (int e = threadIdx.x; e < w * kSolveZ; e += 2 * kSolveZ) {
+      const int i = e % kSolveZ, j = e / kSolveZ;
+      if (i < w && (UPPER ? i <= j : i > j)) t[e] = A[i + (long)j * lda];
+    }
+  };
+  load();
+  bool wide = false;
   if (UPPER) {
     __syncthreads();
     if (part == 0 && row < w) rd[row] = crecip(t[row * kSolveZ + row]);
     __syncthreads();
     // columns p and w - 1 - p together have w - 1 entries above the diagonal
-    bool wide = false;
     for (int p = part; 2 * p <= w - 1; p += 2) {
       const int j = row < p ? p : w - 1 - p, i = row < p ? row : row - p;
       if (row >= w - 1 || (2 * p == w - 1 && row >= p)) continue;
-      wide = wide || !scales_safely(t[j * kSolveZ + i], rd[j]);
-    }
-    plain = __syncthreads_or(wide);
-    for (int p = part; 2 * p <= w - 1 && !plain; p += 2) {
-      const int j = row < p ? p : w - 1 - p, i = row < p ? row : row - p;
-      if (row >= w - 1 || (2 * p == w - 1 && row >= p)) continue;
       const double2 a = t[j * kSolveZ + i], r = rd[j];
+      wide = wide || !scales_safely(a, r);
       t[j * kSolveZ + i] = make_double2(fma(-a.y, r.y, a.x * r.x), fma(a.y, r.x, a.x * r.y));
     }
+    wide = __syncthreads_or(wide);
   }
-  for (int q = 0; q < w; ++q) {
-    const int j = UPPER ? w - 1 - q : q;
-    if (row == j) xs[j][part] = v;
-    __syncthreads();  // also the triangle on the first step
-    double xr = xs[j][0], xi = xs[j][1];
-    if (UPPER && plain) {
-      const double2 r = rd[j];
-      const double y = fma(-xi, r.y, xr * r.x);
-      xi = fma(xi, r.x, xr * r.y);
-      xr = y;
+  if (UPPER && wide) {
+    load();
+    for (int j = w - 1; j >= 0; --j) {
+      if (row == j) xs[j][part] = v;
+      __syncthreads();  // also the triangle on the first step
+      const double yr = xs[j][0], yi = xs[j][1];
+      const double2 r = rd[j], l = t[j * kSolveZ + row];
+      const double xr = fma(-yi, r.y, yr * r.x), xi = fma(yi, r.x, yr * r.y);
+      if (row < j) v -= part ? fma(l.y, xr, l.x * xi) : fma(-l.y, xi, l.x * xr);
     }
-    if (row < w && (UPPER ? row < j : row > j)) {
-      const double2 l = t[j * kSolveZ + row];
-      v -= part ? fma(l.y, xr, l.x * xi) : fma(-l.y, xi, l.x * xr);  // one rounding at v's size
+  } else {
+    for (int q = 0; q < w; ++q) {
+      const int j = UPPER ? w - 1 - q : q;
+      if (row == j) xs[j][part] = v;
+      __syncthreads();  // also the triangle on the first step
+      const double xr = xs[j][0], xi = xs[j][1];
+      if (row < w && (UPPER ? row < j : row > j)) {
+        const double2 l = t[j * kSolveZ + row];
+        v -= part ? fma(l.y, xr, l.x * xi) : fma(-l.y, xi, l.x * xr);  // one rounding at v's size
+      }
     }
   }
   if (row >= w) return;
