@@ -100,10 +100,9 @@ cudaError_t device_alloc(void** p, size_t bytes) {
   return e;
 }
 
-size_t fin_keys_bound(int tn, int n, int near_only, int nlev) {
-  if (!keys_index(tn, n, near_only, nlev)) return 0;
-  const long long all = (long long)tn * n;
-  const int np = (int)(all < kKeyMaxPairs ? all : kKeyMaxPairs);
+size_t fin_keys_bound(long long pairs, int near_only, int nlev) {
+  if (pairs <= 0 || nlev > kKeyMaxLevels) return 0;
+  const int np = (int)(pairs < kKeyMaxPairs ? pairs : kKeyMaxPairs);
   size_t row = 0;  // table bytes of one R in the band with the longest series
   for (int b = 0; b < kKeyBins; ++b) row = std::max(row, (size_t)bin_rows(b) * bin_width(b) * sizeof(double2));
   const size_t keyed = keyed_bytes(np, near_only, np, np), table = std::min(kTableBudget, row * (size_t)np);

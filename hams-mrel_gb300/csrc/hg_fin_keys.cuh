@@ -98,9 +98,9 @@ struct FinKeys : FinKeyData {
   void release();  // frees the device memory: no keys afterwards
 };
 
-// The most that the keys of tn x n pairs over nlev depths can hold, the build's
-// scratch included (0 where they are never keyed): every R and every key distinct.
-size_t fin_keys_bound(int tn, int n, int near_only, int nlev);
+// The most that the keys of np pairs (at most kKeyMaxPairs are keyed) over nlev
+// depths can hold, the build's scratch included: every R and every key distinct.
+size_t fin_keys_bound(long long np, int near_only, int nlev);
 
 // Build the keys of the pairs (field row i < tn, source j < n): all of them, or
 // with near_only those below R/h = 0.05, and everything their evaluation needs.

@@ -23,6 +23,7 @@
 #include <algorithm>
 #include <atomic>
 #include <chrono>
+#include <cmath>
 #include <condition_variable>
 #include <cstring>
 #include <deque>
@@ -39,7 +40,7 @@
 
 namespace hg {
 size_t hmatrix_bytes_estimate(int n, const double* xyz, int nc);  // hg_hmatrix.cu
-size_t fin_keys_bound(int tn, int n, int near_only, int nlev);    // hg_fill_fin.cu
+size_t fin_keys_bound(long long np, int near_only, int nlev);     // hg_fill_fin.cu
 }
 
 // Milliseconds from ref (an event recorded earlier on the context's device)
@@ -231,10 +232,35 @@ void worker(hg_server* s, int k) {
   }
 }
 
+// At least as many pairs as lie closer than r horizontally: those of panels and
+// field points in the same or adjacent squares of side r.
+long long near_pairs_bound(const hg_request& q, double r) {
+  std::map<std::pair<long long, long long>, std::pair<long long, long long>> cell;  // sources, field points
+  const int nl = q.irsp == 1 ? q.nl : 0;
+  for (int i = 0; i < q.n + nl; ++i) {
+    const double x = i < q.n ? q.xyz_p[i] : q.lid_xyz_p[i - q.n];
+    const double y = i < q.n ? q.xyz_p[i + (size_t)q.n] : q.lid_xyz_p[i - q.n + (size_t)q.nl];
+    const double cx = std::floor(x / r), cy = std::floor(y / r);
+    if (!(std::fabs(cx) < 1e15 && std::fabs(cy) < 1e15)) return (long long)(q.n + nl) * q.n;
+    auto& c = cell[{(long long)cx, (long long)cy}];
+    if (i < q.n) ++c.first;
+    ++c.second;
+  }
+  long long pairs = 0;
+  for (const auto& a : cell)
+    for (int dx = -1; dx <= 1; ++dx)
+      for (int dy = -1; dy <= 1; ++dy) {
+        const auto b = cell.find({a.first.first + dx, a.first.second + dy});
+        if (b != cell.end()) pairs += a.second.first * b->second.second;
+      }
+  return pairs;
+}
+
 // Bytes beyond hg_solve_footprint that a request's slots may each hold for their
 // keys, and in *limit all that the keys may hold: up to everything that keys of its
-// size can come to (fin_keys_bound), as far as that leaves every slot of the server
-// an equal part of the budget.  hg_solve_footprint counts 4 bytes a pair for the
+// pairs can come to (fin_keys_bound; with tables only the pairs below R/h = 0.05 are
+// keyed), as far as that leaves every slot of the server an equal part of the
+// budget.  hg_solve_footprint counts 4 bytes a pair for the
 // pair-by-pair fill, in the mixed form 24 more, which keys use instead.  A request
 // over a bottom that fits the budget without this extra is admitted without it, and
 // its pairs are evaluated one by one where the keys then do not fit.
@@ -249,7 +275,7 @@ size_t key_share(const hg_opts& o, const hg_request& q, size_t base, size_t mesh
   std::sort(z.begin(), z.end());
   const int nlev = (int)(std::unique(z.begin(), z.end()) - z.begin());
   const size_t counted = (size_t)pairs * (mixed ? 28 : 4);
-  const size_t bound = rows <= 2147483647LL ? hg::fin_keys_bound((int)rows, q.n, near_only ? 1 : 0, nlev) : 0;
+  const size_t bound = hg::fin_keys_bound(near_only ? near_pairs_bound(q, 0.0500001 * q.h) : pairs, near_only ? 1 : 0, nlev);
   const size_t part = (budget - std::min(budget, mesh)) / nslots;
   const size_t extra = std::min(bound > counted ? bound - counted : 0, part > base ? part - base : 0);
   *limit = std::min(bound, counted + extra);
