@@ -897,7 +897,9 @@ int build_rhs(hg_ctx* c, int nbeta, const double* betas_h, bool modes) {
     // B = S [modes | headings]: digit-sliced on the tensor cores (their digits in the LU's workspace,
     // which the plain form keeps nothing in after the factorisation), below their order on the FP64
     // pipes; one thread per row (launch_rhs) takes 4.2 ms against about 1 ms at 6048 panels, 0.6 ms
-    // against 0.02 ms at 384
+    // against 0.02 ms at 384.  The digits cut each entry 2^-57 below its row's and column's largest and the
+    // sums are exact: on the five-body array columns are 1.1e-16 of their norm off and entries 1.0e-16 of
+    // their own (median), with sums in double precision 4.4e-16 and 4.5e-16.
     const int nc = 6 * c->nbody + nbeta;
     const size_t zb = c->o.lu_tensor != 0 && hg::zgemm_tc_supported() ? hg::zgemm_tc_work_bytes(c->tn, nc, c->n) : 0;
     const bool small = c->n < kSmallOrder, ztc = !small && zb && c->luws.cap >= zb;
@@ -1316,7 +1318,7 @@ int hg_fill_factor(hg_ctx* c, int irsp) {
                        (c->o.fin_table == 1 || (c->o.fin_table < 0 && (long long)tn * n >= 1000000LL));
     if (table) {
       CK(c->tab.ensure(hg::fintab_floats() + (size_t)6 * n));
-      // pairs below R/h = 0.05 (LINTON, PIDCOCK) per pair in FP64 after the
+      // pairs below R/h = 0.05 (LINTON, PIDCOCK) in FP64, keyed, after the
       // tables (the reference's values there are not smooth enough to
       // interpolate), which then hold only the bands above
       const bool near = (long long)tn * n < 2147483647LL;

@@ -17,10 +17,13 @@
 // rounding R to share more of them changes the epsilon-extrapolated values of
 // whole matrices coherently (measured: F moves to 1.2e-4).
 //
-// What bounds it: the FP64 pipe (about one operation per clock and SM), in the
-// extrapolation's reciprocals: n^2 / 2 of them per sum of n terms, three sums
-// per key.  They run from shared memory, one sum per thread, the level pairs
-// of the epsilon table fused into one pass.
+// What bounds it: in the extrapolation n^2 / 2 entries per sum of n terms, three
+// sums per key, each entry a reciprocal on the integer pipes (hg_rcp.cuh) and a
+// difference and a sum on the FP64 pipe, whose two operations a clock and SM are
+// 45 to 70 % used (shared memory holds few warps of sums); before it the FP64 pipe
+// in the Bessel functions of distances and terms.  The sums run from shared
+// memory, one per thread, the level pairs of the epsilon table fused into one
+// pass.
 #pragma once
 #include <cuda_runtime.h>
 #include <mutex>

@@ -286,8 +286,8 @@ k_getf2(typename cx<R>::T* P, long lda, int m, int jb, int* ipiv, int k0, int* i
 // Apply the pivots ipiv[r0..r1) (1-based global rows) to every column of A
 // outside [skip0, skip1).  A warp looks at 32 pivots at once and walks only
 // those that interchange rows: one pivot at a time, each a dependent load, took
-// 83 us for 1440 of them (block-preconditioned solve of the five-body array 18.1
-// against 17.3 ms).
+// 95 us for 1440 of them and 61 us for 864 (38 columns, under ncu); so 22 and 13
+// to 18 us.
 template <typename T>
 __global__ void k_laswp(T* A, long lda, int ncols, const int* ipiv, int r0, int r1, int skip0, int skip1) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;

@@ -7,8 +7,9 @@
 // point: a single-precision seed (22 bits), two Newton steps y += y (1 - m y)
 // in 64-bit integers (43 and then over 60 bits), and a final exact comparison
 // of m (2 q + 1) with 2^106 that rounds the quotient q to nearest (a tie
-// cannot occur).  Three 32-bit multiplies per step and about fifty
-// instructions in all, none of them FP64.
+// cannot occur).  Three 32-bit multiplies in the first step, five in the second
+// and a 64-bit product at the end, about fifty instructions in all, none of them
+// FP64.
 //
 // Same bits as 1.0 / x for every x whose reciprocal is a normal number
 // (checked against it over random and boundary significands); rcp_in_range
