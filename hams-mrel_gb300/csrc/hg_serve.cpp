@@ -41,6 +41,7 @@
 namespace hg {
 size_t hmatrix_bytes_estimate(int n, const double* xyz, int nc);  // hg_hmatrix.cu
 size_t fin_keys_bound(long long np, int near_only, int nlev);     // hg_fill_fin.cu
+size_t fintab_floats();                                           // hg_fintab.cu
 }
 
 // Milliseconds from ref (an event recorded earlier on the context's device)
@@ -261,7 +262,9 @@ long long near_pairs_bound(const hg_request& q, double r) {
 // pairs can come to (fin_keys_bound; with tables only the pairs below R/h = 0.05 are
 // keyed), as far as that leaves every slot of the server an equal part of the
 // budget.  hg_solve_footprint counts 4 bytes a pair for the
-// pair-by-pair fill, in the mixed form 24 more, which keys use instead.  A request
+// pair-by-pair fill, in the mixed form 24 more, which keys use instead, and with them
+// what it does not count, the Green-function tables' scratch and the right-hand
+// sides' source columns.  A request
 // over a bottom that fits the budget without this extra is admitted without it, and
 // its pairs are evaluated one by one where the keys then do not fit.
 size_t key_share(const hg_opts& o, const hg_request& q, size_t base, size_t mesh, size_t budget, int nslots, size_t* limit) {
@@ -274,7 +277,9 @@ size_t key_share(const hg_opts& o, const hg_request& q, size_t base, size_t mesh
   if (q.nl > 0) z.insert(z.end(), q.lid_xyz_p + 2 * (size_t)q.nl, q.lid_xyz_p + 3 * (size_t)q.nl);
   std::sort(z.begin(), z.end());
   const int nlev = (int)(std::unique(z.begin(), z.end()) - z.begin());
-  const size_t counted = (size_t)pairs * (mixed ? 28 : 4);
+  const size_t other = (near_only ? 4 * (hg::fintab_floats() + (size_t)6 * q.n) : 0) +
+                       (size_t)q.n * (6 * (size_t)q.nbody + (size_t)q.nbeta) * 16;
+  const size_t pool = (size_t)pairs * (mixed ? 28 : 4), counted = pool - std::min(pool, other);
   const size_t bound = hg::fin_keys_bound(near_only ? near_pairs_bound(q, 0.0500001 * q.h) : pairs, near_only ? 1 : 0, nlev);
   const size_t part = (budget - std::min(budget, mesh)) / nslots;
   const size_t extra = std::min(bound > counted ? bound - counted : 0, part > base ? part - base : 0);
